@@ -261,6 +261,13 @@ static bool find_turn_threshold(double tu, double* thr) {
     return true;
 }
 
+static void set_turn_test(TraceArgs& a, double tu) {
+    a.tu_angle = tu;
+    a.gc_reject = 0.;
+    a.turn_exact = find_turn_threshold(tu, &a.gc_reject) ? 1 : 0;
+    a.gc_half = 0.5 * (nextafter(a.gc_reject, 2.) - a.gc_reject);
+}
+
 // ---- dispatch over the compile-time model sets ---------------------------
 static bool model_set_ok(const cor_model_set& m) {
     const bool in_ok = m.internal_model == COR_INTERNAL_NONE || m.internal_model == COR_INTERNAL_SH;
@@ -290,6 +297,33 @@ static const ModelOps* find_ops(const cor_model_set& m) {
 // with at most min_park live trajectories) runs without parking.  The host
 // reads the parked count between generations, so this call synchronises the
 // stream once per generation.
+
+// Whether `live` trajectories run by teams (team.cuh) instead of one to a
+// lane: up to half of the lanes of cap_blocks scan blocks.  Below that the
+// lanes' own code leaves sub-partitions idle or lanes of a warp waiting for
+// the longest; above it their throughput is the higher one.  IGRF-14, ms by
+// lanes / by teams: 400 trajectories 331 / 109, 8,000 243 / 86, 20,000
+// 286 / 178, 40,000 375 / 325 (291 when the teams take over at half the
+// lanes), 91,200 562 / 666 (487).
+static bool team_takes(const ModelOps* ops, uint64_t live, uint64_t cap_blocks) {
+    return ops->launch_team && 2 * live <= cap_blocks * (uint64_t)kTraceThreads;
+}
+
+// Slots per block and blocks of a team launch: as many blocks as are resident
+// before a block takes a second slot (a lone trajectory's step is the
+// shortest), at most kTeamSlots slots.
+static int team_shape(cor_ctx* ctx, const ModelOps* ops, uint64_t live, int* slots, unsigned* blocks) {
+    int per_sm = 0;
+    CUDA_TRY(ctx, ops->team_occupancy(kTeamSlots, &per_sm));
+    if (per_sm < 1) per_sm = 1;
+    const uint64_t cap = (uint64_t)per_sm * (uint64_t)ctx->sms;
+    uint64_t n = (live + cap - 1) / cap;
+    if (n > (uint64_t)kTeamSlots) n = kTeamSlots;
+    const uint64_t b = (live + n - 1) / n;
+    *slots = (int)n;
+    *blocks = (unsigned)(b < cap ? b : cap);
+    return COR_OK;
+}
 
 static int launch_trace(cor_ctx* ctx, const ModelOps* ops, TraceArgs a, cudaStream_t s) {
     int per_sm = 0;
@@ -324,7 +358,15 @@ static int launch_trace(cor_ctx* ctx, const ModelOps* ops, TraceArgs a, cudaStre
         ctx->gen_t0 = std::chrono::steady_clock::now();
         ctx->gen_live[g] = live;
         ctx->gen_ms[g] = -1.;
-        {
+        if (team_takes(ops, live, cap_blocks)) {
+            // runs to the end: a block whose slots have all ended leaves
+            a.allow_park = 0;
+            int slots = 1;
+            unsigned team_blocks = 1;
+            if ((rc = team_shape(ctx, ops, live, &slots, &team_blocks)) != COR_OK) return rc;
+            NvtxRange r(g == 0 ? "cor: scan by teams" : "cor: scan by teams (regrouped)");
+            CUDA_TRY(ctx, ops->launch_team(a, slots, team_blocks, s));
+        } else {
             NvtxRange r(g == 0 ? "cor: scan generation 0" : "cor: scan generation (regrouped)");
             CUDA_TRY(ctx, ops->launch_generation(a, (unsigned)blocks, s));
         }
@@ -523,9 +565,7 @@ extern "C" int cor_trace_batch_device(cor_ctx* ctx, const cor_scan_job* jobs_dev
     a.n_traj = n_traj;
     a.params = (const DevParams*)ctx->params.p;
     a.step_limit = step_limit;
-    a.tu_angle = tu_angle;
-    a.gc_reject = 0.;
-    a.turn_exact = find_turn_threshold(tu_angle, &a.gc_reject) ? 1 : 0;
+    set_turn_test(a, tu_angle);
     a.rig_major = 0;
     a.n_rig = 0;
     if (n_jobs > 0 && n_traj % (uint64_t)n_jobs == 0) {
@@ -929,9 +969,7 @@ extern "C" int cor_trace_batch_device_noalloc(cor_ctx* ctx, const cor_scan_job* 
     a.n_traj = n_traj;
     a.params = (const DevParams*)ctx->params.p;
     a.step_limit = step_limit;
-    a.tu_angle = tu_angle;
-    a.gc_reject = 0.;
-    a.turn_exact = find_turn_threshold(tu_angle, &a.gc_reject) ? 1 : 0;
+    set_turn_test(a, tu_angle);
     a.n_rig = 0;
     if (n_jobs > 0 && n_traj % (uint64_t)n_jobs == 0) a.n_rig = (uint32_t)(n_traj / (uint64_t)n_jobs);
     a.rig_major = ((flags & COR_FLAG_UNIFORM_GRID) && a.n_rig > 0) ? 1 : 0;
@@ -965,13 +1003,20 @@ extern "C" int cor_trace_batch_device_noalloc(cor_ctx* ctx, const cor_scan_job* 
         CUDA_TRY(ctx, ops->occupancy(&per_sm));
         if (per_sm < 1) per_sm = 1;
         const uint64_t cap = (uint64_t)ctx->sms * (uint64_t)per_sm;
-        const uint64_t warps = (n_traj + 31) / 32;
-        uint64_t blocks = warps < cap ? warps : cap;
-        uint64_t per_block = 32 * ((warps + blocks - 1) / blocks);
-        if (per_block > (uint64_t)kTraceThreads) per_block = kTraceThreads;
-        a.active_threads = (uint32_t)per_block;
-        a.launched_warps = (uint32_t)(blocks * kTraceWarps);
-        CUDA_TRY(ctx, ops->launch_generation(a, (unsigned)blocks, s));
+        if (team_takes(ops, n_traj, cap)) {
+            int slots = 1;
+            unsigned team_blocks = 1;
+            if ((rc = team_shape(ctx, ops, n_traj, &slots, &team_blocks)) != COR_OK) return rc;
+            CUDA_TRY(ctx, ops->launch_team(a, slots, team_blocks, s));
+        } else {
+            const uint64_t warps = (n_traj + 31) / 32;
+            uint64_t blocks = warps < cap ? warps : cap;
+            uint64_t per_block = 32 * ((warps + blocks - 1) / blocks);
+            if (per_block > (uint64_t)kTraceThreads) per_block = kTraceThreads;
+            a.active_threads = (uint32_t)per_block;
+            a.launched_warps = (uint32_t)(blocks * kTraceWarps);
+            CUDA_TRY(ctx, ops->launch_generation(a, (unsigned)blocks, s));
+        }
         launches++;
     }
     if (n_jobs > 0) {
@@ -1220,9 +1265,7 @@ extern "C" int cor_stream_create(cor_ctx* ctx, cor_model_set models, uint64_t st
         memset(&sa, 0, sizeof sa);
         sa.a.params = s->pool_dev;
         sa.a.step_limit = step_limit;
-        sa.a.tu_angle = tu_angle;
-        sa.a.gc_reject = 0.;
-        sa.a.turn_exact = find_turn_threshold(tu_angle, &sa.a.gc_reject) ? 1 : 0;
+        set_turn_test(sa.a, tu_angle);
         sa.a.mass = particle_mass;
         if ((rc = crustal_tables(ctx, models, &sa.a.crust)) != COR_OK) break;
         sa.ctl = s->ctl_d;

@@ -1,6 +1,8 @@
 // inst.cuh -- instantiates the kernels of one model set and its ModelOps.
 #pragma once
 
+#include <cstddef>
+
 #include "model_ops.h"
 
 #define COR_MODEL_INSTANCE(NAME, I, E, C)                                                                  \
@@ -45,6 +47,32 @@
         if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_ts05, ts05, sizeof(TS05Tables));                    \
         return e;                                                                                          \
     }                                                                                                      \
+    template <class MS, bool TEAM = MS::crustal == 0 && MS::external == 0>                                 \
+    struct Team_##NAME {                                                                                   \
+        static cudaError_t occ(int n_slots, int* n) {                                                      \
+            const size_t smem = (size_t)n_slots * sizeof(TeamSlot<MS>);                                    \
+            cudaError_t e = cudaFuncSetAttribute(team_trace_kernel<MS>,                                    \
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+            if (e != cudaSuccess) return e;                                                                \
+            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, team_trace_kernel<MS>, kTeamThreads, smem); \
+        }                                                                                                  \
+        static cudaError_t run(const TraceArgs& a, int n_slots, unsigned blocks, cudaStream_t s) {         \
+            const size_t smem = (size_t)n_slots * sizeof(TeamSlot<MS>);                                    \
+            cudaError_t e = cudaFuncSetAttribute(team_trace_kernel<MS>,                                    \
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+            if (e != cudaSuccess) return e;                                                                \
+            team_trace_kernel<MS><<<blocks, kTeamThreads, smem, s>>>(a, n_slots);                          \
+            return cudaGetLastError();                                                                     \
+        }                                                                                                  \
+        static constexpr auto occ_ptr = &occ;                                                              \
+        static constexpr auto run_ptr = &run;                                                              \
+    };                                                                                                     \
+    template <class MS>                                                                                    \
+    struct Team_##NAME<MS, false> {                                                                        \
+        static constexpr std::nullptr_t occ_ptr = nullptr;                                                 \
+        static constexpr std::nullptr_t run_ptr = nullptr;                                                 \
+    };                                                                                                     \
     const ModelOps ops_##NAME = {I * 100 + E * 10 + C, occ_##NAME, gen_##NAME, field_##NAME, tables_##NAME, \
-                                 socc_##NAME, stream_##NAME};                                               \
+                                 socc_##NAME, stream_##NAME, Team_##NAME<MS_##NAME>::occ_ptr,               \
+                                 Team_##NAME<MS_##NAME>::run_ptr};                                          \
     }

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include "stream.cuh"
+#include "team.cuh"
 
 namespace cor {
 
@@ -21,6 +22,10 @@ struct ModelOps {
     // the persistent stream kernel (stream.cuh)
     cudaError_t (*stream_occupancy)(int* blocks_per_sm);
     cudaError_t (*launch_stream)(const StreamArgs& a, unsigned blocks, cudaStream_t s);
+    // the scan by teams (team.cuh): blocks of n_slots trajectories each; null
+    // for sets without it
+    cudaError_t (*team_occupancy)(int n_slots, int* blocks_per_sm);
+    cudaError_t (*launch_team)(const TraceArgs& a, int n_slots, unsigned blocks, cudaStream_t s);
 };
 
 extern const ModelOps ops_igrf, ops_igrf_t96, ops_t96, ops_igrf_ts05, ops_ts05, ops_crustal;

@@ -1,0 +1,607 @@
+// team.cuh -- block-cooperative trajectory steps: a block of four warps holds
+// a few trajectories ("slots") and spreads every field evaluation over all of
+// its threads.
+//
+// An FP64 warp instruction holds its sub-partition for 64 cycles however many
+// lanes are active, four sub-partitions together retire one per 19 cycles, and
+// instruction-level parallelism gains nothing (measured; the pipe is the
+// bound).  So a scan with fewer trajectories than the GPU has lanes is bound
+// by the number of warp instructions of one trajectory's step, 31 of 32 lanes
+// idle in the limit.  Here
+//   * four neighbouring lanes (a quad) hold one slot's state, replicated; the
+//     three components of the RK step and independent quotients go to
+//     different lanes of the quad;
+//   * the field evaluation is cut into tasks -- independent terms of the same
+//     form (columns and terms of the spherical harmonics, ...) -- that
+//     warps take 32 at a time, tasks of all slots together, so that lanes are
+//     full whatever branches the slots' positions take;
+//   * sums are then taken in the reference's order by one lane per sum.
+// Every operation is the one-lane code's on the same operands, so results do
+// not move by a bit.
+//
+// Measured (IGRF-14): a lone trajectory's accepted step 126 us by one lane,
+// 43 us by a team; one site of 400 rigidities, limit 2,500 steps, 331-507 ms
+// and 109 ms; 8,000 trajectories, limit 1,000 steps, 243 ms and 86 ms.  The
+// step is bound by the quads' trials (about 115 FP64 instructions each, 3.3
+// per step) and the 105-term sums.
+#pragma once
+
+#include "trace.cuh"
+
+namespace cor {
+
+constexpr int kTeamThreads = 128;
+constexpr int kTeamWarps = kTeamThreads / 32;
+constexpr int kTeamSlots = 8;   // at most: one warp's quads (16 slots were no faster)
+constexpr unsigned kFull = 0xffffffffu;
+
+// ---- quad helpers ---------------------------------------------------------
+__device__ __forceinline__ double quad_get(const double v, const int q) {
+    return __shfl_sync(kFull, v, (threadIdx.x & 28) | q);
+}
+
+__device__ __forceinline__ Vec3 quad_gather(const double v) {
+    return {quad_get(v, 0), quad_get(v, 1), quad_get(v, 2)};
+}
+
+// This lane's component of a vector (lanes 0, 1, 2 of a quad; lane 3 repeats z).
+__device__ __forceinline__ double comp(const Vec3 v, const int c) { return c == 0 ? v.x : c == 1 ? v.y : v.z; }
+
+// rk_velocity with one component per lane: stage k's cross product needs the
+// two other components of the stage velocity, which the quad exchanges.
+__device__ __forceinline__ Vec3 quad_rk_velocity(const double h, const double d, const Vec3 f, const Vec3 v,
+                                                 const int c) {
+    const int c1 = c == 2 ? 0 : c + 1, c2 = c == 0 ? 2 : c - 1;
+    const double f1 = comp(f, c1), f2 = comp(f, c2);
+    const double vc = comp(v, c);
+#define CROSS(S1, S2) (h * (d * ((S1)*f2 - (S2)*f1)))
+#define OTHERS(S) const double S##p = quad_get(S, c1), S##q = quad_get(S, c2)
+    const double a1 = CROSS(comp(v, c1), comp(v, c2));
+    const double s2 = vc + DIV3(a1);
+    OTHERS(s2);
+    const double a2 = CROSS(s2p, s2q);
+    const double s3 = vc + DIV25(4. * a1 + 6. * a2);
+    OTHERS(s3);
+    const double a3 = CROSS(s3p, s3q);
+    const double s4 = vc + DIV4(a1 - 12. * a2 + 15. * a3);
+    OTHERS(s4);
+    const double a4 = CROSS(s4p, s4q);
+    const double s5 = vc + DIV81(6. * a1 + 90. * a2 - 50. * a3 + 8. * a4);
+    OTHERS(s5);
+    const double a5 = CROSS(s5p, s5q);
+    const double s6 = vc + DIV75(6. * a1 + 36. * a2 + 10. * a3 + 8. * a4);
+    OTHERS(s6);
+    const double a6 = CROSS(s6p, s6q);
+#undef CROSS
+#undef OTHERS
+    return quad_gather(vc + DIV192(23. * a1 + 125. * a3 - 81. * a5 + 125. * a6));
+}
+
+__device__ __forceinline__ Vec3 quad_rk_position(const double h, const Vec3 v, const Vec3 x, const int c) {
+    return quad_gather(rk_position_1(h, comp(v, c), comp(x, c)));
+}
+
+// t / nk0 for nk0 = nk1 2^k, given r1 = RN(1 / nk1): the quotient by nk1 in
+// three operations, then an exact shift of its exponent, where both are
+// normal numbers (else the division itself).
+__device__ __forceinline__ double gyro_step(const double t, const int nk1, const double r1, const int nk0) {
+    const double h1 = div_r(t, (double)nk1, r1);
+    const int k = __clz(nk1) - __clz(nk0);
+    const int ex = (int)((to_bits(h1) >> 52) & 0x7ff);
+    if ((nk1 << k) == nk0 && ex > k && ex < 0x7ff) return from_bits(to_bits(h1) - ((long long)k << 52));
+    return t / nk0;
+}
+
+// lane_advance for the slots of a warp, one quad each: every lane of the warp
+// calls it, `run` says whether the lane's quad holds a trajectory.  The trial
+// loop runs while any quad of the warp has a trial to make, with the others'
+// lanes computing on without effect.  Returns the class of run lanes' quads.
+__device__ __forceinline__ int quad_advance(Lane& L, const TraceArgs& a, bool run) {
+    const int q = threadIdx.x & 3, c = q == 3 ? 2 : q;
+    const double zn = run ? L.job->zn : 1.;
+    const int nk1 = run ? L.job->nk1 : 1;
+    const cor_model_params* __restrict__ p = run ? &L.par->p : nullptr;
+    // per trajectory and per step what the trials share; h = t / (nk1 2^k) is
+    // the correctly rounded t / nk1 scaled by a power of two
+    const double dq = 1.E-09 * zn * kQ, tb = fabs(zn) * kQ * L.b, r1 = 1. / nk1;
+    int st = 0;
+    while (__any_sync(kFull, run)) {
+        bool trial = run;
+        double h = 0.;
+        Vec3 nv = {0., 0., 0.};
+        while (__any_sync(kFull, trial)) {
+            const double vc = DIVC(L.v);
+            const double hm = a.mass / sqrt(1. - vc * vc);
+            // t and d in one division: lanes 0, 1 and lanes 2, 3
+            const double td = (q < 2 ? 2. * kPi * hm : dq) / (q < 2 ? tb : hm);
+            const double t = quad_get(td, 0), d = quad_get(td, 2);
+            const double hh = gyro_step(t, nk1, r1, L.nk0);
+            const Vec3 n = quad_rk_velocity(hh, d, L.field, L.vel, c);
+            if (trial) {
+                L.step++;
+                if (vc > 1.) {
+                    st = COR_TRAJ_SUPERLUM;
+                    trial = run = false;
+                } else {
+                    const double vprev = L.v;
+                    L.trials++;
+                    L.v = sqrt(n.x * n.x + n.y * n.y + n.z * n.z);
+                    const bool reject =
+                        turn_rejects(a, n.x * L.vel.x + n.y * L.vel.y + n.z * L.vel.z, L.v * vprev);
+                    if (reject && L.nk0 <= 50000) {
+                        L.nk0 *= 2;
+                        L.step--;
+                    } else {
+                        h = hh;
+                        nv = n;
+                        trial = false;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        const Vec3 np = quad_rk_position(h, L.vel, L.pos, c);
+        if (run) {
+            const double rr = sqrt(np.x * np.x + np.y * np.y + np.z * np.z);
+            const Vec3 gsm = geo_to_gsm(np, p);
+            const double pax = div_c(DIVRE(gsm.x) + 25.3, 36.08, 1. / 36.08);
+            const double paz = DIVRE2(gsm.y * gsm.y + gsm.z * gsm.z);
+            const double r = DIVRE(rr);
+            const double paus = pax * pax + div_c(paz, 459.6736, 1. / 459.6736);
+            if (r >= 25. || paus > 1.) {
+                if ((r >= 25. && fabs(r - 25.) < 0.002) || (r <= 25. && paus > 1. && fabs(paus - 1.) < 0.002)) {
+                    L.pos = np;
+                    L.vel = nv;
+                    st = COR_TRAJ_ALLOWED;
+                    run = false;
+                } else if (L.nk0 >= kNk0Cap) {
+                    st = COR_TRAJ_WATCHDOG;
+                    run = false;
+                } else {
+                    L.nk0 *= 2;
+                    L.step--;
+                }
+            } else {
+                const Vec3 prev = L.pos;
+                L.pos = np;
+                L.vel = nv;
+                run = false;
+                if (r < 1.) {
+                    st = COR_TRAJ_REENTRY;
+                } else if ((uint64_t)L.step > a.step_limit) {
+                    st = COR_TRAJ_STEP_LIMIT;
+                } else {
+                    L.gsm = gsm;
+                    L.time = L.time + h;
+                    L.alength += sqrt((np.x - prev.x) * (np.x - prev.x) + (np.y - prev.y) * (np.y - prev.y) +
+                                      (np.z - prev.z) * (np.z - prev.z));
+                    L.nk0 = nk1;
+                }
+            }
+        }
+        __syncwarp();
+    }
+    return st;
+}
+
+// ---- the internal field in tasks ---------------------------------------------
+constexpr int kShTerms = 105;   // (m, n), 1 <= m <= n <= 14, at n(n-1)/2 + m - 1
+constexpr int kShCols = 14;
+
+// What internal_geo keeps in registers, for one slot.
+struct ShSlot {
+    double x, y, z;                      // GEO position [R_E]
+    double R, rho;
+    double C, S, cf, sf, pp;
+    double pw[kShCols], pwn[kShCols];    // R^-(n+1), n R^-(n+1)
+    double cm[kShCols], sm[kShCols];     // cos/sin of (m-1) phi
+    double pmm[kShCols], dmm[kShCols];   // the diagonal
+    double q[kShTerms], z_[kShTerms];    // P(n,m), dP(n,m)
+    double a1[kShTerms], a2[kShTerms], a3[kShTerms];
+    double sum[2 + kShCols];             // br, bt, and each order's share of bf
+    const cor_model_params* p;
+    int K;
+    int pole;
+};
+static_assert(sizeof(ShSlot) / 8 % 2 == 1, "an odd number of 8-byte words: slots start in different banks");
+
+static __device__ const unsigned char c_sh_n[kShTerms] = {
+    1,  2,  2,  3,  3,  3,  4,  4,  4,  4,  5,  5,  5,  5,  5,  6,  6,  6,  6,  6,  6,  7,  7,  7,  7,  7,  7,
+    7,  8,  8,  8,  8,  8,  8,  8,  8,  9,  9,  9,  9,  9,  9,  9,  9,  9,  10, 10, 10, 10, 10, 10, 10, 10, 10,
+    10, 11, 11, 11, 11, 11, 11, 11, 11, 11, 11, 11, 12, 12, 12, 12, 12, 12, 12, 12, 12, 12, 12, 12, 13, 13, 13,
+    13, 13, 13, 13, 13, 13, 13, 13, 13, 13, 14, 14, 14, 14, 14, 14, 14, 14, 14, 14, 14, 14, 14, 14};
+
+// The geometry of a slot, by its quad (all lanes of the warp call; want: the
+// quad's slot is evaluated): the two square roots and the five quotients on
+// different lanes.  A quotient's correctly rounded value does not depend on
+// how it is computed (div_r in internal_geo, a division here).
+__device__ __forceinline__ void quad_sh_geometry(ShSlot& s, const Vec3 x, const cor_model_params* p, const bool want) {
+    const int q = threadIdx.x & 3;
+    const double rho2 = x.x * x.x + x.y * x.y;
+    const double r2 = rho2 + x.z * x.z;
+    const double root = sqrt(q & 1 ? rho2 : r2);
+    const double R = quad_get(root, 0), rho = quad_get(root, 1);
+    const double quo = (q == 0 ? x.z : q == 1 ? rho : q == 2 ? x.x : x.y) / (q < 2 ? R : rho);
+    const double C = quad_get(quo, 0), S = quad_get(quo, 1), cx = quad_get(quo, 2), sx = quad_get(quo, 3);
+    const double pp = 1. / R;
+    if (want && q == 0) {
+        const bool pole = S < 1.E-5;
+        s.x = x.x;
+        s.y = x.y;
+        s.z = x.z;
+        s.R = R;
+        s.rho = rho;
+        s.C = C;
+        s.S = S;
+        s.cf = pole ? 1. : cx;
+        s.sf = pole ? 0. : sx;
+        s.pp = pp;
+        int nm = 3 + 30 / ((int)R + 2);
+        if (nm > 13) nm = 13;
+        s.K = nm + 1;
+        s.pole = pole;
+        s.p = p;
+    }
+}
+
+// Chains that every column starts from, one lane per slot and chain (three
+// kinds of task, taken by different warps).
+__device__ __forceinline__ void sh_powers(ShSlot& s) {
+    const double pp = s.pp;
+    double pr = pp;
+    for (int n = 1; n <= s.K; n++) {
+        pr = pr * pp;
+        s.pw[n - 1] = pr;
+        s.pwn[n - 1] = pr * n;
+    }
+}
+
+__device__ __forceinline__ void sh_rotations(ShSlot& s) {
+    const double cf = s.cf, sf = s.sf;
+    double cm = 0., sm = 1.;
+    for (int m = 1; m <= s.K; m++) {
+        if (m != 1) {
+            const double w = cm;
+            cm = w * cf + sm * sf;
+            sm = sm * cf - w * sf;
+        }
+        s.cm[m - 1] = cm;
+        s.sm[m - 1] = sm;
+    }
+}
+
+__device__ __forceinline__ void sh_diagonal(ShSlot& s) {
+    const double C = s.C, S = s.S;
+    double pmm = 1., dmm = 0.;
+    for (int m = 1; m <= s.K; m++) {
+        s.pmm[m - 1] = pmm;
+        s.dmm[m - 1] = dmm;
+        dmm = S * dmm + C * pmm;
+        pmm = S * pmm;
+    }
+}
+
+// One column (order m - 1) of the Legendre recursion.
+__device__ __forceinline__ void sh_column(ShSlot& s, const int m) {
+    const double C = s.C, S = s.S;
+    const int K = s.K;
+    const double* __restrict__ REC = s.p->rec;
+    double q = s.pmm[m - 1], zz = s.dmm[m - 1], p2 = 0., d2 = 0.;
+    int i = m * (m - 1) / 2 + m - 1;
+    for (int n = m; n <= K; n++) {
+        s.q[i] = q;
+        s.z_[i] = zz;
+        if (n < K) {
+            const double xk = __ldg(&REC[i]);
+            const double dp = C * zz - S * q - xk * d2;
+            const double pm = C * q - xk * p2;
+            d2 = zz;
+            p2 = q;
+            zz = dp;
+            q = pm;
+        }
+        i += n;
+    }
+}
+
+// The factors of term i that multiply P and dP in the three sums.
+__device__ __forceinline__ void sh_term(ShSlot& s, const int i) {
+    const int n = c_sh_n[i], m = i - n * (n - 1) / 2 + 1;
+    const double an = s.pw[n - 1];
+    const double sm = s.sm[m - 1], cm = s.cm[m - 1];
+    const double e = __ldg(&s.p->g[i]);
+    const double hh = __ldg(&s.p->h[i]);
+    const double w = e * sm + hh * cm;
+    s.a1[i] = s.pwn[n - 1] * w;
+    s.a2[i] = -(an * w);
+    s.a3[i] = an * (e * cm - hh * sm);
+}
+
+// Without contraction the sums add rounded products, which are then taken
+// term by term beforehand.
+__device__ __forceinline__ void sh_product(ShSlot& s, const int i) {
+    const double q = s.q[i], z = s.z_[i];
+    s.a1[i] = s.a1[i] * q;
+    s.a2[i] = s.a2[i] * z;
+    s.a3[i] = s.a3[i] * (s.pole ? z : q);
+}
+
+// One of the sums of internal_geo in its order: br (0), bt (1), or the share
+// of order m - 1 in bf (m = 2 .. K).
+template <bool FMA>
+__device__ __forceinline__ void sh_sum(ShSlot& s, const int which) {
+    const int K = s.K;
+    const double* A = which == 0 ? s.a1 : which == 1 ? s.a2 : s.a3;
+    const double* B = which == 1 || (which >= 2 && s.pole) ? s.z_ : s.q;
+    const int m0 = which < 2 ? 1 : which, m1 = which < 2 ? K : which;
+    double acc = 0.;
+    for (int m = m0; m <= m1; m++) {
+        int i = m * (m - 1) / 2 + m - 1;
+        for (int n = m; n <= K; n++) {
+            if constexpr (FMA) acc = acc + A[i] * B[i];
+            else acc = acc + A[i];
+            i += n;
+        }
+    }
+    if constexpr (!FMA)
+        if (which >= 2) acc = acc * (which - 1);
+    s.sum[which] = acc;
+}
+
+// The end of internal_geo, by the quad.
+template <bool FMA>
+__device__ __forceinline__ Vec3 sh_finish(const ShSlot& s) {
+    const double br = s.sum[0], bt = s.sum[1], C = s.C, S = s.S, cf = s.cf, sf = s.sf;
+    double bf = 0., bphi;
+#pragma unroll
+    for (int m = 2; m <= kShCols; m++) {
+        if (m > s.K) break;
+        if constexpr (FMA) bf = bf + s.sum[m] * (m - 1);
+        else bf = bf + s.sum[m];
+    }
+    if (s.pole) {
+        if (C < 0.) bf = -bf;
+        bphi = bf;
+    } else {
+        bphi = bf / S;
+    }
+    const double he = br * S + bt * C;
+    Vec3 b;
+    b.x = he * cf - bphi * sf;
+    b.y = he * sf + bphi * cf;
+    b.z = br * C - bt * S;
+    return b;
+}
+
+// ---- the block's task loop ----------------------------------------------------
+// Shared state of a team block besides the slots.
+struct TeamShared {
+    unsigned next[8];            // chunk counters of the phases
+    unsigned char need[32];      // slots whose field is evaluated in this pass
+};
+
+// The next chunk of the phase, for the whole warp.
+__device__ __forceinline__ unsigned next_chunk(unsigned* ctr) {
+    unsigned c = 0;
+    if ((threadIdx.x & 31) == 0) c = atomicAdd(ctr, 1u);
+    return __shfl_sync(kFull, c, 0);
+}
+
+// The units of sets with an external model are compiled with FMA contraction.
+template <class MS>
+constexpr bool kFma = MS::external != 0;
+
+template <class MS>
+struct TeamSlot {
+    ShSlot sh;
+};
+
+// The field of the slots in `mask` (not 0), from the geometry the quads wrote.
+// All threads of the block; phases are separated by block barriers.
+template <class MS>
+__device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, const unsigned mask) {
+    const int lane = threadIdx.x & 31;
+    const int n = __popc(mask);
+    const unsigned char* list;
+    __shared__ unsigned char s_list[kTeamWarps][32];
+    {
+        unsigned char* mine = s_list[threadIdx.x >> 5];
+        if ((mask >> lane) & 1u) mine[__popc(mask & ((1u << lane) - 1u))] = (unsigned char)lane;
+        __syncwarp();
+        list = mine;
+    }
+    // phase 1: the chains
+    for (;;) {
+        const unsigned ch = next_chunk(&ts.next[0]);
+        if (ch >= 3) break;
+        if (lane < n) {
+            ShSlot& s = slots[list[lane]].sh;
+            if (ch == 0) sh_rotations(s);
+            else if (ch == 1) sh_diagonal(s);
+            else sh_powers(s);
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    // phase 2: the columns, in pairs of complementary length where the
+    // slots fill the warps that way
+    const bool pairs = n > 2;
+    const int cols = pairs ? kShCols / 2 : kShCols;
+    const unsigned col_chunks = (unsigned)(n * cols + 31) / 32;
+    for (;;) {
+        const unsigned ch = next_chunk(&ts.next[1]);
+        if (ch >= col_chunks) break;
+        const int t = (int)ch * 32 + lane;
+        if (t < n * cols) {
+            ShSlot& s = slots[list[t % n]].sh;
+            const int c = t / n, K = s.K;
+            if (pairs) {
+                if (2 * c < K) {
+                    sh_column(s, c + 1);
+                    if (K - 1 - c > c) sh_column(s, K - c);
+                }
+            } else if (c < K) {
+                sh_column(s, c + 1);
+            }
+        }
+        __syncwarp();
+    }
+    // the terms' factors need only the chains
+    const unsigned term_chunks = (unsigned)(n * kShTerms + 31) / 32;
+    for (;;) {
+        const unsigned ch = next_chunk(&ts.next[2]);
+        if (ch >= term_chunks) break;
+        const int t = (int)ch * 32 + lane;
+        if (t < n * kShTerms) {
+            ShSlot& s = slots[list[t % n]].sh;
+            const int i = t / n;
+            if (i < s.K * (s.K + 1) / 2) sh_term(s, i);
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) ts.next[0] = ts.next[1] = ts.next[2] = 0;
+    if constexpr (!kFma<MS>) {
+        for (;;) {
+            const unsigned ch = next_chunk(&ts.next[3]);
+            if (ch >= term_chunks) break;
+            const int t = (int)ch * 32 + lane;
+            if (t < n * kShTerms) {
+                ShSlot& s = slots[list[t % n]].sh;
+                const int i = t / n;
+                if (i < s.K * (s.K + 1) / 2) sh_product(s, i);
+            }
+            __syncwarp();
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) ts.next[3] = 0;
+    }
+    // phase 3: the sums, the two long ones of every slot in one chunk
+    const unsigned sum_chunks = (unsigned)(n * (kShCols - 1) + 31) / 32 + 1;
+    for (;;) {
+        const unsigned ch = next_chunk(&ts.next[4]);
+        if (ch >= sum_chunks) break;
+        if (ch == 0) {
+            if (lane < 2 * n) sh_sum<kFma<MS>>(slots[list[lane >> 1]].sh, lane & 1);
+        } else {
+            const int t = (int)(ch - 1) * 32 + lane;
+            if (t < n * (kShCols - 1)) sh_sum<kFma<MS>>(slots[list[t % n]].sh, 2 + t / n);
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) ts.next[4] = 0;
+}
+
+// The scan by teams: one generation, as trace_kernel's.  `n_slots` (at most
+// kTeamSlots) trajectories per block.
+
+template <class MS>
+__global__ void __launch_bounds__(kTeamThreads) team_trace_kernel(const TraceArgs a, const int n_slots) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    __shared__ TeamShared ts;
+    TeamSlot<MS>* slots = reinterpret_cast<TeamSlot<MS>*>(s_dyn);
+    const int tid = threadIdx.x, slot = tid >> 2, q = tid & 3;
+    if (tid < 8) ts.next[tid] = 0;
+    if (tid < 32) ts.need[tid] = 0;
+    __syncthreads();
+    Lane L;
+    L.v = 0.;
+    L.b = 1.;
+    L.nk0 = 1;
+    L.vel = L.pos = L.field = L.gsm = Vec3{0., 0., 0.};
+    bool has = false, done = slot >= n_slots;
+    unsigned long long n_steps = 0, n_trials = 0, n_traj = 0, n_wd = 0;
+    const bool rig_major = a.rig_major && (!a.grid_ok || *(volatile const unsigned int*)a.grid_ok != 0u);
+    for (;;) {
+        bool need = false;
+        if (__any_sync(kFull, has)) {
+            const int st = quad_advance(L, a, has);
+            if (has) {
+                if (st == 0) {
+                    need = true;
+                    if (a.step_records && L.step <= a.step_cap && q == 0) {
+                        cor_step_record r;
+                        r.gsm[0] = L.gsm.x; r.gsm[1] = L.gsm.y; r.gsm[2] = L.gsm.z;
+                        r.pos[0] = L.pos.x; r.pos[1] = L.pos.y; r.pos[2] = L.pos.z;
+                        r.v = L.v;
+                        r.time = L.time;
+                        r.length = L.alength;
+                        r.step = L.step;
+                        r.reserved = 0;
+                        a.step_records[L.traj * a.step_cap + (L.step - 1)] = r;
+                    }
+                } else {
+                    if (q == 0) {
+                        lane_finish(L, a, st);
+                        n_steps += (st == COR_TRAJ_ALLOWED) ? L.step - 1 : L.step;
+                        n_trials += L.trials;
+                        n_traj += 1;
+                        n_wd += (st == COR_TRAJ_WATCHDOG);
+                    }
+                    has = false;
+                }
+            }
+            __syncwarp();
+        }
+        bool want = !has && !done;
+        if (a.n_restore) {
+            uint64_t r = queue_pop(&a.gen->restore_cursor, want && q == 0);
+            r = __shfl_sync(kFull, (unsigned long long)r, tid & 28);
+            if (want && r < a.n_restore) {
+                need = lane_restore(L, a.restore[r], a.jobs, a.params);
+                has = true;
+                want = false;
+            }
+        }
+        uint64_t t = queue_pop(a.queue, want && q == 0);
+        t = __shfl_sync(kFull, (unsigned long long)t, tid & 28);
+        if (want) {
+            if (t < a.n_traj) {
+                lane_init(L, a, t, rig_major);
+                has = true;
+                need = true;
+            } else {
+                done = true;
+            }
+        }
+        __syncwarp();
+        const bool warp_need = __any_sync(kFull, need);
+        Vec3 pos = {0., 0., 0.};
+        const cor_model_params* p = nullptr;
+        if (warp_need) {
+            Vec3 geo = {1., 0., 0.};
+            if (need) {
+                p = &L.par->p;
+                pos = {DIVRE(L.gsm.x), DIVRE(L.gsm.y), DIVRE(L.gsm.z)};
+                geo = gsm_to_geo(pos, p);
+            }
+            __syncwarp();
+            quad_sh_geometry(slots[slot < n_slots ? slot : 0].sh, geo, p, need);
+        }
+        if (q == 0 && slot < 32) ts.need[slot] = need;
+        if (__syncthreads_and(done)) break;
+        const unsigned mask = __ballot_sync(kFull, ts.need[tid & 31] != 0);
+        if (!mask) {
+            __syncthreads();
+            continue;
+        }
+        team_field<MS>(ts, slots, mask);
+        if (need) {
+            Vec3 tot = {0., 0., 0.};
+            const Vec3 bs = geo_to_gsm(sh_finish<kFma<MS>>(slots[slot].sh), p);
+            tot.x += bs.x;
+            tot.y += bs.y;
+            tot.z += bs.z;
+            L.field = gsm_to_geo(tot, p);
+            L.b = 1.E-09 * sqrt(L.field.x * L.field.x + L.field.y * L.field.y + L.field.z * L.field.z);
+        }
+        __syncwarp();
+    }
+    warp_add_u64(reinterpret_cast<unsigned long long*>(&a.counters->accepted_steps), n_steps);
+    warp_add_u64(reinterpret_cast<unsigned long long*>(&a.counters->trials), n_trials);
+    warp_add_u64(reinterpret_cast<unsigned long long*>(&a.counters->trajectories), n_traj);
+    warp_add_u64(reinterpret_cast<unsigned long long*>(&a.counters->watchdog), n_wd);
+}
+
+}  // namespace cor

@@ -55,6 +55,7 @@ struct TraceArgs {
     uint64_t step_limit;
     double tu_angle;
     double gc_reject;   // turn test: reject iff gc <= gc_reject (exact host-derived threshold)
+    double gc_half;     // half an ulp of gc_reject
     int turn_exact;     // 1: use gc_reject; 0: evaluate atan2 as the reference does
     int rig_major;      // 1: queue index runs over rigidity first (all jobs share n_rig)
     // device word written by grid_check_kernel before the launch: non-zero iff
@@ -211,6 +212,33 @@ __device__ __forceinline__ void lane_init(Lane& L, const TraceArgs& a, uint64_t 
     lane_start(L, a.jobs + j, a.trig[j], a.params + a.jobs[j].param_index, j, i, a.offsets[j] + i, a.mass);
 }
 
+// Turn-angle test, :69-79: reject iff gc < 1 and
+// atan2(sqrt((1-gc)(1+gc)), gc) >= tu_angle, with gc = dot / den rounded.
+// That predicate of the rounded gc is a step function; the host finds its
+// last true value gc_reject with the C library and checks the step, so one
+// comparison gives the reference's decision exactly.  The quotient itself is
+// needed only on the boundary: RN(dot/den) <= gc_reject iff dot/den is below
+// (or, for an even gc_reject, on) the midpoint above it, and
+// e = RN(dot - gc_reject den) compares with the exact den gc_half as the
+// exact difference does unless the two are equal.  Two FP64 instructions
+// instead of a division's nine and a compare; bit patterns order as the
+// values do where den gc_half is positive.
+__device__ __forceinline__ bool turn_rejects(const TraceArgs& a, const double dot, const double den) {
+    if (a.turn_exact) {
+        const double e = __fma_rn(-a.gc_reject, den, dot), m = __dmul_rn(den, a.gc_half);
+        const long long eb = to_bits(e), mb = to_bits(m);
+        const bool plain = (eb & 0x7fffffffffffffffll) < 0x7ff0000000000000ll && mb > 0 && mb < 0x7ff0000000000000ll &&
+                           eb != mb;
+        return plain ? eb < mb : dot / den <= a.gc_reject;
+    }
+    const double gc = dot / den;
+    if (gc < 1.) {
+        const double gs = sqrt((1. - gc) * (1. + gc));
+        return atan2(gs, gc) >= a.tu_angle;
+    }
+    return false;
+}
+
 // Advances one lane to its next accepted step (returns 0) or to its
 // termination (returns the COR_TRAJ_* class).  src/trajectory.c:45-152,
 // with the field evaluation left to the caller.  Bounded: at most 10
@@ -221,7 +249,7 @@ __device__ __forceinline__ int lane_advance(Lane& L, const TraceArgs& a) {
     const int nk1 = L.job->nk1;
     for (;;) {
         L.step++;
-        const double vc = div_c(L.v, kC, 1. / kC);
+        const double vc = DIVC(L.v);
         if (vc > 1.) return COR_TRAJ_SUPERLUM;  // :48-54
         const double hm = a.mass / sqrt(1. - vc * vc);
         const double t = (2. * kPi * hm) / (fabs(zn) * kQ * L.b);
@@ -231,22 +259,7 @@ __device__ __forceinline__ int lane_advance(Lane& L, const TraceArgs& a) {
         const Vec3 nv = rk_velocity(h, d, L.field, L.vel);
         L.trials++;
         L.v = sqrt(nv.x * nv.x + nv.y * nv.y + nv.z * nv.z);
-        const double gc = (nv.x * L.vel.x + nv.y * L.vel.y + nv.z * L.vel.z) / (L.v * vprev);
-        // Turn-angle test, :69-79: reject iff gc < 1 and
-        // atan2(sqrt((1-gc)(1+gc)), gc) >= tu_angle.  That predicate of the
-        // rounded gc is a step function; the host finds its last true value
-        // with the C library and checks the step, so one comparison gives
-        // the reference's decision exactly.
-        bool reject;
-        if (a.turn_exact) {
-            reject = gc <= a.gc_reject;
-        } else {
-            reject = false;
-            if (gc < 1.) {
-                const double gs = sqrt((1. - gc) * (1. + gc));
-                reject = atan2(gs, gc) >= a.tu_angle;
-            }
-        }
+        const bool reject = turn_rejects(a, nv.x * L.vel.x + nv.y * L.vel.y + nv.z * L.vel.z, L.v * vprev);
         if (reject && L.nk0 <= 50000) {
             L.nk0 *= 2;
             L.step--;
@@ -256,7 +269,7 @@ __device__ __forceinline__ int lane_advance(Lane& L, const TraceArgs& a) {
         const double rr = sqrt(np.x * np.x + np.y * np.y + np.z * np.z);  // car_to_sph radius
         const Vec3 gsm = geo_to_gsm(np, &L.par->p);
         const double pax = div_c(DIVRE(gsm.x) + 25.3, 36.08, 1. / 36.08);
-        const double paz = div_c(gsm.y * gsm.y + gsm.z * gsm.z, kRe * kRe, 1. / (kRe * kRe));
+        const double paz = DIVRE2(gsm.y * gsm.y + gsm.z * gsm.z);
         const double r = DIVRE(rr);
         const double paus = pax * pax + div_c(paz, 459.6736, 1. / 459.6736);
         if (r >= 25. || paus > 1.) {  // :89-131
