@@ -304,9 +304,20 @@ static const ModelOps* find_ops(const cor_model_set& m) {
 // the longest; above it their throughput is the higher one.  IGRF-14, ms by
 // lanes / by teams: 400 trajectories 331 / 109, 8,000 243 / 86, 20,000
 // 286 / 178, 40,000 375 / 325 (291 when the teams take over at half the
-// lanes), 91,200 562 / 666 (487).
+// lanes), 91,200 562 / 666 (487).  With T96, limit 1,000 steps: 400
+// trajectories 432 / 63, 2,000 484 / 92; limit 250: 8,000 103 / 110, 20,000
+// 291 / 187, 66,000 (the tail by teams) 629 / 497.
 static bool team_takes(const ModelOps* ops, uint64_t live, uint64_t cap_blocks) {
     return ops->launch_team && 2 * live <= cap_blocks * (uint64_t)kTraceThreads;
+}
+
+// The same for a field batch of n points, where every lane does the same
+// amount of work: up to a sixth of the lanes.  T96, us by lanes / by teams
+// (the call's allocations and copies included): 1 point 403 / 114, 1,000
+// 614 / 184, 5,000 625 / 433, 8,000 639 / 736; IGRF-14: 1 116 / 83, 2,664
+// 177 / 127, 8,000 177 / 184.
+static bool team_takes_field(const ModelOps* ops, uint64_t n, int sms) {
+    return ops->launch_team_field && 6 * n <= (uint64_t)sms * (uint64_t)kTraceThreads;
 }
 
 // Slots per block and blocks of a team launch: as many blocks as are resident
@@ -719,8 +730,17 @@ extern "C" int cor_field_batch(cor_ctx* ctx, cor_model_set models, const cor_mod
         if (param_index) cudaMemcpyAsync(didx, param_index, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, s);
         CrustalTables crust;
         if ((rc = crustal_tables(ctx, models, &crust)) != COR_OK) break;
-        find_ops(models)->launch_field((const DevParams*)dp, n_params, (const int32_t*)didx, (const double*)dpos, n,
-                                       (double*)dout, crust, s);
+        const ModelOps* ops = find_ops(models);
+        int slots = 1;
+        unsigned blocks = 1;
+        if (team_takes_field(ops, (uint64_t)n, ctx->sms)) {
+            if ((rc = team_shape(ctx, ops, (uint64_t)n, &slots, &blocks)) != COR_OK) break;
+            ops->launch_team_field((const DevParams*)dp, n_params, (const int32_t*)didx, (const double*)dpos, n,
+                                   (double*)dout, slots, blocks, s);
+        } else {
+            ops->launch_field((const DevParams*)dp, n_params, (const int32_t*)didx, (const double*)dpos, n,
+                              (double*)dout, crust, s);
+        }
         cudaMemcpyAsync(geo_field, dout, sizeof(double) * 3 * (size_t)n, cudaMemcpyDeviceToHost, s);
         cudaError_t e = cudaStreamSynchronize(s);
         if (e == cudaSuccess) e = cudaGetLastError();

@@ -44,10 +44,11 @@
     }                                                                                                      \
     static cudaError_t tables_##NAME(const T96Tables* t96, const TS05Tables* ts05) {                       \
         cudaError_t e = cudaMemcpyToSymbol(c_t96, t96, sizeof(T96Tables));                                 \
+        if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_t96, t96, sizeof(T96Tables));                       \
         if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_ts05, ts05, sizeof(TS05Tables));                    \
         return e;                                                                                          \
     }                                                                                                      \
-    template <class MS, bool TEAM = MS::crustal == 0 && MS::external == 0>                                 \
+    template <class MS, bool TEAM = MS::crustal == 0 && MS::external != COR_EXTERNAL_TS05>                 \
     struct Team_##NAME {                                                                                   \
         static cudaError_t occ(int n_slots, int* n) {                                                      \
             const size_t smem = (size_t)n_slots * sizeof(TeamSlot<MS>);                                    \
@@ -64,15 +65,26 @@
             team_trace_kernel<MS><<<blocks, kTeamThreads, smem, s>>>(a, n_slots);                          \
             return cudaGetLastError();                                                                     \
         }                                                                                                  \
+        static cudaError_t field(const DevParams* p, int np, const int32_t* idx, const double* pos, int64_t n, \
+                                 double* out, int n_slots, unsigned blocks, cudaStream_t s) {              \
+            const size_t smem = (size_t)n_slots * sizeof(TeamSlot<MS>);                                    \
+            cudaError_t e = cudaFuncSetAttribute(team_field_kernel<MS>,                                    \
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+            if (e != cudaSuccess) return e;                                                                \
+            team_field_kernel<MS><<<blocks, kTeamThreads, smem, s>>>(p, np, idx, pos, n, out, n_slots);    \
+            return cudaGetLastError();                                                                     \
+        }                                                                                                  \
         static constexpr auto occ_ptr = &occ;                                                              \
+        static constexpr auto field_ptr = &field;                                                          \
         static constexpr auto run_ptr = &run;                                                              \
     };                                                                                                     \
     template <class MS>                                                                                    \
     struct Team_##NAME<MS, false> {                                                                        \
         static constexpr std::nullptr_t occ_ptr = nullptr;                                                 \
         static constexpr std::nullptr_t run_ptr = nullptr;                                                 \
+        static constexpr std::nullptr_t field_ptr = nullptr;                                               \
     };                                                                                                     \
     const ModelOps ops_##NAME = {I * 100 + E * 10 + C, occ_##NAME, gen_##NAME, field_##NAME, tables_##NAME, \
                                  socc_##NAME, stream_##NAME, Team_##NAME<MS_##NAME>::occ_ptr,               \
-                                 Team_##NAME<MS_##NAME>::run_ptr};                                          \
+                                 Team_##NAME<MS_##NAME>::run_ptr, Team_##NAME<MS_##NAME>::field_ptr};       \
     }

@@ -26,6 +26,9 @@ struct ModelOps {
     // for sets without it
     cudaError_t (*team_occupancy)(int n_slots, int* blocks_per_sm);
     cudaError_t (*launch_team)(const TraceArgs& a, int n_slots, unsigned blocks, cudaStream_t s);
+    // launch_field by teams
+    cudaError_t (*launch_team_field)(const DevParams* params, int n_params, const int32_t* pidx, const double* pos,
+                                     int64_t n, double* out, int n_slots, unsigned blocks, cudaStream_t s);
 };
 
 extern const ModelOps ops_igrf, ops_igrf_t96, ops_t96, ops_igrf_ts05, ops_ts05, ops_crustal;

@@ -275,6 +275,7 @@ static __device__ __noinline__ Vec3 t96_taildisk(const double x, const double y,
 // tail87, :445-498: three line currents (z, z-40, z+40) with the same form.
 struct T87Line {
     double s0, s1, s2, g1, g2, xln1;
+    double xa2;
 };
 
 __device__ __forceinline__ T87Line t96_tail87_line(const double b2, const double xnx, const double xnx2, const double xc1,
@@ -296,6 +297,7 @@ __device__ __forceinline__ T87Line t96_tail87_line(const double b2, const double
     o.s2 = (xc2 * xa2 * xln2 + 0.1071 - f * xa2 * s0) * xa2;
     o.g1 = div_r(b2 * s0 - 0.5 * xc1 * xln1, xa1, rxa1);
     o.g2 = ((0.5 * f * xln2 + 2. * s0 * b2 * xc2) * xa2 + xr2) * xa2;
+    o.xa2 = xa2;
     o.xln1 = xln1;
     return o;
 }
@@ -828,42 +830,51 @@ static __device__ __noinline__ Vec3 t96_r2outer(const double x, const double y, 
 #define T96_POW5(u) ((u) * (u) * (u) * (u) * (u))
 #endif
 
+// The Region-2 sheet's harmonics (r2sheet, :1481-1512) by component: [l][m] of
+// {1, t1, t2, t3}.
+#define T96_SHEET_X                                                                     \
+    {                                                                                   \
+    {{8.07190, -7.39582, -7.62341, 0.684671}, {-13.5672, 11.6681, 13.1154, -0.890217},  \
+    {7.78726, -5.38346, -8.08738, 0.609385}, {-2.70410, 3.53741, 3.15549, -1.11069}},   \
+    {{-8.47555, 0.278122, 2.73514, 4.55625}, {13.1134, 1.15848, -3.52648, -8.24698},    \
+    {-6.85710, -2.81369, 2.03795, 4.64383}, {2.49309, -1.22041, -1.67432, -0.422526}},  \
+    {{-5.39796, 7.10326, 5.53730, -13.1918}, {4.67853, -7.60329, -2.53066, 7.76338},    \
+    {5.60165, 5.34816, -4.56441, 7.05976}, {-2.62723, -0.529078, 1.42019, -2.93919}},   \
+    {{55.6338, -1.55181, 39.8311, -80.6561}, {-46.9655, 32.8925, -6.32296, 19.7841},    \
+    {124.731, 10.4347, -30.7581, 102.680}, {-47.4037, -3.31278, 9.37141, -50.0268}},    \
+    {{-533.319, 110.426, 1000.20, -1051.40}, {1619.48, 589.855, -1462.73, 1087.10},     \
+    {-1994.73, -1654.12, 1263.33, -260.210}, {1424.84, 1255.71, -956.733, 219.946}}}
+#define T96_SHEET_Y                                                                       \
+    {                                                                                     \
+    {{-9.08427, 10.6777, 10.3288, -0.969987}, {6.45257, -8.42508, -7.97464, 1.41996},     \
+    {-1.92490, 3.93575, 2.83283, -1.48621}, {0.244033, -0.757941, -0.386557, 0.344566}},  \
+    {{9.56674, -2.5365, -3.32916, -5.86712}, {-6.19625, 1.83879, 2.52772, 4.34417},       \
+    {1.87268, -2.13213, -1.69134, -0.176379}, {-0.261359, 0.566419, 0.3138, -0.134699}},  \
+    {{-3.83086, -8.4154, 4.77005, -9.31479}, {37.5715, 19.3992, -17.9582, 36.4604},       \
+    {-14.9993, -3.1442, 6.17409, -15.5519}, {2.28621, -0.00891549, -0.462912, 2.47314}},  \
+    {{41.7555, 208.614, -45.7861, -77.8687}, {239.357, -67.9226, 66.8743, 238.534},       \
+    {-112.136, 16.2069, -40.4706, -134.328}, {21.56, -0.201725, 2.21, 32.5855}},          \
+    {{-108.217, -1005.98, 585.753, 323.668}, {-817.056, 235.750, -560.965, -576.892},     \
+    {684.193, 85.0275, 168.394, 477.776}, {-289.253, -123.216, 75.6501, -178.605}}}
+#define T96_SHEET_Z                                                                           \
+    {                                                                                         \
+    {{1167.61, -917.782, -1253.2, -274.128}, {-1538.75, 1257.62, 1745.07, 113.479},           \
+    {393.326, -426.858, -641.1, 190.833}, {-29.9435, -1.04881, 117.125, -25.7663}},           \
+    {{-1168.16, 910.247, 1239.31, 289.515}, {1540.56, -1248.29, -1727.61, -131.785},          \
+    {-394.577, 426.163, 637.422, -187.965}, {30.0348, 0.221898, -116.68, 26.0291}},           \
+    {{12.6804, 4.84091, 1.18166, -2.75946}, {-17.9822, -6.80357, -1.47134, 3.02266},          \
+    {4.79648, 0.665255, -0.256229, -0.0857282}, {-0.588997, 0.0634812, 0.164303, -0.15285}},  \
+    {{22.2524, -22.4376, -3.85595, 6.07625}, {-105.959, -41.6698, 0.378615, 1.55958},         \
+    {44.3981, 18.8521, 3.19466, 5.89142}, {-8.63227, -2.36418, -1.027, -2.31515}},            \
+    {{1035.38, 2040.66, -131.881, -744.533}, {-3274.93, -4845.61, 482.438, 1567.43},          \
+    {1354.02, 2040.47, -151.653, -845.012}, {-111.723, -265.343, -26.1171, 216.632}}}
+
 // r2sheet, :1472-1586, with xksi passed in (the reference evaluates the same
 // xksi(X, Y, Z) again).
 static __device__ __noinline__ Vec3 t96_r2sheet(const double x, const double y, const double z, const double xks) {
-    constexpr double CX[5][4][4] = {
-        {{8.07190, -7.39582, -7.62341, 0.684671}, {-13.5672, 11.6681, 13.1154, -0.890217},
-         {7.78726, -5.38346, -8.08738, 0.609385}, {-2.70410, 3.53741, 3.15549, -1.11069}},
-        {{-8.47555, 0.278122, 2.73514, 4.55625}, {13.1134, 1.15848, -3.52648, -8.24698},
-         {-6.85710, -2.81369, 2.03795, 4.64383}, {2.49309, -1.22041, -1.67432, -0.422526}},
-        {{-5.39796, 7.10326, 5.53730, -13.1918}, {4.67853, -7.60329, -2.53066, 7.76338},
-         {5.60165, 5.34816, -4.56441, 7.05976}, {-2.62723, -0.529078, 1.42019, -2.93919}},
-        {{55.6338, -1.55181, 39.8311, -80.6561}, {-46.9655, 32.8925, -6.32296, 19.7841},
-         {124.731, 10.4347, -30.7581, 102.680}, {-47.4037, -3.31278, 9.37141, -50.0268}},
-        {{-533.319, 110.426, 1000.20, -1051.40}, {1619.48, 589.855, -1462.73, 1087.10},
-         {-1994.73, -1654.12, 1263.33, -260.210}, {1424.84, 1255.71, -956.733, 219.946}}};
-    constexpr double CY[5][4][4] = {
-        {{-9.08427, 10.6777, 10.3288, -0.969987}, {6.45257, -8.42508, -7.97464, 1.41996},
-         {-1.92490, 3.93575, 2.83283, -1.48621}, {0.244033, -0.757941, -0.386557, 0.344566}},
-        {{9.56674, -2.5365, -3.32916, -5.86712}, {-6.19625, 1.83879, 2.52772, 4.34417},
-         {1.87268, -2.13213, -1.69134, -0.176379}, {-0.261359, 0.566419, 0.3138, -0.134699}},
-        {{-3.83086, -8.4154, 4.77005, -9.31479}, {37.5715, 19.3992, -17.9582, 36.4604},
-         {-14.9993, -3.1442, 6.17409, -15.5519}, {2.28621, -0.00891549, -0.462912, 2.47314}},
-        {{41.7555, 208.614, -45.7861, -77.8687}, {239.357, -67.9226, 66.8743, 238.534},
-         {-112.136, 16.2069, -40.4706, -134.328}, {21.56, -0.201725, 2.21, 32.5855}},
-        {{-108.217, -1005.98, 585.753, 323.668}, {-817.056, 235.750, -560.965, -576.892},
-         {684.193, 85.0275, 168.394, 477.776}, {-289.253, -123.216, 75.6501, -178.605}}};
-    constexpr double CZ[5][4][4] = {
-        {{1167.61, -917.782, -1253.2, -274.128}, {-1538.75, 1257.62, 1745.07, 113.479},
-         {393.326, -426.858, -641.1, 190.833}, {-29.9435, -1.04881, 117.125, -25.7663}},
-        {{-1168.16, 910.247, 1239.31, 289.515}, {1540.56, -1248.29, -1727.61, -131.785},
-         {-394.577, 426.163, 637.422, -187.965}, {30.0348, 0.221898, -116.68, 26.0291}},
-        {{12.6804, 4.84091, 1.18166, -2.75946}, {-17.9822, -6.80357, -1.47134, 3.02266},
-         {4.79648, 0.665255, -0.256229, -0.0857282}, {-0.588997, 0.0634812, 0.164303, -0.15285}},
-        {{22.2524, -22.4376, -3.85595, 6.07625}, {-105.959, -41.6698, 0.378615, 1.55958},
-         {44.3981, 18.8521, 3.19466, 5.89142}, {-8.63227, -2.36418, -1.027, -2.31515}},
-        {{1035.38, 2040.66, -131.881, -744.533}, {-3274.93, -4845.61, 482.438, 1567.43},
-         {1354.02, 2040.47, -151.653, -845.012}, {-111.723, -265.343, -26.1171, 216.632}}};
+    constexpr double CX[5][4][4] = T96_SHEET_X;
+    constexpr double CY[5][4][4] = T96_SHEET_Y;
+    constexpr double CZ[5][4][4] = T96_SHEET_Z;
     const double xks2 = xks * xks;
     const double t1x = xks / sqrt(xks2 + 0.483750e-01 * 0.483750e-01);
     const double px72 = 0.396953e-01 * 0.396953e-01;

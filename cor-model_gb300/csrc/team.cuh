@@ -26,7 +26,16 @@
 // per step) and the 105-term sums.
 #pragma once
 
+#include <type_traits>
+
 #include "trace.cuh"
+
+namespace cor {
+// One component of a vector by number.
+__device__ __forceinline__ double comp(const Vec3 v, const int c) { return c == 0 ? v.x : c == 1 ? v.y : v.z; }
+}  // namespace cor
+
+#include "team_t96.cuh"
 
 namespace cor {
 
@@ -43,9 +52,6 @@ __device__ __forceinline__ double quad_get(const double v, const int q) {
 __device__ __forceinline__ Vec3 quad_gather(const double v) {
     return {quad_get(v, 0), quad_get(v, 1), quad_get(v, 2)};
 }
-
-// This lane's component of a vector (lanes 0, 1, 2 of a quad; lane 3 repeats z).
-__device__ __forceinline__ double comp(const Vec3 v, const int c) { return c == 0 ? v.x : c == 1 ? v.y : v.z; }
 
 // rk_velocity with one component per lane: stage k's cross product needs the
 // two other components of the stage velocity, which the quad exchanges.
@@ -203,7 +209,6 @@ struct ShSlot {
     int K;
     int pole;
 };
-static_assert(sizeof(ShSlot) / 8 % 2 == 1, "an odd number of 8-byte words: slots start in different banks");
 
 static __device__ const unsigned char c_sh_n[kShTerms] = {
     1,  2,  2,  3,  3,  3,  4,  4,  4,  4,  5,  5,  5,  5,  5,  6,  6,  6,  6,  6,  6,  7,  7,  7,  7,  7,  7,
@@ -244,6 +249,12 @@ __device__ __forceinline__ void quad_sh_geometry(ShSlot& s, const Vec3 x, const 
     }
 }
 
+// a b + c, with one rounding where internal_geo's is contracted.
+template <bool FMA>
+__device__ __forceinline__ double sh_mad(const double a, const double b, const double c) {
+    return FMA ? __fma_rn(a, b, c) : __dadd_rn(__dmul_rn(a, b), c);
+}
+
 // Chains that every column starts from, one lane per slot and chain (three
 // kinds of task, taken by different warps).
 __device__ __forceinline__ void sh_powers(ShSlot& s) {
@@ -256,32 +267,35 @@ __device__ __forceinline__ void sh_powers(ShSlot& s) {
     }
 }
 
+template <bool FMA>
 __device__ __forceinline__ void sh_rotations(ShSlot& s) {
     const double cf = s.cf, sf = s.sf;
     double cm = 0., sm = 1.;
     for (int m = 1; m <= s.K; m++) {
         if (m != 1) {
             const double w = cm;
-            cm = w * cf + sm * sf;
-            sm = sm * cf - w * sf;
+            cm = sh_mad<FMA>(w, cf, __dmul_rn(sm, sf));
+            sm = sh_mad<FMA>(sm, cf, -__dmul_rn(w, sf));
         }
         s.cm[m - 1] = cm;
         s.sm[m - 1] = sm;
     }
 }
 
+template <bool FMA>
 __device__ __forceinline__ void sh_diagonal(ShSlot& s) {
     const double C = s.C, S = s.S;
     double pmm = 1., dmm = 0.;
     for (int m = 1; m <= s.K; m++) {
         s.pmm[m - 1] = pmm;
         s.dmm[m - 1] = dmm;
-        dmm = S * dmm + C * pmm;
+        dmm = sh_mad<FMA>(C, pmm, __dmul_rn(S, dmm));
         pmm = S * pmm;
     }
 }
 
 // One column (order m - 1) of the Legendre recursion.
+template <bool FMA>
 __device__ __forceinline__ void sh_column(ShSlot& s, const int m) {
     const double C = s.C, S = s.S;
     const int K = s.K;
@@ -293,8 +307,8 @@ __device__ __forceinline__ void sh_column(ShSlot& s, const int m) {
         s.z_[i] = zz;
         if (n < K) {
             const double xk = __ldg(&REC[i]);
-            const double dp = C * zz - S * q - xk * d2;
-            const double pm = C * q - xk * p2;
+            const double dp = sh_mad<FMA>(-xk, d2, sh_mad<FMA>(C, zz, -__dmul_rn(S, q)));
+            const double pm = sh_mad<FMA>(C, q, -__dmul_rn(xk, p2));
             d2 = zz;
             p2 = q;
             zz = dp;
@@ -305,16 +319,17 @@ __device__ __forceinline__ void sh_column(ShSlot& s, const int m) {
 }
 
 // The factors of term i that multiply P and dP in the three sums.
+template <bool FMA>
 __device__ __forceinline__ void sh_term(ShSlot& s, const int i) {
     const int n = c_sh_n[i], m = i - n * (n - 1) / 2 + 1;
     const double an = s.pw[n - 1];
     const double sm = s.sm[m - 1], cm = s.cm[m - 1];
     const double e = __ldg(&s.p->g[i]);
     const double hh = __ldg(&s.p->h[i]);
-    const double w = e * sm + hh * cm;
+    const double w = sh_mad<FMA>(e, sm, __dmul_rn(hh, cm));
     s.a1[i] = s.pwn[n - 1] * w;
     s.a2[i] = -(an * w);
-    s.a3[i] = an * (e * cm - hh * sm);
+    s.a3[i] = an * sh_mad<FMA>(e, cm, -__dmul_rn(hh, sm));
 }
 
 // Without contraction the sums add rounded products, which are then taken
@@ -338,13 +353,11 @@ __device__ __forceinline__ void sh_sum(ShSlot& s, const int which) {
     for (int m = m0; m <= m1; m++) {
         int i = m * (m - 1) / 2 + m - 1;
         for (int n = m; n <= K; n++) {
-            if constexpr (FMA) acc = acc + A[i] * B[i];
-            else acc = acc + A[i];
+            acc = FMA ? __fma_rn(A[i], B[i], acc) : __dadd_rn(acc, A[i]);
             i += n;
         }
     }
-    if constexpr (!FMA)
-        if (which >= 2) acc = acc * (which - 1);
+    if (which >= 2) acc = __dmul_rn(acc, which - 1);   // rounded before it is added, in both kinds of unit
     s.sum[which] = acc;
 }
 
@@ -356,8 +369,7 @@ __device__ __forceinline__ Vec3 sh_finish(const ShSlot& s) {
 #pragma unroll
     for (int m = 2; m <= kShCols; m++) {
         if (m > s.K) break;
-        if constexpr (FMA) bf = bf + s.sum[m] * (m - 1);
-        else bf = bf + s.sum[m];
+        bf = bf + s.sum[m];
     }
     if (s.pole) {
         if (C < 0.) bf = -bf;
@@ -365,20 +377,29 @@ __device__ __forceinline__ Vec3 sh_finish(const ShSlot& s) {
     } else {
         bphi = bf / S;
     }
-    const double he = br * S + bt * C;
+    const double he = sh_mad<FMA>(br, S, __dmul_rn(bt, C));
     Vec3 b;
-    b.x = he * cf - bphi * sf;
-    b.y = he * sf + bphi * cf;
-    b.z = br * C - bt * S;
+    b.x = sh_mad<FMA>(he, cf, -__dmul_rn(bphi, sf));
+    b.y = sh_mad<FMA>(he, sf, __dmul_rn(bphi, cf));
+    b.z = sh_mad<FMA>(br, C, -__dmul_rn(bt, S));
     return b;
 }
 
 // ---- the block's task loop ----------------------------------------------------
 // Shared state of a team block besides the slots.
 struct TeamShared {
-    unsigned next[8];            // chunk counters of the phases
-    unsigned char need[32];      // slots whose field is evaluated in this pass
+    unsigned next[4];                       // chunk counters of the phases
+    unsigned char need[32];                 // slots whose field is evaluated in this pass
+    unsigned char list[kTeamWarps][6][32];  // slots by kind of task, one copy per warp
 };
+
+// The slots set in `mask` as this warp's list k.
+__device__ __forceinline__ const unsigned char* team_list(TeamShared& ts, const int k, const unsigned mask) {
+    const int lane = threadIdx.x & 31;
+    unsigned char* l = ts.list[threadIdx.x >> 5][k];
+    if ((mask >> lane) & 1u) l[__popc(mask & ((1u << lane) - 1u))] = (unsigned char)lane;
+    return l;
+}
 
 // The next chunk of the phase, for the whole warp.
 __device__ __forceinline__ unsigned next_chunk(unsigned* ctr) {
@@ -387,84 +408,196 @@ __device__ __forceinline__ unsigned next_chunk(unsigned* ctr) {
     return __shfl_sync(kFull, c, 0);
 }
 
+// Whether the phase's chunk ch is one of the next n; if not, ch counts on
+// from there.
+__device__ __forceinline__ bool takes(unsigned& ch, const unsigned n) {
+    if (ch < n) return true;
+    ch -= n;
+    return false;
+}
+
+__device__ __forceinline__ unsigned chunks(const int tasks) { return (unsigned)(tasks + 31) >> 5; }
+
 // The units of sets with an external model are compiled with FMA contraction.
 template <class MS>
 constexpr bool kFma = MS::external != 0;
 
+struct NoSlot {};
 template <class MS>
-struct TeamSlot {
-    ShSlot sh;
+struct TeamSlotBody {
+    std::conditional_t<MS::internal != 0, ShSlot, NoSlot> sh;
+    std::conditional_t<MS::external == COR_EXTERNAL_T96, T96Slot, NoSlot> t96;
+};
+// An odd number of 8-byte words, so that slots start in different banks.
+template <class MS>
+struct TeamSlot : TeamSlotBody<MS> {
+    double pad[1 + (sizeof(TeamSlotBody<MS>) / 8) % 2];
 };
 
-// The field of the slots in `mask` (not 0), from the geometry the quads wrote.
-// All threads of the block; phases are separated by block barriers.
+// The field of the slots in `mask` (not 0), from what the quads wrote.  All
+// threads of the block; the phases are separated by block barriers, and
+// within one the warps take chunks of 32 tasks, the longest kinds first.
 template <class MS>
 __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, const unsigned mask) {
+    constexpr bool kSh = MS::internal != 0, kT96 = MS::external == COR_EXTERNAL_T96;
     const int lane = threadIdx.x & 31;
     const int n = __popc(mask);
-    const unsigned char* list;
-    __shared__ unsigned char s_list[kTeamWarps][32];
-    {
-        unsigned char* mine = s_list[threadIdx.x >> 5];
-        if ((mask >> lane) & 1u) mine[__popc(mask & ((1u << lane) - 1u))] = (unsigned char)lane;
-        __syncwarp();
-        list = mine;
-    }
-    // phase 1: the chains
+    const unsigned char* list = team_list(ts, 0, mask);
+    __syncwarp();
+    // phase 1
     for (;;) {
-        const unsigned ch = next_chunk(&ts.next[0]);
-        if (ch >= 3) break;
-        if (lane < n) {
-            ShSlot& s = slots[list[lane]].sh;
-            if (ch == 0) sh_rotations(s);
-            else if (ch == 1) sh_diagonal(s);
-            else sh_powers(s);
+        unsigned ch = next_chunk(&ts.next[0]);
+        bool any = false;
+        if constexpr (kT96) {
+            any = true;
+            if (takes(ch, 1)) {
+                if (lane < n) t96_task_b1(slots[list[lane]].t96);
+            } else if (takes(ch, chunks(6 * n))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 6 * n) t96_task_rt(slots[list[t % n]].t96, t / n);
+            } else if (takes(ch, chunks(6 * n))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 6 * n) t96_task_bes(slots[list[t % n]].t96, t / n);
+            } else if (takes(ch, chunks(3 * n))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 3 * n) t96_task_t87(slots[list[t % n]].t96, t / n);
+            } else if (takes(ch, 1)) {
+                if (lane < n) t96_task_xksi(slots[list[lane]].t96);
+            } else if (takes(ch, 1)) {
+                if (lane < n) t96_task_main(slots[list[lane]].t96);
+            } else if (takes(ch, chunks(kT96Sc * n))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < kT96Sc * n) t96_task_sc(slots[list[t % n]].t96, t / n);
+            } else {
+                any = false;
+            }
         }
-        __syncwarp();
-    }
-    __syncthreads();
-    // phase 2: the columns, in pairs of complementary length where the
-    // slots fill the warps that way
-    const bool pairs = n > 2;
-    const int cols = pairs ? kShCols / 2 : kShCols;
-    const unsigned col_chunks = (unsigned)(n * cols + 31) / 32;
-    for (;;) {
-        const unsigned ch = next_chunk(&ts.next[1]);
-        if (ch >= col_chunks) break;
-        const int t = (int)ch * 32 + lane;
-        if (t < n * cols) {
-            ShSlot& s = slots[list[t % n]].sh;
-            const int c = t / n, K = s.K;
-            if (pairs) {
-                if (2 * c < K) {
-                    sh_column(s, c + 1);
-                    if (K - 1 - c > c) sh_column(s, K - c);
+        if constexpr (kSh) {
+            if (!any) {
+                any = true;
+                if (ch < 3) {
+                    if (lane < n) {
+                        ShSlot& s = slots[list[lane]].sh;
+                        if (ch == 0) sh_rotations<kFma<MS>>(s);
+                        else if (ch == 1) sh_diagonal<kFma<MS>>(s);
+                        else sh_powers(s);
+                    }
+                } else {
+                    any = false;
                 }
-            } else if (c < K) {
-                sh_column(s, c + 1);
             }
         }
         __syncwarp();
-    }
-    // the terms' factors need only the chains
-    const unsigned term_chunks = (unsigned)(n * kShTerms + 31) / 32;
-    for (;;) {
-        const unsigned ch = next_chunk(&ts.next[2]);
-        if (ch >= term_chunks) break;
-        const int t = (int)ch * 32 + lane;
-        if (t < n * kShTerms) {
-            ShSlot& s = slots[list[t % n]].sh;
-            const int i = t / n;
-            if (i < s.K * (s.K + 1) / 2) sh_term(s, i);
-        }
-        __syncwarp();
+        if (!any) break;
     }
     __syncthreads();
-    if (threadIdx.x == 0) ts.next[0] = ts.next[1] = ts.next[2] = 0;
-    if constexpr (!kFma<MS>) {
+    // phase 2
+    int nl = 0, nc = 0, no = 0, ni = 0, ns = 0;
+    const unsigned char *ll = list, *lc = list, *lo = list, *li = list, *ls = list;
+    if constexpr (kT96) {
+        unsigned fl = 0;
+        int band = 2;
+        bool in = false;
+        if ((mask >> lane) & 1u) {
+            const T96Slot& s = slots[lane].t96;
+            fl = s.flags;
+            band = s.band;
+            in = !(s.sigma >= 1.08 + 0.005);
+        }
+        const unsigned ml = __ballot_sync(kFull, in && (fl & kT96Loops)), mc = __ballot_sync(kFull, in && (fl & kT96Con));
+        const unsigned mo = __ballot_sync(kFull, in && band <= 1), mi = __ballot_sync(kFull, in && band >= 3);
+        const unsigned ms = __ballot_sync(kFull, in && band >= 1 && band <= 3);
+        ll = team_list(ts, 1, ml);
+        lc = team_list(ts, 2, mc);
+        lo = team_list(ts, 3, mo);
+        li = team_list(ts, 4, mi);
+        ls = team_list(ts, 5, ms);
+        nl = __popc(ml);
+        nc = __popc(mc);
+        no = __popc(mo);
+        ni = __popc(mi);
+        ns = __popc(ms);
+        __syncwarp();
+    }
+    // the columns in pairs of complementary length where the slots fill the
+    // warps that way
+    const bool pairs = n > 2;
+    const int cols = pairs ? kShCols / 2 : kShCols;
+    for (;;) {
+        unsigned ch = next_chunk(&ts.next[1]);
+        bool any = false;
+        if constexpr (kT96) {
+            any = true;
+            const int ncir = 3 * nl + 11 * no + 4 * ni;
+            if (takes(ch, ns ? 3 : 0)) {
+                if (lane < ns) {
+                    T96Slot& s = slots[ls[lane]].t96;
+                    if (ch == 0) t96_task_sheet<0>(s);
+                    else if (ch == 1) t96_task_sheet<1>(s);
+                    else t96_task_sheet<2>(s);
+                }
+            } else if (takes(ch, nc ? 1 : 0)) {
+                if (lane < nc) t96_task_con(slots[lc[lane]].t96);
+            } else if (takes(ch, ni ? 1 : 0)) {
+                if (lane < ni) t96_task_inner(slots[li[lane]].t96);
+            } else if (takes(ch, chunks(ncir))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 3 * nl) t96_task_circle(slots[ll[t % nl]].t96, t / nl, false);
+                else if (t - 3 * nl < 11 * no) t96_task_circle(slots[lo[(t - 3 * nl) % no]].t96, 3 + (t - 3 * nl) / no, false);
+                else if (t < ncir)
+                    t96_task_circle(slots[li[(t - 3 * nl - 11 * no) % ni]].t96, 3 + (t - 3 * nl - 11 * no) / ni, true);
+            } else if (takes(ch, chunks(kT96Dip * nc))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < kT96Dip * nc) t96_task_dip(slots[lc[t % nc]].t96, t / nc);
+            } else if (takes(ch, chunks(kT96Exp * n))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < kT96Exp * n) t96_task_exp(slots[list[t % n]].t96, t / n);
+            } else if (takes(ch, chunks(kT96Lop * nl))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < kT96Lop * nl) t96_task_lop(slots[ll[t % nl]].t96, t / nl);
+            } else {
+                any = false;
+            }
+        }
+        if constexpr (kSh) {
+            if (!any) {
+                any = true;
+                if (takes(ch, chunks(n * cols))) {
+                    const int t = (int)ch * 32 + lane;
+                    if (t < n * cols) {
+                        ShSlot& s = slots[list[t % n]].sh;
+                        const int c = t / n, K = s.K;
+                        if (pairs) {
+                            if (2 * c < K) {
+                                sh_column<kFma<MS>>(s, c + 1);
+                                if (K - 1 - c > c) sh_column<kFma<MS>>(s, K - c);
+                            }
+                        } else if (c < K) {
+                            sh_column<kFma<MS>>(s, c + 1);
+                        }
+                    }
+                } else if (takes(ch, chunks(n * kShTerms))) {
+                    // the terms' factors need only the chains
+                    const int t = (int)ch * 32 + lane;
+                    if (t < n * kShTerms) {
+                        ShSlot& s = slots[list[t % n]].sh;
+                        const int i = t / n;
+                        if (i < s.K * (s.K + 1) / 2) sh_term<kFma<MS>>(s, i);
+                    }
+                } else {
+                    any = false;
+                }
+            }
+        }
+        __syncwarp();
+        if (!any) break;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) ts.next[0] = 0;
+    if constexpr (kSh && !kFma<MS>) {
         for (;;) {
-            const unsigned ch = next_chunk(&ts.next[3]);
-            if (ch >= term_chunks) break;
+            const unsigned ch = next_chunk(&ts.next[2]);
+            if (ch >= chunks(n * kShTerms)) break;
             const int t = (int)ch * 32 + lane;
             if (t < n * kShTerms) {
                 ShSlot& s = slots[list[t % n]].sh;
@@ -474,23 +607,136 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
             __syncwarp();
         }
         __syncthreads();
-        if (threadIdx.x == 0) ts.next[3] = 0;
     }
-    // phase 3: the sums, the two long ones of every slot in one chunk
-    const unsigned sum_chunks = (unsigned)(n * (kShCols - 1) + 31) / 32 + 1;
+    if (threadIdx.x == 0) ts.next[1] = 0;
+    // phase 3: the sums, the two long ones of the internal field first
     for (;;) {
-        const unsigned ch = next_chunk(&ts.next[4]);
-        if (ch >= sum_chunks) break;
-        if (ch == 0) {
-            if (lane < 2 * n) sh_sum<kFma<MS>>(slots[list[lane >> 1]].sh, lane & 1);
-        } else {
-            const int t = (int)(ch - 1) * 32 + lane;
-            if (t < n * (kShCols - 1)) sh_sum<kFma<MS>>(slots[list[t % n]].sh, 2 + t / n);
+        unsigned ch = next_chunk(&ts.next[3]);
+        bool any = false;
+        if constexpr (kSh) {
+            any = true;
+            if (takes(ch, 1)) {
+                if (lane < 2 * n) sh_sum<kFma<MS>>(slots[list[lane >> 1]].sh, lane & 1);
+            } else if (takes(ch, chunks(n * (kShCols - 1)))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < n * (kShCols - 1)) sh_sum<kFma<MS>>(slots[list[t % n]].sh, 2 + t / n);
+            } else {
+                any = false;
+            }
+        }
+        if constexpr (kT96) {
+            if (!any) {
+                any = true;
+                if (takes(ch, nc ? 1 : 0)) {
+                    if (lane < 3 * nc) t96_sum_con(slots[lc[lane % nc]].t96, lane / nc);
+                } else if (takes(ch, nl ? 1 : 0)) {
+                    if (lane < 3 * nl) t96_sum_loops(slots[ll[lane % nl]].t96, lane / nl);
+                } else if (takes(ch, no ? 1 : 0)) {
+                    if (lane < no) t96_sum_outer(slots[lo[lane]].t96);
+                } else if (takes(ch, ni ? 1 : 0)) {
+                    if (lane < ni) t96_sum_inner(slots[li[lane]].t96);
+                } else if (takes(ch, chunks(18 * n))) {
+                    const int t = (int)ch * 32 + lane;
+                    if (t < 18 * n) {
+                        const int k = t / n;
+                        t96_sum_shield(slots[list[t % n]].t96, k / 3, k % 3);
+                    }
+                } else if (takes(ch, 1)) {
+                    if (lane < n) t96_sum_t87(slots[list[lane]].t96);
+                } else if (takes(ch, 1)) {
+                    if (lane < 3 * n) t96_sum_cyl(slots[list[lane % n]].t96, lane / n);
+                } else if (takes(ch, chunks(6 * n))) {
+                    const int t = (int)ch * 32 + lane;
+                    if (t < 6 * n) {
+                        const int k = t / n;
+                        t96_sum_rt(slots[list[t % n]].t96, k >= 3, k % 3);
+                    }
+                } else {
+                    any = false;
+                }
+            }
+        }
+        __syncwarp();
+        if (!any) break;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) ts.next[2] = ts.next[3] = 0;
+}
+
+// What a quad writes for its slot before team_field (all lanes of the warp
+// call; need: the quad's slot is evaluated) and reads after it.
+template <class MS>
+__device__ __forceinline__ void team_begin(TeamSlot<MS>& s, const Vec3 pos, const DevParams* par, const bool need) {
+    if constexpr (MS::internal != 0) {
+        Vec3 geo = {1., 0., 0.};
+        if (need) geo = gsm_to_geo(pos, &par->p);
+        __syncwarp();
+        quad_sh_geometry(s.sh, geo, need ? &par->p : nullptr, need);
+    }
+    if constexpr (MS::external == COR_EXTERNAL_T96) {
+        if (need && (threadIdx.x & 3) == 0) t96_slot_start(s.t96, par->t96, pos);
+    }
+    __syncwarp();
+}
+
+template <class MS>
+__device__ __forceinline__ Vec3 team_end(const TeamSlot<MS>& s, const DevParams* par) {
+    const cor_model_params* p = &par->p;
+    Vec3 tot = {0., 0., 0.};
+    if constexpr (MS::internal != 0) {
+        const Vec3 bs = geo_to_gsm(sh_finish<kFma<MS>>(s.sh), p);
+        tot.x += bs.x;
+        tot.y += bs.y;
+        tot.z += bs.z;
+    }
+    if constexpr (MS::external == COR_EXTERNAL_T96) {
+        const Vec3 b = t96_slot_end(s.t96);
+        tot.x += b.x;
+        tot.y += b.y;
+        tot.z += b.z;
+    }
+    return gsm_to_geo(tot, p);
+}
+
+// The field at n points by teams (field_kernel's arguments): block b takes
+// points b n_slots .. and on.
+template <class MS>
+__global__ void __launch_bounds__(kTeamThreads)
+    team_field_kernel(const DevParams* __restrict__ params, const int n_params, const int32_t* __restrict__ pidx,
+                      const double* __restrict__ pos, const int64_t n, double* __restrict__ out, const int n_slots) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    __shared__ TeamShared ts;
+    TeamSlot<MS>* slots = reinterpret_cast<TeamSlot<MS>*>(s_dyn);
+    const int tid = threadIdx.x, slot = tid >> 2;
+    if (tid < 4) ts.next[tid] = 0;
+    for (int64_t i0 = (int64_t)blockIdx.x * n_slots; i0 < n; i0 += (int64_t)gridDim.x * n_slots) {
+        const int64_t i = i0 + slot;
+        const bool need = slot < n_slots && i < n;
+        const DevParams* par = params;
+        if (__any_sync(kFull, need)) {
+            Vec3 x = {0., 0., 0.};
+            if (need) {
+                const int k = pidx ? pidx[i] : 0;
+                par = params + (k < 0 || k >= n_params ? 0 : k);
+                x = {DIVRE(pos[3 * i]), DIVRE(pos[3 * i + 1]), DIVRE(pos[3 * i + 2])};
+            }
+            __syncwarp();
+            team_begin<MS>(slots[slot < n_slots ? slot : 0], x, par, need);
+        }
+        const int64_t left = n - i0;
+        const int m = left < n_slots ? (int)left : n_slots;
+        __syncthreads();
+        team_field<MS>(ts, slots, m == 32 ? kFull : (1u << m) - 1u);
+        if (need) {
+            const Vec3 b = team_end<MS>(slots[slot], par);
+            if ((tid & 3) == 0) {
+                out[3 * i] = b.x;
+                out[3 * i + 1] = b.y;
+                out[3 * i + 2] = b.z;
+            }
         }
         __syncwarp();
     }
-    __syncthreads();
-    if (threadIdx.x == 0) ts.next[4] = 0;
 }
 
 // The scan by teams: one generation, as trace_kernel's.  `n_slots` (at most
@@ -502,7 +748,7 @@ __global__ void __launch_bounds__(kTeamThreads) team_trace_kernel(const TraceArg
     __shared__ TeamShared ts;
     TeamSlot<MS>* slots = reinterpret_cast<TeamSlot<MS>*>(s_dyn);
     const int tid = threadIdx.x, slot = tid >> 2, q = tid & 3;
-    if (tid < 8) ts.next[tid] = 0;
+    if (tid < 4) ts.next[tid] = 0;
     if (tid < 32) ts.need[tid] = 0;
     __syncthreads();
     Lane L;
@@ -567,17 +813,10 @@ __global__ void __launch_bounds__(kTeamThreads) team_trace_kernel(const TraceArg
         }
         __syncwarp();
         const bool warp_need = __any_sync(kFull, need);
-        Vec3 pos = {0., 0., 0.};
-        const cor_model_params* p = nullptr;
         if (warp_need) {
-            Vec3 geo = {1., 0., 0.};
-            if (need) {
-                p = &L.par->p;
-                pos = {DIVRE(L.gsm.x), DIVRE(L.gsm.y), DIVRE(L.gsm.z)};
-                geo = gsm_to_geo(pos, p);
-            }
-            __syncwarp();
-            quad_sh_geometry(slots[slot < n_slots ? slot : 0].sh, geo, p, need);
+            Vec3 pos = {0., 0., 0.};
+            if (need) pos = {DIVRE(L.gsm.x), DIVRE(L.gsm.y), DIVRE(L.gsm.z)};
+            team_begin<MS>(slots[slot < n_slots ? slot : 0], pos, L.par, need);
         }
         if (q == 0 && slot < 32) ts.need[slot] = need;
         if (__syncthreads_and(done)) break;
@@ -588,12 +827,7 @@ __global__ void __launch_bounds__(kTeamThreads) team_trace_kernel(const TraceArg
         }
         team_field<MS>(ts, slots, mask);
         if (need) {
-            Vec3 tot = {0., 0., 0.};
-            const Vec3 bs = geo_to_gsm(sh_finish<kFma<MS>>(slots[slot].sh), p);
-            tot.x += bs.x;
-            tot.y += bs.y;
-            tot.z += bs.z;
-            L.field = gsm_to_geo(tot, p);
+            L.field = team_end<MS>(slots[slot], L.par);
             L.b = 1.E-09 * sqrt(L.field.x * L.field.x + L.field.y * L.field.y + L.field.z * L.field.z);
         }
         __syncwarp();
