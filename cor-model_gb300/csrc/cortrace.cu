@@ -306,18 +306,23 @@ static const ModelOps* find_ops(const cor_model_set& m) {
 // 286 / 178, 40,000 375 / 325 (291 when the teams take over at half the
 // lanes), 91,200 562 / 666 (487).  With T96, limit 1,000 steps: 400
 // trajectories 432 / 63, 2,000 484 / 92; limit 250: 8,000 103 / 110, 20,000
-// 291 / 187, 66,000 (the tail by teams) 629 / 497.
+// 291 / 187, 66,000 (the tail by teams) 629 / 497.  With TS05: 3,573
+// trajectories, limit 400, 607 / 172; limit 100: 8,000 143 / 84, 20,000
+// 235 / 153.
 static bool team_takes(const ModelOps* ops, uint64_t live, uint64_t cap_blocks) {
     return ops->launch_team && 2 * live <= cap_blocks * (uint64_t)kTraceThreads;
 }
 
 // The same for a field batch of n points, where every lane does the same
-// amount of work: up to a sixth of the lanes.  T96, us by lanes / by teams
-// (the call's allocations and copies included): 1 point 403 / 114, 1,000
-// 614 / 184, 5,000 625 / 433, 8,000 639 / 736; IGRF-14: 1 116 / 83, 2,664
-// 177 / 127, 8,000 177 / 184.
-static bool team_takes_field(const ModelOps* ops, uint64_t n, int sms) {
-    return ops->launch_team_field && 6 * n <= (uint64_t)sms * (uint64_t)kTraceThreads;
+// amount of work: up to a sixth of the lanes, with TS05 (whose tasks fill a
+// team best) up to half.  T96, us by lanes / by teams (the call's allocations
+// and copies included): 1 point 403 / 114, 1,000 614 / 184, 5,000 625 / 433,
+// 8,000 639 / 736; IGRF-14: 1 116 / 83, 2,664 177 / 127, 8,000 177 / 184;
+// TS05: 1 979 / 188, 2,664 1,085 / 364, 12,000 1,110 / 985, 20,000
+// 1,989 / 1,603.
+static bool team_takes_field(const ModelOps* ops, cor_model_set models, uint64_t n, int sms) {
+    const uint64_t share = models.external_model == COR_EXTERNAL_TS05 ? 2 : 6;
+    return ops->launch_team_field && share * n <= (uint64_t)sms * (uint64_t)kTraceThreads;
 }
 
 // Slots per block and blocks of a team launch: as many blocks as are resident
@@ -733,7 +738,7 @@ extern "C" int cor_field_batch(cor_ctx* ctx, cor_model_set models, const cor_mod
         const ModelOps* ops = find_ops(models);
         int slots = 1;
         unsigned blocks = 1;
-        if (team_takes_field(ops, (uint64_t)n, ctx->sms)) {
+        if (team_takes_field(ops, models, (uint64_t)n, ctx->sms)) {
             if ((rc = team_shape(ctx, ops, (uint64_t)n, &slots, &blocks)) != COR_OK) break;
             ops->launch_team_field((const DevParams*)dp, n_params, (const int32_t*)didx, (const double*)dpos, n,
                                    (double*)dout, slots, blocks, s);

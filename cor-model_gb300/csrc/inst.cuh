@@ -46,9 +46,10 @@
         cudaError_t e = cudaMemcpyToSymbol(c_t96, t96, sizeof(T96Tables));                                 \
         if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_t96, t96, sizeof(T96Tables));                       \
         if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_ts05, ts05, sizeof(TS05Tables));                    \
+        if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_ts05, ts05, sizeof(TS05Tables));                    \
         return e;                                                                                          \
     }                                                                                                      \
-    template <class MS, bool TEAM = MS::crustal == 0 && MS::external != COR_EXTERNAL_TS05>                 \
+    template <class MS, bool TEAM = MS::crustal == 0>                                                      \
     struct Team_##NAME {                                                                                   \
         static cudaError_t occ(int n_slots, int* n) {                                                      \
             const size_t smem = (size_t)n_slots * sizeof(TeamSlot<MS>);                                    \

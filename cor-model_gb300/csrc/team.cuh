@@ -36,6 +36,7 @@ __device__ __forceinline__ double comp(const Vec3 v, const int c) { return c == 
 }  // namespace cor
 
 #include "team_t96.cuh"
+#include "team_ts05.cuh"
 
 namespace cor {
 
@@ -427,6 +428,7 @@ template <class MS>
 struct TeamSlotBody {
     std::conditional_t<MS::internal != 0, ShSlot, NoSlot> sh;
     std::conditional_t<MS::external == COR_EXTERNAL_T96, T96Slot, NoSlot> t96;
+    std::conditional_t<MS::external == COR_EXTERNAL_TS05, TS05Slot, NoSlot> ts05;
 };
 // An odd number of 8-byte words, so that slots start in different banks.
 template <class MS>
@@ -439,7 +441,8 @@ struct TeamSlot : TeamSlotBody<MS> {
 // within one the warps take chunks of 32 tasks, the longest kinds first.
 template <class MS>
 __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, const unsigned mask) {
-    constexpr bool kSh = MS::internal != 0, kT96 = MS::external == COR_EXTERNAL_T96;
+    constexpr bool kSh = MS::internal != 0, kT96 = MS::external == COR_EXTERNAL_T96,
+                   kTS05 = MS::external == COR_EXTERNAL_TS05;
     const int lane = threadIdx.x & 31;
     const int n = __popc(mask);
     const unsigned char* list = team_list(ts, 0, mask);
@@ -468,6 +471,30 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
             } else if (takes(ch, chunks(kT96Sc * n))) {
                 const int t = (int)ch * 32 + lane;
                 if (t < kT96Sc * n) t96_task_sc(slots[list[t % n]].t96, t / n);
+            } else {
+                any = false;
+            }
+        }
+        if constexpr (kTS05) {
+            any = true;
+            if (takes(ch, chunks(4 * n))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 4 * n) ts05_task_shield(slots[list[t % n]].ts05, t / n);
+            } else if (takes(ch, 1)) {
+                if (lane < n) {
+                    TS05Slot& s = slots[list[lane]].ts05;
+                    put3(s.cf, ts05_shlcar3x3(s.x, s.y, s.z));
+                }
+            } else if (takes(ch, 1)) {
+                if (lane < 2 * n) ts05_task_birk(slots[list[lane >> 1]].ts05, lane & 1);
+            } else if (takes(ch, 1)) {
+                if (lane < 2 * n) ts05_task_symm(slots[list[lane >> 1]].ts05, lane & 1);
+            } else if (takes(ch, 1)) {
+                if (lane < n) ts05_task_quad(slots[list[lane]].ts05);
+            } else if (takes(ch, 1)) {
+                if (lane < n) ts05_task_warp(slots[list[lane]].ts05);
+            } else if (takes(ch, 1)) {
+                if (lane < n) ts05_task_main(slots[list[lane]].ts05);
             } else {
                 any = false;
             }
@@ -519,6 +546,12 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
         ns = __popc(ms);
         __syncwarp();
     }
+    if constexpr (kTS05) {
+        const unsigned mc = __ballot_sync(kFull, ((mask >> lane) & 1u) && slots[lane].ts05.sigma < 1.1960 + 0.005);
+        lc = team_list(ts, 2, mc);
+        nc = __popc(mc);
+        __syncwarp();
+    }
     // the columns in pairs of complementary length where the slots fill the
     // warps that way
     const bool pairs = n > 2;
@@ -555,6 +588,30 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
             } else if (takes(ch, chunks(kT96Lop * nl))) {
                 const int t = (int)ch * 32 + lane;
                 if (t < kT96Lop * nl) t96_task_lop(slots[ll[t % nl]].t96, t / nl);
+            } else {
+                any = false;
+            }
+        }
+        if constexpr (kTS05) {
+            any = true;
+            if (takes(ch, chunks(4 * nc))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 4 * nc) ts05_task_cone(slots[lc[t % nc]].ts05, t / nc);
+            } else if (takes(ch, chunks(4 * nc))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 4 * nc) ts05_task_ap(slots[lc[t % nc]].ts05, 1, t / nc);
+            } else if (takes(ch, nc ? 1 : 0)) {
+                if (lane < 3 * nc) ts05_task_br(slots[lc[lane % nc]].ts05, lane / nc);
+            } else if (takes(ch, nc ? 1 : 0)) {
+                if (lane < 3 * nc) ts05_task_bt(slots[lc[lane % nc]].ts05, lane / nc);
+            } else if (takes(ch, nc ? 1 : 0)) {
+                if (lane < 2 * nc) ts05_task_disk(slots[lc[lane >> 1]].ts05, lane & 1);
+            } else if (takes(ch, chunks(4 * nc))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 4 * nc) ts05_task_ap(slots[lc[t % nc]].ts05, 0, t / nc);
+            } else if (takes(ch, chunks(20 * nc))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 20 * nc) ts05_task_sc(slots[lc[t % nc]].ts05, t / nc);
             } else {
                 any = false;
             }
@@ -624,6 +681,23 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
                 any = false;
             }
         }
+        if constexpr (kTS05) {
+            if (!any) {
+                any = true;
+                if (takes(ch, chunks(50 * nc))) {
+                    const int t = (int)ch * 32 + lane;
+                    if (t < 50 * nc) ts05_task_exp(slots[lc[t % nc]].ts05, t / nc);
+                } else if (takes(ch, nc ? 1 : 0)) {
+                    if (lane < 2 * nc) ts05_end_birk(slots[lc[lane >> 1]].ts05, lane & 1);
+                } else if (takes(ch, nc ? 1 : 0)) {
+                    if (lane < 2 * nc) ts05_end_symm(slots[lc[lane >> 1]].ts05, lane & 1);
+                } else if (takes(ch, nc ? 1 : 0)) {
+                    if (lane < nc) ts05_end_quad(slots[lc[lane]].ts05);
+                } else {
+                    any = false;
+                }
+            }
+        }
         if constexpr (kT96) {
             if (!any) {
                 any = true;
@@ -660,6 +734,14 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
         if (!any) break;
     }
     __syncthreads();
+    if constexpr (kTS05) {
+        const int t = (int)threadIdx.x;   // one pass: at most 6 kTeamSlots tasks
+        if (t < 6 * nc) {
+            const int k = t / nc;
+            ts05_sum5(slots[lc[t % nc]].ts05, k / 3, k % 3);
+        }
+        __syncthreads();
+    }
     if (threadIdx.x == 0) ts.next[2] = ts.next[3] = 0;
 }
 
@@ -676,6 +758,9 @@ __device__ __forceinline__ void team_begin(TeamSlot<MS>& s, const Vec3 pos, cons
     if constexpr (MS::external == COR_EXTERNAL_T96) {
         if (need && (threadIdx.x & 3) == 0) t96_slot_start(s.t96, par->t96, pos);
     }
+    if constexpr (MS::external == COR_EXTERNAL_TS05) {
+        if (need && (threadIdx.x & 3) == 0) ts05_slot_start(s.ts05, par->ts05, pos);
+    }
     __syncwarp();
 }
 
@@ -691,6 +776,12 @@ __device__ __forceinline__ Vec3 team_end(const TeamSlot<MS>& s, const DevParams*
     }
     if constexpr (MS::external == COR_EXTERNAL_T96) {
         const Vec3 b = t96_slot_end(s.t96);
+        tot.x += b.x;
+        tot.y += b.y;
+        tot.z += b.z;
+    }
+    if constexpr (MS::external == COR_EXTERNAL_TS05) {
+        const Vec3 b = ts05_slot_end(s.ts05);
         tot.x += b.x;
         tot.y += b.y;
         tot.z += b.z;

@@ -13,6 +13,7 @@ import pyoracle
 pytestmark = pytest.mark.gpu
 
 TIME7 = [2020, 6, 21, 173, 12, 0, 0]
+PARMOD = [3.0, -60.0, 4.0, -7.0, 0.4, 0.8, 0.3, 1.1, 0.6, 0.9]
 
 
 def jobs_of(n_sites: int, n_rig: int, seed: int) -> np.ndarray:
@@ -57,13 +58,14 @@ def test_step_settings_equal_oracle(ctx, tu, nk1):
         assert np.array_equal(gpu.records[k], cpu.records[k]), k
 
 
+@pytest.mark.parametrize("external", [ct.EXTERNAL_T96, ct.EXTERNAL_TS05])
 @pytest.mark.parametrize("internal", [ct.INTERNAL_SH, ct.INTERNAL_NONE])
-def test_t96_same_bits_among_many_and_alone(ctx, internal):
+def test_same_bits_among_many_and_alone(ctx, internal, external):
     """20,480 trajectories start one to a lane; the same ones in calls of 7, 640 and
     4,100 run by teams.  Every class, count and final state is the same bits."""
     jobs = jobs_of(640, 32, 5)
-    p = ct.internal_setup("igrf14", TIME7, parmod=[3.0, -60.0, 4.0, -7.0])
-    m = ct.model_set(internal, ct.EXTERNAL_T96)
+    p = ct.internal_setup("igrf14", TIME7, parmod=PARMOD)
+    m = ct.model_set(internal, external)
     want = ctx.trace_batch(jobs, p, m, step_limit=70, want_records=True)
     for a, b in ((3, 3 + 1), (100, 120), (500, 628)):
         got = ctx.trace_batch(jobs[a:b], p, m, step_limit=70, want_records=True)
@@ -74,26 +76,29 @@ def test_t96_same_bits_among_many_and_alone(ctx, internal):
 
 # points: one, a slot more than a block's eight, the last count that goes by
 # teams and the first that does not
-@pytest.mark.parametrize("external", [ct.EXTERNAL_NONE, ct.EXTERNAL_T96])
-@pytest.mark.parametrize("n", [1, 9, 6485, 6486])
+@pytest.mark.parametrize("external,n", [(ct.EXTERNAL_NONE, 1), (ct.EXTERNAL_NONE, 9), (ct.EXTERNAL_NONE, 6485),
+                                        (ct.EXTERNAL_NONE, 6486), (ct.EXTERNAL_T96, 1), (ct.EXTERNAL_T96, 9),
+                                        (ct.EXTERNAL_T96, 6485), (ct.EXTERNAL_T96, 6486), (ct.EXTERNAL_TS05, 1),
+                                        (ct.EXTERNAL_TS05, 9), (ct.EXTERNAL_TS05, 19456), (ct.EXTERNAL_TS05, 19457)])
 def test_field_against_oracle(ctx, external, n):
     rng = np.random.default_rng(n)
     u = rng.normal(size=(n, 3))
     u /= np.linalg.norm(u, axis=1)[:, None]
     pts = u * np.exp(rng.uniform(np.log(1.003), np.log(24.0), n))[:, None] * ct.DEF_RE
-    p = ct.internal_setup("igrf14", TIME7, parmod=[3.0, -60.0, 4.0, -7.0])
+    p = ct.internal_setup("igrf14", TIME7, parmod=PARMOD)
     m = ct.model_set(ct.INTERNAL_SH, external)
     got = ctx.field_batch(pts, p, m)
     want = pyoracle.calculate_field(pts[:200], p, m)
     if external == ct.EXTERNAL_NONE:
         assert np.array_equal(got[:200].view(np.uint64), want.view(np.uint64))
     else:
-        # within the reference's own spread at these conditions (8.2e-12) of the
-        # sum's largest part (outside the magnetopause the dipole cancels the
-        # internal field), or 16 times the point's own spread under one-ulp
-        # changes of the C library
+        # within the reference's own spread under one-ulp changes of the C library
+        # over storm conditions (T96 8.2e-12; TS05's central differences 2.4e-7) of
+        # the sum's largest part (outside the magnetopause the dipole cancels the
+        # internal field), or 16 times the point's own
+        rel = 8.2e-12 if external == ct.EXTERNAL_T96 else 2.4e-7
         own = pyoracle.calculate_field_nudged(pts[:200], p, m)
         scale = np.linalg.norm(pyoracle.calculate_field(pts[:200], p, ct.model_set(ct.INTERNAL_SH)), axis=1)
         scale = np.maximum(scale, np.linalg.norm(want, axis=1))
-        bar = np.maximum(8.2e-12 * scale, 16.0 * np.linalg.norm(own - want, axis=1))
+        bar = np.maximum(rel * scale, 16.0 * np.linalg.norm(own - want, axis=1))
         assert np.all(np.linalg.norm(got[:200] - want, axis=1) <= bar)
