@@ -13,13 +13,19 @@
 //    and walks each column down the degrees with the column recursion
 //    (P(n,m) needs only P(n-1,m) and P(n-2,m)), the diagonal P(m,m) and the
 //    radial powers (a/r)^(n+1) carried along as the reference's sequential
-//    products; sin(m*phi), cos(m*phi) once per column;
+//    products; sin(m*phi), cos(m*phi) once per column.  A lane's columns are
+//    one run of terms: it goes on to its next column when one ends, so the 32
+//    lanes finish together (543 to 548 terms each) instead of waiting at every
+//    column for the longest (636);
 //  * the recursion factors k = sqrt((2n-1)/2n), k1 = (2n-1)/sqrt(n^2-m^2),
 //    k2 = sqrt(((n-1)^2-m^2)/(n^2-m^2)) come from tables the host built with
 //    the same expressions (IEEE division and square root are correctly
 //    rounded on both sides, so they hold the reference's values);
 //  * the three sums are taken per column, then across the lanes, where the
 //    reference sums degree by degree.
+// Bound by the FP64 pipe: 22 instructions a term (25 before the products with m
+// and the factors -(n + 1) came from the tables).  40,001 points at 1 to 1.5
+// R_E with IGRF-14: 88.1 ms -> 37.3 ms, with field_kernel's even split.
 // The device atan2/sin/cos are not glibc's either, so results agree with the
 // reference to a few ulp of the crustal field, not bit for bit.
 #pragma once
@@ -52,13 +58,29 @@ struct CrustalTables {
     int external;
 };
 
+constexpr int kChaosCols = kChaosMaxN / 32;   // columns of a lane, at most
+
+// Two consecutive table entries (16-byte aligned) in one load.
+struct Double2 {
+    double x, y;
+};
+__device__ __forceinline__ Double2 ldg2(const double* p) {
+#ifdef __CUDA_ARCH__
+    const double2 v = __ldg(reinterpret_cast<const double2*>(p));
+    return {v.x, v.y};
+#else
+    return {p[0], p[1]};
+#endif
+}
+
 // Called by all 32 lanes of a warp together; a lane with `want` set gets
 // chaos_geo at its own GEO position x [R_E].
 static __device__ __noinline__ Vec3 chaos_geo_warp(const bool want, const Vec3 x, const CrustalTables& t) {
     const int lane = threadIdx.x & 31;
     const int nmax = t.nmax;
-    const double* __restrict__ G = t.g;
-    const double* __restrict__ H = t.h;
+    // the tables by order (crustal_block)
+    const double* __restrict__ col = t.kd + ((nmax + 1) & ~1);
+    const double* __restrict__ nd = col + 6 * (size_t)(nmax * (nmax + 1) / 2);
     unsigned todo = __ballot_sync(0xffffffffu, want);
     Vec3 mine = {0., 0., 0.};
     while (todo) {
@@ -89,10 +111,13 @@ static __device__ __noinline__ Vec3 chaos_geo_warp(const bool want, const Vec3 x
         const double tem = kChaosReKm / r;
         const double rr = 1. / r;
         double br = 0., bt = 0., bp = 0.;
-        // diagonal P(d,d), dP(d,d) and the radial power ar[d] = tem^(d+1)
+        // starts of this lane's columns: the diagonal P(m,m), dP(m,m), the
+        // radial power tem^(m+1), sin and cos of m phi
         double pd = 1., dpd = 0., rnd = tem;
+        double spd[kChaosCols], sdpd[kChaosCols], srn[kChaosCols], ssm[kChaosCols], scm[kChaosCols];
         int d = 0;
-        for (int c = 0;; c++) {
+#pragma unroll 1
+        for (int c = 0; c < kChaosCols; c++) {
             const int m = c * 32 + ((c & 1) ? 31 - lane : lane);
             if (m >= nmax) break;
             while (d < m) {                       // chaos.c:159-170
@@ -108,44 +133,55 @@ static __device__ __noinline__ Vec3 chaos_geo_warp(const bool want, const Vec3 x
                     pd = st * kp;
                 }
             }
-            double sm, cm;
-            sincos(m * phi, &sm, &cm);
-            const double md = (double)m;
-            double p1 = pd, dp1 = dpd, p2 = 0., dp2 = 0.;   // P(n-1,m), P(n-2,m); P(m-1,m) = 0
-            double rn = rnd;
-            for (int n = m; n < nmax; n++) {
+            spd[c] = pd;
+            sdpd[c] = dpd;
+            srn[c] = rnd;
+            sincos(m * phi, &ssm[c], &scm[c]);
+        }
+        // the terms, column after column
+        int c = -1, m = 0, n = nmax;
+        double p1 = 0., dp1 = 0., p2 = 0., dp2 = 0., rn = 0., sm = 0., cm = 0.;
+        const double* q6 = nullptr;
+        for (;;) {
+            const bool first = n == nmax;
+            if (first) {
+                c++;
+                m = c * 32 + ((c & 1) ? 31 - lane : lane);
+                if (c == kChaosCols || m >= nmax) break;
+                n = m;
+                p1 = spd[c];
+                dp1 = sdpd[c];
+                p2 = dp2 = 0.;                    // P(m-1,m) = 0
+                rn = srn[c];
+                sm = ssm[c];
+                cm = scm[c];
+                q6 = col + 6 * (m * nmax - m * (m - 1) / 2);
+            } else {
                 double pnm, dpnm;
-                if (n == m) {
-                    pnm = p1;
-                    dpnm = dp1;
-                } else {
-                    if (n == 1) {                 // P(1,0), dP(1,0) are set directly, :161-163
-                        pnm = ct;
-                        dpnm = -st;
-                    } else {                      // :172-194
-                        const int idx = n * (n + 1) / 2 + m;
-                        const double k1 = __ldg(t.k1 + idx);
-                        const double k2 = __ldg(t.k2 + idx);
-                        pnm = k1 * ct * p1 - k2 * p2;
-                        dpnm = k1 * (-st * p1 + ct * dp1) - k2 * dp2;
-                    }
-                    p2 = p1;
-                    dp2 = dp1;
-                    p1 = pnm;
-                    dp1 = dpnm;
-                    rn = rn * tem;
+                if (n == 1) {                     // P(1,0), dP(1,0) are set directly, :161-163
+                    pnm = ct;
+                    dpnm = -st;
+                } else {                          // :172-194
+                    const Double2 k = ldg2(q6);
+                    pnm = k.x * ct * p1 - k.y * p2;
+                    dpnm = k.x * (-st * p1 + ct * dp1) - k.y * dp2;
                 }
-                if (n >= t.n_first) {             // :201-216
-                    const double drn = div_r(-(double)(n + 1) * rn, r, rr);
-                    const int idx = n * (n + 1) / 2 + m;
-                    const double g = __ldg(G + idx);
-                    const double h = __ldg(H + idx);
-                    const double tt = g * cm + h * sm;
-                    br += tt * pnm * drn;
-                    bt += tt * dpnm * rn;
-                    bp += (-g * md * sm + h * md * cm) * pnm * rn;
-                }
+                p2 = p1;
+                dp2 = dp1;
+                p1 = pnm;
+                dp1 = dpnm;
+                rn = rn * tem;
             }
+            if (n >= t.n_first) {                 // :201-216
+                const double drn = div_r(__ldg(nd + n) * rn, r, rr);
+                const Double2 gh = ldg2(q6 + 2), gm = ldg2(q6 + 4);
+                const double tt = gh.x * cm + gh.y * sm;
+                br += tt * p1 * drn;
+                bt += tt * dp1 * rn;
+                bp += (-gm.x * sm + gm.y * cm) * p1 * rn;
+            }
+            n++;
+            q6 += 6;
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {

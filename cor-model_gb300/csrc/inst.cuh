@@ -38,15 +38,33 @@
     }                                                                                                      \
     static cudaError_t field_##NAME(const DevParams* p, int np, const int32_t* idx, const double* pos,     \
                                     int64_t n, double* out, CrustalTables crust, cudaStream_t s) {         \
-        const unsigned blocks = (unsigned)((n + 127) / 128);                                               \
-        field_kernel<MS_##NAME><<<blocks, 128, 0, s>>>(p, np, idx, pos, n, out, crust);                    \
+        unsigned blocks = (unsigned)((n + 127) / 128);                                                     \
+        int64_t per_warp = 1;                                                                              \
+        if (C != 0) {                                                                                      \
+            int dev = 0, sms = 1, per_sm = 1;                                                              \
+            cudaError_t e = cudaGetDevice(&dev);                                                           \
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);   \
+            if (e == cudaSuccess)                                                                          \
+                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, field_kernel<MS_##NAME>, 128, 0); \
+            if (e != cudaSuccess) return e;                                                                \
+            const int64_t resident = (int64_t)sms * (per_sm > 0 ? per_sm : 1);                             \
+            per_warp = (n + 4 * resident - 1) / (4 * resident);                                            \
+            blocks = (unsigned)((n + 4 * per_warp - 1) / (4 * per_warp));                                  \
+        }                                                                                                  \
+        field_kernel<MS_##NAME><<<blocks, 128, 0, s>>>(p, np, idx, pos, n, out, crust, per_warp);          \
         return cudaGetLastError();                                                                         \
     }                                                                                                      \
     static cudaError_t tables_##NAME(const T96Tables* t96, const TS05Tables* ts05) {                       \
-        cudaError_t e = cudaMemcpyToSymbol(c_t96, t96, sizeof(T96Tables));                                 \
-        if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_t96, t96, sizeof(T96Tables));                       \
-        if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_ts05, ts05, sizeof(TS05Tables));                    \
-        if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_ts05, ts05, sizeof(TS05Tables));                    \
+        /* only what the set's kernels read: a copy takes about 8 us of cor_ctx_create */                  \
+        cudaError_t e = cudaSuccess;                                                                       \
+        if (E != COR_EXTERNAL_NONE && E != COR_EXTERNAL_TS05) {                                            \
+            e = cudaMemcpyToSymbol(c_t96, t96, sizeof(T96Tables));                                         \
+            if (e == cudaSuccess && C == 0) e = cudaMemcpyToSymbol(g_t96, t96, sizeof(T96Tables));         \
+        }                                                                                                  \
+        if (e == cudaSuccess && E != COR_EXTERNAL_NONE && E != COR_EXTERNAL_T96) {                         \
+            e = cudaMemcpyToSymbol(c_ts05, ts05, sizeof(TS05Tables));                                      \
+            if (e == cudaSuccess && C == 0) e = cudaMemcpyToSymbol(g_ts05, ts05, sizeof(TS05Tables));      \
+        }                                                                                                  \
         return e;                                                                                          \
     }                                                                                                      \
     template <class MS, bool TEAM = MS::crustal == 0>                                                      \

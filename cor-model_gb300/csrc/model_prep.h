@@ -235,10 +235,14 @@ static void prepare_params(const cor_model_params* in, int32_t n, DevParams* out
 // The crustal model's tables, as one block: g, h, k1, k2 (packed lower
 // triangles of nmax(nmax+1)/2 entries each), then kd (nmax entries).  k1, k2
 // and kd are the recursion factors of lib/chaos/chaos.c:163-180, computed with
-// its expressions.  `host` holds crustal_block_size(nmax) zeroed doubles.
-// Returns the first degree with a non-zero coefficient (nmax if none).
+// its expressions.  Then, for the device, the same by order (chaos_columns):
+// per term k1, k2, g, h, g m, h m (the products the sums start with), column
+// by column, and -(n + 1) per degree.  `host` holds crustal_block_size(nmax)
+// zeroed doubles.  Returns the first degree with a non-zero coefficient (nmax
+// if none).
 static size_t crustal_block_size(int32_t nmax) {
-    return 4 * ((size_t)nmax * (size_t)(nmax + 1) / 2) + (size_t)nmax;
+    const size_t nt = (size_t)nmax * (size_t)(nmax + 1) / 2;
+    return 4 * nt + (size_t)((nmax + 1) & ~1) + 6 * nt + (size_t)nmax;
 }
 
 static int crustal_block(const double* g, const double* h, int32_t nmax, double* host) {
@@ -268,6 +272,20 @@ static int crustal_block(const double* g, const double* h, int32_t nmax, double*
             hk2[n * (n + 1) / 2 + m] = sqrt((n1 * n1 - mm) / nnmm);
         }
     }
+    double* col = hkd + ((nmax + 1) & ~1);
+    double* nd = col + 6 * nt;
+    for (int m = 0; m < nmax; m++)
+        for (int n = m; n < nmax; n++) {
+            const size_t i = (size_t)n * (size_t)(n + 1) / 2 + (size_t)m;
+            col[0] = hk1[i];
+            col[1] = hk2[i];
+            col[2] = g[i];
+            col[3] = h[i];
+            col[4] = g[i] * (double)m;
+            col[5] = h[i] * (double)m;
+            col += 6;
+        }
+    for (int n = 0; n < nmax; n++) nd[n] = -(double)(n + 1);
     return n_first;
 }
 

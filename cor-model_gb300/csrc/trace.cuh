@@ -558,25 +558,40 @@ __global__ void __launch_bounds__(kTraceThreads, 1) trace_kernel(const TraceArgs
     warp_add_u64(reinterpret_cast<unsigned long long*>(&a.counters->watchdog), n_wd);
 }
 
+// calculate_field at n points.  With the crustal model, whose sum takes a whole
+// warp per point, the resident warps take per_warp points each, so
+// that no wave of blocks is left nearly empty (40,001 points in blocks of 128
+// threads, 128 points each, were two waves, the second of 9 blocks); without
+// it, a thread takes one point.
 template <class MS>
 __global__ void field_kernel(const DevParams* __restrict__ params, int n_params,
                              const int32_t* __restrict__ pidx, const double* __restrict__ pos, int64_t n,
-                             double* __restrict__ out, CrustalTables crust) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool want = i < n;
-    if (MS::crustal == 0 && !want) return;   // with the crustal model every lane takes part
-    int k = 0;
-    Vec3 x = {0., 0., 0.};
-    if (want) {
-        k = pidx ? pidx[i] : 0;
-        if (k < 0 || k >= n_params) k = 0;
-        x = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
+                             double* __restrict__ out, CrustalTables crust, int64_t per_warp) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (MS::crustal == 0 && t >= n) return;
+    int64_t lo = t, hi = n;
+    if (MS::crustal != 0) {
+        lo = (t >> 5) * per_warp;
+        hi = lo + per_warp < n ? lo + per_warp : n;
     }
-    const Vec3 b = calculate_field<MS>(want, x, params + k, crust);
-    if (!want) return;
-    out[3 * i] = b.x;
-    out[3 * i + 1] = b.y;
-    out[3 * i + 2] = b.z;
+    for (int64_t i0 = lo; i0 < hi; i0 += 32) {
+        const int64_t i = MS::crustal != 0 ? i0 + (threadIdx.x & 31) : i0;
+        const bool want = i < hi;
+        int k = 0;
+        Vec3 x = {0., 0., 0.};
+        if (want) {
+            k = pidx ? pidx[i] : 0;
+            if (k < 0 || k >= n_params) k = 0;
+            x = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
+        }
+        const Vec3 b = calculate_field<MS>(want, x, params + k, crust);
+        if (want) {
+            out[3 * i] = b.x;
+            out[3 * i + 1] = b.y;
+            out[3 * i + 2] = b.z;
+        }
+        if (MS::crustal == 0) return;
+    }
 }
 
 }  // namespace cor
