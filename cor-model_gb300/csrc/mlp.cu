@@ -1,24 +1,36 @@
 // mlp.cu -- the learned rigidity window's network (include/cor_window.h): a
 // BF16 MLP whose every matrix product runs on the 5th-generation tensor cores.
 //
-// One GEMM kernel serves the forward and backward passes:
-//   C[M][N] = A[M][K] . B[N][K]^T      (A, B BF16 and K-major, C FP32 in TMEM)
-// with M a multiple of 128 (one 128-row tile per CTA), N a multiple of 16 up
-// to 256 (the whole N in one tcgen05.mma), K a multiple of 64 (one 64-deep
-// shared-memory stage = four K=16 MMAs).  Operand tiles sit in shared memory
-// in the no-swizzle K-major core-matrix layout (8 rows x 16 bytes per core
-// matrix; LBO = 128 B between core matrices along K, SBO = 1024 B between
-// 8-row groups).  One thread issues the MMAs and commits them to an mbarrier;
-// the four warps then read the accumulator out of TMEM (warp w owns lanes
-// 32w..32w+31, i.e. rows) and apply the epilogue of the pass:
-//   FWD_SILU  z = acc + b -> Z (FP32), H = silu(z) and H^T (BF16)
-//   LINEAR    y = acc (+ b) -> C (FP32)
-//   BWD_SILU  dz = acc * silu'(Z) -> dZ and dZ^T (BF16), db += column sums
-// The transposed copies make every backward product K-major again:
-//   dH = dZ . W       uses W^T [in][out]   as B
-//   dW = dZ^T . X^T   uses dZ^T [out][batch] as A and X^T [in][batch] as B.
-// Waits on the mbarrier are bounded (about 2 s of SM clock); a wait that
-// runs out sets the error word, skips the rest and still frees the TMEM.
+// rows_kernel takes 128 rows of the batch through the whole network in one
+// launch: the activations stay in shared memory from layer to layer, and the
+// weights stream through a ring of shared-memory stages (one 64-deep K block,
+// up to 32 KB, per cp.async.bulk).  For a training step it goes on through the
+// loss and back through the layers (dZ of every layer), and leaves what the
+// weight gradients need in global memory.  grad_kernel then takes the weight
+// gradients (one CTA per 128 x 64 tile, K = the batch) and applies AdamW to
+// its tile in the epilogue.
+//
+// Products: C[M][N] = A[M][K] . B[N][K]^T with A, B BF16 and K-major, C FP32 in
+// tensor memory, one tcgen05.mma (M = 128, N up to 256, K = 16) per K slice.
+// Operand tiles sit in shared memory in the no-swizzle K-major core-matrix
+// layout (8 rows x 16 bytes per core matrix; LBO = 128 B between core matrices
+// along K, SBO = 1024 B between 8-row groups), and everything a product reads
+// from global memory is stored that way, K block by K block (`packed`), so a
+// stage is one contiguous copy.  Transposed copies (for dW = dZ^T . X) come out
+// of shared memory through ldmatrix.trans, core matrix by core matrix.
+//
+// Warps 0-15 are the epilogue (warp w owns rows 32 (w % 4) .. and columns
+// 64 (w / 4) .. of the accumulator), warp 16 feeds the ring, warp 17 issues the
+// MMAs.  Waits are bounded (about 2 s of SM clock); a wait that runs out sets
+// the error word, and every role leaves its loop, waits for its copies and
+// frees the TMEM.
+//
+// Measured: 2,664 rows forward 404 -> 58 us a call; a training step of 512
+// rows 1,150 -> 210 us.  One GEMM per launch had spent its time in
+// synchronous stages (load, fence, MMA, wait: 5 to 7 us each), in epilogues that
+// wrote rows with a stride, and in 25 launches a step.  What bounds it now is
+// the chain of the layers: the SiLU of 128 x 256 elements, about 3 us of issue
+// slots a layer, and the latency between its parts.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -38,35 +50,32 @@ typedef __nv_bfloat16 bf16;
 
 constexpr int kBM = 128;
 constexpr int kBK = 64;
-constexpr int kThreads = 128;
-constexpr int kInPad = 64;      // 19 input features, zero-padded to one K stage
+constexpr int kInPad = 64;      // 19 input features, zero-padded to one K block
 constexpr int kOutPad = 16;     // 2 outputs, padded to the smallest N
 constexpr int kH = COR_MLP_HIDDEN;
 constexpr int kLayers = COR_MLP_LAYERS + 1;   // 5 weight matrices
-constexpr size_t kSmemBytes = 96 * 1024;     // also caps residency at 2 CTAs/SM (2 x 256 TMEM columns)
 constexpr long long kWaitCycles = 4000000000ll;
 
-enum Mode { FWD_SILU = 0, LINEAR = 1, BWD_SILU = 2 };
+// Bytes of one K block of a packed matrix with `rows` rows.
+__host__ __device__ constexpr uint32_t block_bytes(int rows) { return (uint32_t)rows * kBK * 2; }
 
-struct GemmArgs {
-    const bf16* A;
-    int lda;
-    const bf16* B;
-    int ldb;
-    int M, N, K;
-    int mode;
-    const float* bias;  // LINEAR / FWD_SILU, may be null for LINEAR
-    float* C;           // FP32 out (Z for FWD_SILU, C for LINEAR)
-    int ldc;
-    bf16* H;            // BF16 out, row-major (H or dZ)
-    int ldh;
-    bf16* Ht;           // BF16 out, transposed [N][M]
-    int ldht;
-    const float* Zin;   // BWD_SILU: the pre-activation of the layer
-    int ldz;
-    float* dbias;       // BWD_SILU: column sums accumulate here
-    int* err;
-};
+// Byte offset of element (r, k) in a packed matrix with `rows` rows.
+__host__ __device__ constexpr size_t packed_at(int rows, int r, int k) {
+    return (size_t)(k / kBK) * rows * kBK * 2 + (size_t)(r >> 3) * 1024 + (size_t)((k % kBK) >> 3) * 128 + (r & 7) * 16 +
+           (k & 7) * 2;
+}
+
+// ---- the weight stream of rows_kernel ------------------------------------------
+// Products in order: layers 1 .. 5 forward, then back through W5^T, W4^T, W3^T, W2^T.
+constexpr int kFwdProducts = 5, kProducts = 9;
+__host__ __device__ constexpr int product_n(int p) { return p == 4 ? kOutPad : kH; }
+__host__ __device__ constexpr int product_blocks(int p) { return p == 0 || p == 5 ? 1 : 4; }
+__host__ __device__ constexpr size_t product_bytes(int p) { return (size_t)product_blocks(p) * block_bytes(product_n(p)); }
+__host__ __device__ constexpr size_t product_offset(int p) {
+    size_t o = 0;
+    for (int i = 0; i < p; i++) o += product_bytes(i);
+    return o;
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -106,213 +115,509 @@ __device__ __forceinline__ float silu_grad(float z) {
     return s * (1.f + z * (1.f - s));
 }
 
-// Copies rows [r0, r0+rows) x K columns [k0, k0+64) of a row-major BF16 matrix
-// into the core-matrix layout at `dst`.
-__device__ __forceinline__ void load_tile(uint8_t* dst, const bf16* src, int ld, int r0, int rows, int k0) {
-    for (int v = threadIdx.x; v < rows * 8; v += kThreads) {
-        const int r = v >> 3, c = v & 7;
-        const uint4 x = *reinterpret_cast<const uint4*>(src + (size_t)(r0 + r) * ld + k0 + c * 8);
-        *reinterpret_cast<uint4*>(dst + (r >> 3) * 1024 + c * 128 + (r & 7) * 16) = x;
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+// One contiguous copy into shared memory (16-byte aligned, a multiple of 16 bytes).
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32(bar))
+        : "memory");
+}
+__device__ __forceinline__ void commit_to(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                 : "memory");
+}
+
+// The four K = 16 products of one K block: A 128 rows at a0, B N rows at b0.
+__device__ __forceinline__ void mma_block(uint32_t tmem, uint32_t a0, uint32_t b0, uint32_t idesc, bool first) {
+#pragma unroll
+    for (int s = 0; s < kBK / 16; s++) {
+        const uint64_t ad = smem_desc(a0 + s * 256, 128, 1024);
+        const uint64_t bd = smem_desc(b0 + s * 256, 128, 1024);
+        const uint32_t acc = (!first || s > 0) ? 1u : 0u;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+            "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
     }
 }
 
-__global__ void __launch_bounds__(kThreads) gemm_kernel(const GemmArgs g) {
+__device__ __forceinline__ void tmem_ld16(float* v, uint32_t taddr) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
+        "[%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// 16 values of one row, as BF16, to columns c0 .. c0+15 of a K block in shared memory.
+__device__ __forceinline__ void put_row16(uint8_t* block, int row, int c0, const float* v) {
+    uint32_t w[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const bf16 lo = __float2bfloat16(v[2 * i]), hi = __float2bfloat16(v[2 * i + 1]);
+        w[i] = (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
+    }
+    uint8_t* d = block + (row >> 3) * 1024 + (c0 >> 3) * 128 + (row & 7) * 16;
+    *reinterpret_cast<uint4*>(d) = make_uint4(w[0], w[1], w[2], w[3]);
+    *reinterpret_cast<uint4*>(d + 128) = make_uint4(w[4], w[5], w[6], w[7]);
+}
+
+// The transpose of this warp's 32 rows (quadrant q of the tile) and `cols`
+// columns of a K block in shared memory, to the packed matrix [feature][batch]
+// at `dst` with R features: features f0 .., batch b0 ...
+__device__ __forceinline__ void put_transposed(uint8_t* dst, int R, int f0, int b0, const uint8_t* block, int q, int cols) {
+    const int lane = threadIdx.x & 31;
+    for (int c8 = 0; c8 < cols / 8; c8++) {
+        // four core matrices: rows 32q .. 32q+31 of columns 8 c8 ..
+        const uint32_t a = smem_u32(block + (4 * q + (lane >> 3)) * 1024 + c8 * 128 + (lane & 7) * 16);
+        uint32_t r[4];
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(a)
+                     : "memory");
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int b = b0 + 32 * q + 8 * k;
+            *reinterpret_cast<uint32_t*>(dst + packed_at(R, f0 + 8 * c8, b) + lane * 4) = r[k];
+        }
+    }
+}
+
+constexpr int kEpiWarps = 16, kRowsThreads = 32 * (kEpiWarps + 2);
+constexpr int kRing = 4;
+constexpr uint32_t kStageBytes = block_bytes(kH);
+constexpr uint32_t kABytes = 4 * block_bytes(kBM);
+constexpr size_t kRowsSmem = 1024 + kABytes + kRing * kStageBytes;
+
+struct RowsArgs {
+    const float* x;          // n x 19
+    const float* target;     // n x 2 (training)
+    int n;
+    float* y;                // n x 2 (inference)
+    const uint8_t* weights;  // the weight stream
+    const float* bias[kLayers];
+    // training
+    float* z[COR_MLP_LAYERS];       // [tile][column][row]
+    uint8_t* x0t;                   // packed [64][bt]
+    uint8_t* ht[COR_MLP_LAYERS];    // packed [256][bt]
+    uint8_t* dzt[COR_MLP_LAYERS];   // packed [256][bt]
+    uint8_t* dyt;                   // packed [16][bt]
+    float* gb[kLayers];             // bias gradients, zero at launch
+    float* loss;                    // zero at launch
+    int* err;
+};
+
+struct RowsShared {
+    uint64_t full[kRing], empty[kRing], acc, a_ready;
+    uint32_t tmem;
+};
+static_assert(sizeof(RowsShared) <= 1024, "rows_kernel header");
+
+template <bool TRAIN>
+__global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const RowsArgs g) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* sa = smem;                       // 128 x 64 BF16 = 16 KB
-    uint8_t* sb = smem + 16 * 1024;           // N x 64 BF16 <= 32 KB
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 48 * 1024);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 48 * 1024 + 64);
+    RowsShared& sh = *reinterpret_cast<RowsShared*>(smem);
+    uint8_t* sa = smem + 1024;
+    uint8_t* ring = sa + kABytes;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.x * kBM;
-    uint32_t ncols = 32;
-    while ((int)ncols < g.N) ncols <<= 1;
+    constexpr int kLast = TRAIN ? kProducts : kFwdProducts;
+    constexpr uint32_t kCols = 256;
 
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)));
+        for (int k = 0; k < kRing; k++) {
+            mbar_init(&sh.full[k], 1);
+            mbar_init(&sh.empty[k], 1);
+        }
+        mbar_init(&sh.acc, 1);
+        mbar_init(&sh.a_ready, 32 * kEpiWarps);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(ncols));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem)),
+                     "r"(kCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
-    const uint32_t idesc = instr_desc(kBM, g.N);
-
+    const uint32_t tmem = sh.tmem;
     bool ok = true;
-    const int kb_n = g.K / kBK;
-    for (int kb = 0; kb < kb_n && ok; kb++) {
-        load_tile(sa, g.A, g.lda, m0, kBM, kb * kBK);
-        load_tile(sb, g.B, g.ldb, 0, g.N, kb * kBK);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t a0 = smem_u32(sa), b0 = smem_u32(sb);
-#pragma unroll
-            for (int s = 0; s < kBK / 16; s++) {
-                const uint64_t ad = smem_desc(a0 + s * 256, 128, 1024);
-                const uint64_t bd = smem_desc(b0 + s * 256, 128, 1024);
-                const uint32_t acc = (kb > 0 || s > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-                    "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(bar))
-                         : "memory");
-        }
-        ok = mbar_wait(bar, (uint32_t)(kb & 1));
-        if (!ok) atomicExch(g.err, 1);
-        // the MMAs of this stage are complete: the tiles may be overwritten
-        __syncthreads();
-        ok = __syncthreads_and(ok);
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
-    if (ok) {
-        const int row = m0 + warp * 32 + lane;
-        for (int c0 = 0; c0 < g.N; c0 += 16) {
-            uint32_t r[16];
-            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
-                "[%16];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                  "=r"(r[15])
-                : "r"(taddr));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    if (warp == kEpiWarps) {
+        if (lane == 0) {
+            int s = 0;
+            for (int p = 0; p < kLast && ok; p++) {
+                const uint32_t bytes = block_bytes(product_n(p));
+                const uint8_t* src = g.weights + product_offset(p);
+                for (int kb = 0; kb < product_blocks(p) && ok; kb++, s++) {
+                    const int k = s % kRing;
+                    if (s >= kRing) ok = mbar_wait(&sh.empty[k], (uint32_t)((s / kRing - 1) & 1));
+                    if (!ok) break;
+                    mbar_expect(&sh.full[k], bytes);
+                    bulk_load(ring + k * kStageBytes, src + (size_t)kb * bytes, bytes, &sh.full[k]);
+                }
+            }
+            if (!ok) {
+                atomicExch(g.err, 1);
+                // the copies in flight land before the block leaves
+                for (int i = s > kRing ? s - kRing : 0; i < s; i++)
+                    mbar_wait(&sh.full[i % kRing], (uint32_t)((i / kRing) & 1));
+            }
+        }
+    } else if (warp == kEpiWarps + 1) {
+        if (lane == 0) {
+            int s = 0;
+            for (int p = 0; p < kLast && ok; p++) {
+                const uint32_t idesc = instr_desc(kBM, product_n(p));
+                ok = mbar_wait(&sh.a_ready, (uint32_t)(p & 1));
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int kb = 0; kb < product_blocks(p) && ok; kb++, s++) {
+                    const int k = s % kRing;
+                    ok = mbar_wait(&sh.full[k], (uint32_t)((s / kRing) & 1));
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    mma_block(tmem, smem_u32(sa + kb * block_bytes(kBM)), smem_u32(ring + k * kStageBytes), idesc, kb == 0);
+                    commit_to(&sh.empty[k]);
+                }
+                if (ok) commit_to(&sh.acc);
+            }
+            if (!ok) atomicExch(g.err, 1);
+        }
+    } else {
+        const int q = warp & 3, cg = warp >> 2;
+        const int row = 32 * q + lane;
+        const int gr = m0 + row;
+        const bool valid = gr < g.n;
+        const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16);
+        // the input: 16 columns per column group
+        {
             float v[16];
 #pragma unroll
-            for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
-            if (g.mode == FWD_SILU) {
+            for (int i = 0; i < 16; i++) {
+                const int c = 16 * cg + i;
+                v[i] = valid && c < COR_MLP_IN ? g.x[(size_t)gr * COR_MLP_IN + c] : 0.f;
+            }
+            put_row16(sa, row, 16 * cg, v);
+            if (TRAIN) {
+                __syncwarp();
+                put_transposed(g.x0t, kInPad, 16 * cg, m0, sa + 2 * cg * 128, q, 16);
+            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_arrive(&sh.a_ready);
+        for (int p = 0; p < kLast; p++) {
+            ok = mbar_wait(&sh.acc, (uint32_t)(p & 1));
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            uint8_t* block = sa + cg * block_bytes(kBM);
+            if (p < COR_MLP_LAYERS) {
+                for (int c0 = 0; c0 < 64; c0 += 16) {
+                    float v[16];
+                    tmem_ld16(v, trow + 64 * cg + c0);
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const int c = c0 + i;
-                    const float z = v[i] + g.bias[c];
-                    g.C[(size_t)row * g.ldc + c] = z;
-                    const bf16 h = __float2bfloat16(silu(z));
-                    g.H[(size_t)row * g.ldh + c] = h;
-                    g.Ht[(size_t)c * g.ldht + row] = h;
+                    for (int i = 0; i < 16; i++) {
+                        const int c = 64 * cg + c0 + i;
+                        const float z = v[i] + g.bias[p][c];
+                        if (TRAIN) g.z[p][((size_t)blockIdx.x * kH + c) * kBM + row] = z;
+                        v[i] = silu(z);
+                    }
+                    put_row16(block, row, c0, v);
                 }
-            } else if (g.mode == LINEAR) {
+                if (TRAIN) {
+                    __syncwarp();
+                    put_transposed(g.ht[p], kH, 64 * cg, m0, block, q, 64);
+                }
+            } else if (p == COR_MLP_LAYERS) {
+                if (cg == 0) {
+                    float v[16];
+                    tmem_ld16(v, trow);
+                    const float y0 = v[0] + g.bias[4][0], y1 = v[1] + g.bias[4][1];
+                    if (!TRAIN) {
+                        if (valid) {
+                            g.y[2 * (size_t)gr] = y0;
+                            g.y[2 * (size_t)gr + 1] = y1;
+                        }
+                    } else {
+                        // mean squared error over the n rows and 2 outputs
+                        const float scale = 2.f / (float)(g.n * COR_MLP_OUT);
+                        float e0 = 0.f, e1 = 0.f;
+                        if (valid) {
+                            e0 = y0 - g.target[2 * (size_t)gr];
+                            e1 = y1 - g.target[2 * (size_t)gr + 1];
+                        }
+                        float l = (e0 * e0 + e1 * e1) / (float)(g.n * COR_MLP_OUT);
+                        float d0 = scale * e0, d1 = scale * e1;
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const int c = c0 + i;
-                    g.C[(size_t)row * g.ldc + c] = v[i] + (g.bias ? g.bias[c] : 0.f);
+                        for (int i = 0; i < 16; i++) v[i] = i == 0 ? d0 : i == 1 ? d1 : 0.f;
+                        put_row16(sa, row, 0, v);
+                        v[0] = v[1] = 0.f;
+                        for (int c0 = 16; c0 < 64; c0 += 16) put_row16(sa, row, c0, v);
+                        __syncwarp();
+                        put_transposed(g.dyt, kOutPad, 0, m0, sa, q, 16);
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) {
+                            l += __shfl_xor_sync(0xffffffffu, l, o);
+                            d0 += __shfl_xor_sync(0xffffffffu, d0, o);
+                            d1 += __shfl_xor_sync(0xffffffffu, d1, o);
+                        }
+                        if (lane == 0) {
+                            atomicAdd(g.loss, l);
+                            atomicAdd(g.gb[4], d0);
+                            atomicAdd(g.gb[4] + 1, d1);
+                        }
+                    }
                 }
             } else {
+                const int l = kProducts - 1 - p;   // dZ of layer l + 1
+                for (int c0 = 0; c0 < 64; c0 += 16) {
+                    float v[16];
+                    tmem_ld16(v, trow + 64 * cg + c0);
+#pragma unroll
+                    for (int i = 0; i < 16; i++) {
+                        const int c = 64 * cg + c0 + i;
+                        v[i] = v[i] * silu_grad(g.z[l][((size_t)blockIdx.x * kH + c) * kBM + row]);
+                    }
+                    put_row16(block, row, c0, v);
+                    // column sums over the warp's 32 rows: lanes 2c and 2c+1 end with column c's
+#pragma unroll
+                    for (int o = 16, m = 8; m > 0; o >>= 1, m >>= 1) {
+                        const bool up = (lane & o) != 0;
+#pragma unroll
+                        for (int i = 0; i < m; i++) {
+                            const float give = up ? v[i] : v[i + m];
+                            v[i] = (up ? v[i + m] : v[i]) + __shfl_xor_sync(0xffffffffu, give, o);
+                        }
+                    }
+                    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+                    if ((lane & 1) == 0) atomicAdd(g.gb[l] + 64 * cg + c0 + (lane >> 1), v[0]);
+                }
+                __syncwarp();
+                put_transposed(g.dzt[l], kH, 64 * cg, m0, block, q, 64);
+            }
+            if (p + 1 < kLast) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                mbar_arrive(&sh.a_ready);
+            }
+        }
+        if (!ok) atomicExch(g.err, 1);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
+}
+
+// ---- weight gradients and AdamW ---------------------------------------------------
+constexpr int kGradN = 64;                                   // columns of a tile
+constexpr int kGradTiles = 2 + 3 * 2 * (kH / kGradN) + 2;    // W1: 2, W2-W4: 8 each, W5: 2
+constexpr int kGradThreads = 32 * 10;                        // 8 epilogue warps, the ring's feeder, the MMAs' issuer
+constexpr int kGradRing = 6;
+constexpr uint32_t kGradStage = block_bytes(kBM) + block_bytes(kGradN);
+constexpr size_t kGradSmem = 1024 + kGradRing * kGradStage;
+
+struct GradArgs {
+    const uint8_t* x0t;
+    const uint8_t* ht[COR_MLP_LAYERS];
+    const uint8_t* dzt[COR_MLP_LAYERS];
+    const uint8_t* dyt;
+    int blocks;              // K blocks: batch / 64
+    float* w;                // parameters, moments: the packed parameter order
+    float* m;
+    float* v;
+    const float* gb[kLayers];
+    const float* loss;       // the batch's loss, copied to loss_out
+    float* loss_out;
+    float* grads;            // packed gradient export (may be null)
+    uint8_t* weights;        // the weight stream
+    float lr, b1c, b2c, decay;
+    int update;
+    int* err;
+};
+
+// Offsets of each tensor in the packed parameter order.
+__host__ __device__ constexpr int layer_in(int l) { return l == 0 ? COR_MLP_IN : kH; }
+__host__ __device__ constexpr int layer_out(int l) { return l == 4 ? COR_MLP_OUT : kH; }
+__host__ __device__ constexpr int weight_at(int l) {
+    int o = 0;
+    for (int i = 0; i < l; i++) o += layer_out(i) * layer_in(i) + layer_out(i);
+    return o;
+}
+__host__ __device__ constexpr int bias_at(int l) { return weight_at(l) + layer_out(l) * layer_in(l); }
+
+// W(l) element (r, c) into the BF16 copies the products read.
+__device__ __forceinline__ void store_weight(uint8_t* stream, int l, int r, int c, float w) {
+    const bf16 b = __float2bfloat16(w);
+    *reinterpret_cast<bf16*>(stream + product_offset(l) + packed_at(product_n(l), r, c)) = b;
+    if (l > 0) *reinterpret_cast<bf16*>(stream + product_offset(9 - l) + packed_at(kH, c, r)) = b;
+}
+
+// AdamW on parameter i with gradient gr; returns the new value.
+__device__ __forceinline__ float adamw(const GradArgs& g, int i, float gr, float decay) {
+    const float m = 0.9f * g.m[i] + 0.1f * gr;
+    const float v = 0.999f * g.v[i] + 0.001f * gr * gr;
+    g.m[i] = m;
+    g.v[i] = v;
+    float w = g.w[i];
+    w -= g.lr * ((m / g.b1c) / (sqrtf(v / g.b2c) + 1e-8f) + decay * w);
+    g.w[i] = w;
+    return w;
+}
+
+// One tile of a weight gradient (blocks 0 .. kGradTiles - 1), or the biases (the last block).
+__global__ void __launch_bounds__(kGradThreads, 1) grad_kernel(const GradArgs g) {
+    if (blockIdx.x == kGradTiles) {
+        for (int l = 0; l < kLayers; l++)
+            for (int r = threadIdx.x; r < layer_out(l); r += kGradThreads) {
+                const float gr = g.gb[l][r];
+                if (g.grads) g.grads[bias_at(l) + r] = gr;
+                if (g.update) adamw(g, bias_at(l) + r, gr, 0.f);
+            }
+        if (threadIdx.x == 0) *g.loss_out = *g.loss;
+        return;
+    }
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ uint64_t full[kGradRing], empty[kGradRing], accb;
+    __shared__ uint32_t s_tmem;
+    uint8_t* ring = smem + 1024;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // tile -> layer, M tile, N tile: C[m][n] = A[m][batch] . B[n][batch]^T
+    int l, mt, n0 = 0, N = kGradN;
+    const uint8_t *A, *B;
+    int b_rows;
+    if (blockIdx.x < 2) {
+        l = 0;
+        mt = blockIdx.x;
+        A = g.dzt[0];
+        B = g.x0t;
+        b_rows = kInPad;
+    } else if (blockIdx.x < kGradTiles - 2) {
+        const int t = blockIdx.x - 2, per = 2 * (kH / kGradN);
+        l = 1 + t / per;
+        mt = (t % per) & 1;
+        n0 = (t % per) / 2 * kGradN;
+        A = g.dzt[l];
+        B = g.ht[l - 1];
+        b_rows = kH;
+    } else {
+        l = 4;
+        mt = blockIdx.x - (kGradTiles - 2);
+        A = g.ht[3];
+        B = g.dyt;
+        b_rows = kOutPad;
+        N = kOutPad;
+    }
+    A += (size_t)mt * block_bytes(kBM);
+    B += (size_t)n0 * kBK * 2;
+    constexpr uint32_t kCols = 64;
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < kGradRing; k++) {
+            mbar_init(&full[k], 1);
+            mbar_init(&empty[k], 1);
+        }
+        mbar_init(&accb, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
+                     "r"(kCols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    bool ok = true;
+    if (warp == 8) {
+        if (lane == 0) {
+            int s = 0;
+            for (; s < g.blocks; s++) {
+                const int k = s % kGradRing;
+                if (s >= kGradRing) ok = mbar_wait(&empty[k], (uint32_t)((s / kGradRing - 1) & 1));
+                if (!ok) break;
+                mbar_expect(&full[k], block_bytes(kBM) + block_bytes(N));
+                uint8_t* d = ring + k * kGradStage;
+                bulk_load(d, A + (size_t)s * block_bytes(kH), block_bytes(kBM), &full[k]);
+                bulk_load(d + block_bytes(kBM), B + (size_t)s * block_bytes(b_rows), block_bytes(N), &full[k]);
+            }
+            if (!ok) {
+                atomicExch(g.err, 1);
+                for (int i = s > kGradRing ? s - kGradRing : 0; i < s; i++)
+                    mbar_wait(&full[i % kGradRing], (uint32_t)((i / kGradRing) & 1));
+            }
+        }
+    } else if (warp == 9) {
+        if (lane == 0) {
+            const uint32_t idesc = instr_desc(kBM, N);
+            for (int s = 0; s < g.blocks && ok; s++) {
+                const int k = s % kGradRing;
+                ok = mbar_wait(&full[k], (uint32_t)((s / kGradRing) & 1));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t a0 = smem_u32(ring + k * kGradStage);
+                mma_block(tmem, a0, a0 + block_bytes(kBM), idesc, s == 0);
+                commit_to(&empty[k]);
+            }
+            if (ok) commit_to(&accb);
+            else atomicExch(g.err, 1);
+        }
+    } else {
+        ok = mbar_wait(&accb, 0);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+            atomicExch(g.err, 1);
+        } else {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int q = warp & 3, cg = warp >> 2;
+            const int row = mt * kBM + 32 * q + lane;
+            for (int c0 = 32 * cg; c0 < 32 * cg + 32 && c0 < N; c0 += 16) {
+                float v[16];
+                tmem_ld16(v, tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)c0);
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
-                    const int c = c0 + i;
-                    const float d = v[i] * silu_grad(g.Zin[(size_t)row * g.ldz + c]);
-                    const bf16 h = __float2bfloat16(d);
-                    g.H[(size_t)row * g.ldh + c] = h;
-                    g.Ht[(size_t)c * g.ldht + row] = h;
-                    float s = d;
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                    if (lane == 0) atomicAdd(g.dbias + c, s);
+                    const int col = n0 + c0 + i;
+                    const int r = l == 4 ? col : row, c = l == 4 ? row : col;
+                    if (r < layer_out(l) && c < layer_in(l)) {
+                        const int at = weight_at(l) + r * layer_in(l) + c;
+                        if (g.grads) g.grads[at] = v[i];
+                        if (g.update) store_weight(g.weights, l, r, c, adamw(g, at, v[i], g.decay));
+                    }
                 }
             }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
 }
 
-// ---- element-wise kernels -------------------------------------------------------
-// features (n x 19 FP32) -> X0 (Bt x 64 BF16, zero-padded rows and columns)
-// and X0^T (64 x Bt)
-__global__ void input_kernel(const float* __restrict__ x, int n, int bt, bf16* __restrict__ x0,
-                             bf16* __restrict__ x0t) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= bt * kInPad) return;
-    const int r = i / kInPad, c = i % kInPad;
-    const float v = (r < n && c < COR_MLP_IN) ? x[(size_t)r * COR_MLP_IN + c] : 0.f;
-    const bf16 b = __float2bfloat16(v);
-    x0[i] = b;
-    x0t[(size_t)c * bt + r] = b;
-}
-
-// mean squared error over the n valid rows and COR_MLP_OUT outputs, its
-// gradient dY (Bt x 64, zero outside), dY^T (16 x Bt) and db5
-__global__ void loss_kernel(const float* __restrict__ y, const float* __restrict__ t, int n, int bt,
-                            bf16* __restrict__ dy, bf16* __restrict__ dyt, float* __restrict__ db5,
-                            float* __restrict__ loss) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= bt) return;
-    const float scale = 2.f / (float)(n * COR_MLP_OUT);
-    float l = 0.f;
-    for (int c = 0; c < kInPad; c++) {
-        float d = 0.f;
-        if (r < n && c < COR_MLP_OUT) {
-            const float e = y[(size_t)r * kOutPad + c] - t[(size_t)r * COR_MLP_OUT + c];
-            l += e * e;
-            d = scale * e;
-            atomicAdd(db5 + c, d);
+// Every weight into its BF16 copies.
+__global__ void cast_kernel(const float* __restrict__ w, uint8_t* __restrict__ weights) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int l = 0; l < kLayers; l++) {
+        const int n = layer_out(l) * layer_in(l);
+        if (i < n) {
+            store_weight(weights, l, i / layer_in(l), i % layer_in(l), w[weight_at(l) + i]);
+            return;
         }
-        dy[(size_t)r * kInPad + c] = __float2bfloat16(d);
-        if (c < kOutPad) dyt[(size_t)c * bt + r] = __float2bfloat16(d);
+        i -= n;
     }
-    if (r < n) atomicAdd(loss, l / (float)(n * COR_MLP_OUT));
-}
-
-__global__ void copy_out_kernel(const float* __restrict__ y, int n, float* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n * COR_MLP_OUT) return;
-    out[i] = y[(size_t)(i / COR_MLP_OUT) * kOutPad + i % COR_MLP_OUT];
-}
-
-// One weight matrix or bias vector: FP32 master, moments, gradient source and
-// the BF16 copies the GEMMs read.
-struct ParamView {
-    float* w;          // master [rows][cols]
-    float* m;
-    float* v;
-    const float* g;    // gradient
-    int g_transposed;  // gradient stored [cols][g_ld] (layer 5)
-    int g_ld;
-    int rows, cols;
-    bf16* wb;          // [rows][wb_ld] zero-padded   (null for biases)
-    int wb_ld;
-    bf16* wt;          // [cols][wt_ld] zero-padded   (null for biases)
-    int wt_ld;
-    float* gout;       // packed gradient export (may be null)
-    float decay;
-};
-
-__global__ void adamw_kernel(ParamView p, float lr, float b1c, float b2c, int update) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.rows * p.cols) return;
-    const int r = i / p.cols, c = i % p.cols;
-    const float g = p.g_transposed ? p.g[(size_t)c * p.g_ld + r] : p.g[(size_t)r * p.g_ld + c];
-    if (p.gout) p.gout[i] = g;
-    if (!update) return;
-    const float m = 0.9f * p.m[i] + 0.1f * g;
-    const float v = 0.999f * p.v[i] + 0.001f * g * g;
-    p.m[i] = m;
-    p.v[i] = v;
-    float w = p.w[i];
-    w -= lr * ((m / b1c) / (sqrtf(v / b2c) + 1e-8f) + p.decay * w);
-    p.w[i] = w;
-    if (p.wb) p.wb[(size_t)r * p.wb_ld + c] = __float2bfloat16(w);
-    if (p.wt) p.wt[(size_t)c * p.wt_ld + r] = __float2bfloat16(w);
-}
-
-__global__ void cast_kernel(ParamView p) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.rows * p.cols) return;
-    const int r = i / p.cols, c = i % p.cols;
-    if (p.wb) p.wb[(size_t)r * p.wb_ld + c] = __float2bfloat16(p.w[i]);
-    if (p.wt) p.wt[(size_t)c * p.wt_ld + r] = __float2bfloat16(p.w[i]);
 }
 
 }  // namespace mlp
@@ -324,19 +629,16 @@ struct cor_mlp {
     int max_bt = 0;
     char err[256] = {0};
     int step = 0;
-    void* block = nullptr;      // one allocation holds every buffer
-    float *w[kLayers], *b[kLayers], *mw[kLayers], *vw[kLayers], *mb[kLayers], *vb[kLayers];
-    float *gw[kLayers], *gb[kLayers];
-    bf16 *wb[kLayers], *wt[kLayers];
-    bf16 *x0, *x0t, *h[COR_MLP_LAYERS], *ht[COR_MLP_LAYERS], *dz, *dzt, *dz2, *dz2t, *dy, *dyt;
-    float *z[COR_MLP_LAYERS], *y;
-    int* dev_err = nullptr;
+    void* block = nullptr;      // one allocation holds every device buffer
+    float *w, *mom, *vel;       // parameters and moments, the packed parameter order
+    uint8_t* weights;           // BF16 copies in the order the products read them
+    float* gb[kLayers];         // bias gradients, then the batch's loss
+    float* loss;
+    float* z[COR_MLP_LAYERS];
+    uint8_t *x0t, *ht[COR_MLP_LAYERS], *dzt[COR_MLP_LAYERS], *dyt;
+    int* err_h = nullptr;       // mapped: set by a wait that ran out
+    int* err_d = nullptr;
 };
-
-static const int kIn[kLayers] = {COR_MLP_IN, kH, kH, kH, kH};
-static const int kOut[kLayers] = {kH, kH, kH, kH, COR_MLP_OUT};
-static const int kInP[kLayers] = {kInPad, kH, kH, kH, kH};
-static const int kOutP[kLayers] = {kH, kH, kH, kH, kOutPad};
 
 static int mfail(cor_mlp* m, int code, const char* fmt, ...) {
     if (m) {
@@ -354,150 +656,31 @@ static int mfail(cor_mlp* m, int code, const char* fmt, ...) {
         if (e_ != cudaSuccess) return mfail((m), COR_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
 
-static int gemm(cor_mlp* m, GemmArgs g, cudaStream_t s) {
-    if (g.M % kBM || g.N % 16 || g.N < 16 || g.N > 256 || g.K % kBK || g.K <= 0 || g.lda % 8 || g.ldb % 8)
-        return mfail(m, COR_ERR_INVALID, "gemm shape %d x %d x %d not supported", g.M, g.N, g.K);
-    g.err = m->dev_err;
-    gemm_kernel<<<g.M / kBM, kThreads, kSmemBytes, s>>>(g);
-    MTRY(m, cudaGetLastError());
-    return COR_OK;
-}
+static const size_t kGbBytes = sizeof(float) * (kLayers * kH + 64);
 
-static int forward(cor_mlp* m, const float* x, int n, int bt, cudaStream_t s) {
-    const int th = 256;
-    input_kernel<<<(bt * kInPad + th - 1) / th, th, 0, s>>>(x, n, bt, m->x0, m->x0t);
-    MTRY(m, cudaGetLastError());
-    const bf16* in = m->x0;
-    int in_ld = kInPad;
+static RowsArgs rows_args(const cor_mlp* m, const float* x, int n) {
+    RowsArgs g = {};
+    g.x = x;
+    g.n = n;
+    g.weights = m->weights;
+    for (int l = 0; l < kLayers; l++) {
+        g.bias[l] = m->w + bias_at(l);
+        g.gb[l] = m->gb[l];
+    }
     for (int l = 0; l < COR_MLP_LAYERS; l++) {
-        GemmArgs g = {};
-        g.A = in;
-        g.lda = in_ld;
-        g.B = m->wb[l];
-        g.ldb = kInP[l];
-        g.M = bt;
-        g.N = kH;
-        g.K = kInP[l];
-        g.mode = FWD_SILU;
-        g.bias = m->b[l];
-        g.C = m->z[l];
-        g.ldc = kH;
-        g.H = m->h[l];
-        g.ldh = kH;
-        g.Ht = m->ht[l];
-        g.ldht = bt;
-        int rc = gemm(m, g, s);
-        if (rc != COR_OK) return rc;
-        in = m->h[l];
-        in_ld = kH;
+        g.z[l] = m->z[l];
+        g.ht[l] = m->ht[l];
+        g.dzt[l] = m->dzt[l];
     }
-    GemmArgs g = {};
-    g.A = in;
-    g.lda = kH;
-    g.B = m->wb[4];
-    g.ldb = kH;
-    g.M = bt;
-    g.N = kOutPad;
-    g.K = kH;
-    g.mode = LINEAR;
-    g.bias = m->b[4];
-    g.C = m->y;
-    g.ldc = kOutPad;
-    return gemm(m, g, s);
-}
-
-static int backward(cor_mlp* m, const float* t, int n, int bt, float* loss, cudaStream_t s) {
-    for (int l = 0; l < kLayers; l++) MTRY(m, cudaMemsetAsync(m->gb[l], 0, sizeof(float) * kOut[l], s));
-    MTRY(m, cudaMemsetAsync(loss, 0, sizeof(float), s));
-    loss_kernel<<<(bt + 127) / 128, 128, 0, s>>>(m->y, t, n, bt, m->dy, m->dyt, m->gb[4], loss);
-    MTRY(m, cudaGetLastError());
-    int rc;
-    {   // dW5^T [256][16] = H4^T . dY^T
-        GemmArgs g = {};
-        g.A = m->ht[3]; g.lda = bt; g.B = m->dyt; g.ldb = bt;
-        g.M = kH; g.N = kOutPad; g.K = bt; g.mode = LINEAR; g.C = m->gw[4]; g.ldc = kOutPad;
-        if ((rc = gemm(m, g, s)) != COR_OK) return rc;
-    }
-    // dZ4 = (dY . W5) * silu'(Z4); W5^T is [256][64] (zero beyond the 2 outputs)
-    const bf16* up = m->dy;
-    int up_ld = kInPad;
-    int up_k = kInPad;
-    bf16* dzb[2] = {m->dz, m->dz2};
-    bf16* dztb[2] = {m->dzt, m->dz2t};
-    for (int l = COR_MLP_LAYERS - 1; l >= 0; l--) {
-        const int cur = l & 1;
-        GemmArgs g = {};
-        g.A = up; g.lda = up_ld; g.B = m->wt[l + 1]; g.ldb = up_k;
-        g.M = bt; g.N = kH; g.K = up_k; g.mode = BWD_SILU;
-        g.Zin = m->z[l]; g.ldz = kH; g.H = dzb[cur]; g.ldh = kH; g.Ht = dztb[cur]; g.ldht = bt;
-        g.dbias = m->gb[l];
-        if ((rc = gemm(m, g, s)) != COR_OK) return rc;
-        // dW_l [256][in_pad] = dZ_l^T . X_{l-1}^T
-        GemmArgs w = {};
-        w.A = dztb[cur]; w.lda = bt; w.B = l == 0 ? m->x0t : m->ht[l - 1]; w.ldb = bt;
-        w.M = kH; w.N = kInP[l]; w.K = bt; w.mode = LINEAR; w.C = m->gw[l]; w.ldc = kInP[l];
-        if ((rc = gemm(m, w, s)) != COR_OK) return rc;
-        up = dzb[cur];
-        up_ld = kH;
-        up_k = kH;
-    }
-    return COR_OK;
-}
-
-static ParamView view(cor_mlp* m, int l, bool bias, float* gout) {
-    ParamView p = {};
-    if (!bias) {
-        p.w = m->w[l]; p.m = m->mw[l]; p.v = m->vw[l];
-        p.g = m->gw[l];
-        p.g_transposed = l == 4;
-        p.g_ld = l == 4 ? kOutPad : kInP[l];
-        p.rows = kOut[l]; p.cols = kIn[l];
-        p.wb = m->wb[l]; p.wb_ld = kInP[l];
-        p.wt = m->wt[l]; p.wt_ld = l == 4 ? kInPad : kOutP[l];
-        p.decay = 1.f;
-    } else {
-        p.w = m->b[l]; p.m = m->mb[l]; p.v = m->vb[l];
-        p.g = m->gb[l]; p.g_ld = 1;
-        p.rows = kOut[l]; p.cols = 1;
-        p.decay = 0.f;
-    }
-    p.gout = gout;
-    return p;
-}
-
-// offsets of each tensor in the packed parameter layout
-static void param_offsets(size_t* wo, size_t* bo) {
-    size_t o = 0;
-    for (int l = 0; l < kLayers; l++) {
-        wo[l] = o;
-        o += (size_t)kOut[l] * kIn[l];
-        bo[l] = o;
-        o += kOut[l];
-    }
-}
-
-static int update(cor_mlp* m, float lr, float wd, float* grads, int do_update, cudaStream_t s) {
-    size_t wo[kLayers], bo[kLayers];
-    param_offsets(wo, bo);
-    if (do_update) m->step++;
-    const float b1c = 1.f - powf(0.9f, (float)(m->step > 0 ? m->step : 1));
-    const float b2c = 1.f - powf(0.999f, (float)(m->step > 0 ? m->step : 1));
-    for (int l = 0; l < kLayers; l++) {
-        for (int bias = 0; bias < 2; bias++) {
-            ParamView p = view(m, l, bias, grads ? grads + (bias ? bo[l] : wo[l]) : nullptr);
-            if (!bias) p.decay = wd;
-            const int n = p.rows * p.cols;
-            adamw_kernel<<<(n + 255) / 256, 256, 0, s>>>(p, lr, b1c, b2c, do_update);
-            MTRY(m, cudaGetLastError());
-        }
-    }
-    return COR_OK;
+    g.x0t = m->x0t;
+    g.dyt = m->dyt;
+    g.loss = m->loss;
+    g.err = m->err_d;
+    return g;
 }
 
 static int check_err(cor_mlp* m) {
-    int e = 0;
-    MTRY(m, cudaMemcpy(&e, m->dev_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (e) return mfail(m, COR_ERR_WATCHDOG, "a tensor-core wait ran out of time");
+    if (*(volatile int*)m->err_h) return mfail(m, COR_ERR_WATCHDOG, "a tensor-core wait ran out of time");
     return COR_OK;
 }
 
@@ -526,54 +709,50 @@ int cor_mlp_create(int device, int32_t max_batch, cor_mlp** out) {
         total += (bytes + 255) & ~(size_t)255;
         return o;
     };
-    size_t ow[kLayers], ob[kLayers], omw[kLayers], ovw[kLayers], omb[kLayers], ovb[kLayers], ogw[kLayers],
-        ogb[kLayers], owb[kLayers], owt[kLayers];
-    for (int l = 0; l < kLayers; l++) {
-        const size_t nw = (size_t)kOut[l] * kIn[l];
-        ow[l] = take(4 * nw); omw[l] = take(4 * nw); ovw[l] = take(4 * nw);
-        ob[l] = take(4 * kOut[l]); omb[l] = take(4 * kOut[l]); ovb[l] = take(4 * kOut[l]);
-        ogw[l] = take(4 * (size_t)kOutP[l] * kInP[l] + 4 * (size_t)kH * kOutPad);
-        ogb[l] = take(4 * (size_t)kOutP[l]);
-        owb[l] = take(2 * (size_t)kOutP[l] * kInP[l]);
-        owt[l] = take(2 * (size_t)kInP[l] * (l == 4 ? kInPad : kOutP[l]));
-    }
-    const size_t ox0 = take(2 * bt * kInPad), ox0t = take(2 * bt * kInPad);
-    size_t oh[COR_MLP_LAYERS], oht[COR_MLP_LAYERS], oz[COR_MLP_LAYERS];
+    const size_t ow = take(4 * COR_MLP_PARAMS), om = take(4 * COR_MLP_PARAMS), ov = take(4 * COR_MLP_PARAMS);
+    const size_t owt = take(product_offset(kProducts));
+    const size_t ogb = take(kGbBytes);
+    size_t oz[COR_MLP_LAYERS], oht[COR_MLP_LAYERS], odz[COR_MLP_LAYERS];
     for (int l = 0; l < COR_MLP_LAYERS; l++) {
-        oh[l] = take(2 * bt * kH);
-        oht[l] = take(2 * bt * kH);
         oz[l] = take(4 * bt * kH);
+        oht[l] = take(2 * bt * kH);
+        odz[l] = take(2 * bt * kH);
     }
-    const size_t odz = take(2 * bt * kH), odzt = take(2 * bt * kH), odz2 = take(2 * bt * kH),
-                 odz2t = take(2 * bt * kH);
-    const size_t ody = take(2 * bt * kInPad), odyt = take(2 * bt * kOutPad), oy = take(4 * bt * kOutPad);
-    const size_t oerr = take(sizeof(int));
+    const size_t ox = take(2 * bt * kInPad), ody = take(2 * bt * kOutPad);
     if (cudaMalloc(&m->block, total) != cudaSuccess) {
         delete m;
         return COR_ERR_NOMEM;
     }
-    cudaMemset(m->block, 0, total);
     uint8_t* B = (uint8_t*)m->block;
-    for (int l = 0; l < kLayers; l++) {
-        m->w[l] = (float*)(B + ow[l]); m->mw[l] = (float*)(B + omw[l]); m->vw[l] = (float*)(B + ovw[l]);
-        m->b[l] = (float*)(B + ob[l]); m->mb[l] = (float*)(B + omb[l]); m->vb[l] = (float*)(B + ovb[l]);
-        m->gw[l] = (float*)(B + ogw[l]); m->gb[l] = (float*)(B + ogb[l]);
-        m->wb[l] = (bf16*)(B + owb[l]); m->wt[l] = (bf16*)(B + owt[l]);
-    }
-    m->x0 = (bf16*)(B + ox0); m->x0t = (bf16*)(B + ox0t);
+    m->w = (float*)(B + ow);
+    m->mom = (float*)(B + om);
+    m->vel = (float*)(B + ov);
+    m->weights = B + owt;
+    for (int l = 0; l < kLayers; l++) m->gb[l] = (float*)(B + ogb) + l * kH;
+    m->loss = (float*)(B + ogb) + kLayers * kH;
     for (int l = 0; l < COR_MLP_LAYERS; l++) {
-        m->h[l] = (bf16*)(B + oh[l]); m->ht[l] = (bf16*)(B + oht[l]); m->z[l] = (float*)(B + oz[l]);
+        m->z[l] = (float*)(B + oz[l]);
+        m->ht[l] = B + oht[l];
+        m->dzt[l] = B + odz[l];
     }
-    m->dz = (bf16*)(B + odz); m->dzt = (bf16*)(B + odzt); m->dz2 = (bf16*)(B + odz2); m->dz2t = (bf16*)(B + odz2t);
-    m->dy = (bf16*)(B + ody); m->dyt = (bf16*)(B + odyt); m->y = (float*)(B + oy);
-    m->dev_err = (int*)(B + oerr);
-    if (cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) !=
+    m->x0t = B + ox;
+    m->dyt = B + ody;
+    // the parameters, moments and BF16 copies (with their padding) start at zero
+    if (cudaMemset(m->block, 0, ogb + kGbBytes) != cudaSuccess ||
+        cudaHostAlloc((void**)&m->err_h, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void**)&m->err_d, m->err_h, 0) != cudaSuccess ||
+        cudaFuncSetAttribute(rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem) !=
             cudaSuccess ||
+        cudaFuncSetAttribute(rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGradSmem) != cudaSuccess ||
         cudaDeviceSynchronize() != cudaSuccess) {
         cudaFree(m->block);
+        if (m->err_h) cudaFreeHost(m->err_h);
         delete m;
         return COR_ERR_CUDA;
     }
+    *m->err_h = 0;
     *out = m;
     return COR_OK;
 }
@@ -583,6 +762,7 @@ int cor_mlp_destroy(cor_mlp* m) {
     cudaSetDevice(m->device);
     cudaDeviceSynchronize();
     if (m->block) cudaFree(m->block);
+    if (m->err_h) cudaFreeHost(m->err_h);
     delete m;
     return COR_OK;
 }
@@ -590,20 +770,11 @@ int cor_mlp_destroy(cor_mlp* m) {
 int cor_mlp_set_params(cor_mlp* m, const float* params) {
     if (!m || !params) return COR_ERR_INVALID;
     MTRY(m, cudaSetDevice(m->device));
-    size_t wo[kLayers], bo[kLayers];
-    param_offsets(wo, bo);
-    for (int l = 0; l < kLayers; l++) {
-        const size_t nw = (size_t)kOut[l] * kIn[l];
-        MTRY(m, cudaMemcpy(m->w[l], params + wo[l], 4 * nw, cudaMemcpyHostToDevice));
-        MTRY(m, cudaMemcpy(m->b[l], params + bo[l], 4 * (size_t)kOut[l], cudaMemcpyHostToDevice));
-        MTRY(m, cudaMemset(m->mw[l], 0, 4 * nw));
-        MTRY(m, cudaMemset(m->vw[l], 0, 4 * nw));
-        MTRY(m, cudaMemset(m->mb[l], 0, 4 * (size_t)kOut[l]));
-        MTRY(m, cudaMemset(m->vb[l], 0, 4 * (size_t)kOut[l]));
-        ParamView p = view(m, l, false, nullptr);
-        cast_kernel<<<(p.rows * p.cols + 255) / 256, 256>>>(p);
-        MTRY(m, cudaGetLastError());
-    }
+    MTRY(m, cudaMemcpy(m->w, params, sizeof(float) * COR_MLP_PARAMS, cudaMemcpyHostToDevice));
+    MTRY(m, cudaMemset(m->mom, 0, sizeof(float) * COR_MLP_PARAMS));
+    MTRY(m, cudaMemset(m->vel, 0, sizeof(float) * COR_MLP_PARAMS));
+    cast_kernel<<<(COR_MLP_PARAMS + 255) / 256, 256>>>(m->w, m->weights);
+    MTRY(m, cudaGetLastError());
     m->step = 0;
     MTRY(m, cudaDeviceSynchronize());
     return COR_OK;
@@ -613,12 +784,7 @@ int cor_mlp_get_params(cor_mlp* m, float* params) {
     if (!m || !params) return COR_ERR_INVALID;
     MTRY(m, cudaSetDevice(m->device));
     MTRY(m, cudaDeviceSynchronize());
-    size_t wo[kLayers], bo[kLayers];
-    param_offsets(wo, bo);
-    for (int l = 0; l < kLayers; l++) {
-        MTRY(m, cudaMemcpy(params + wo[l], m->w[l], 4 * (size_t)kOut[l] * kIn[l], cudaMemcpyDeviceToHost));
-        MTRY(m, cudaMemcpy(params + bo[l], m->b[l], 4 * (size_t)kOut[l], cudaMemcpyDeviceToHost));
-    }
+    MTRY(m, cudaMemcpy(params, m->w, sizeof(float) * COR_MLP_PARAMS, cudaMemcpyDeviceToHost));
     return COR_OK;
 }
 
@@ -629,10 +795,9 @@ int cor_mlp_forward(cor_mlp* m, const float* x_dev, int32_t n, float* y_dev, voi
     if (n == 0) return COR_OK;
     MTRY(m, cudaSetDevice(m->device));
     cudaStream_t s = (cudaStream_t)stream;
-    const int bt = (n + kBM - 1) / kBM * kBM;
-    int rc = forward(m, x_dev, n, bt, s);
-    if (rc != COR_OK) return rc;
-    copy_out_kernel<<<(n * COR_MLP_OUT + 255) / 256, 256, 0, s>>>(m->y, n, y_dev);
+    RowsArgs g = rows_args(m, x_dev, n);
+    g.y = y_dev;
+    rows_kernel<false><<<(n + kBM - 1) / kBM, kRowsThreads, kRowsSmem, s>>>(g);
     MTRY(m, cudaGetLastError());
     MTRY(m, cudaStreamSynchronize(s));
     return check_err(m);
@@ -645,11 +810,37 @@ static int train(cor_mlp* m, const float* x, const float* t, int32_t n, float lr
         return mfail(m, COR_ERR_INVALID, "batch of %d outside [1, %d] or missing buffer", n, m->max_bt);
     MTRY(m, cudaSetDevice(m->device));
     cudaStream_t s = (cudaStream_t)stream;
-    const int bt = (n + kBM - 1) / kBM * kBM;
-    int rc = forward(m, x, n, bt, s);
-    if (rc == COR_OK) rc = backward(m, t, n, bt, loss, s);
-    if (rc == COR_OK) rc = update(m, lr, wd, grads, do_update, s);
-    if (rc != COR_OK) return rc;
+    const int tiles = (n + kBM - 1) / kBM;
+    MTRY(m, cudaMemsetAsync(m->gb[0], 0, kGbBytes, s));
+    RowsArgs g = rows_args(m, x, n);
+    g.target = t;
+    rows_kernel<true><<<tiles, kRowsThreads, kRowsSmem, s>>>(g);
+    MTRY(m, cudaGetLastError());
+    if (do_update) m->step++;
+    GradArgs a = {};
+    a.x0t = m->x0t;
+    a.dyt = m->dyt;
+    for (int l = 0; l < COR_MLP_LAYERS; l++) {
+        a.ht[l] = m->ht[l];
+        a.dzt[l] = m->dzt[l];
+    }
+    a.blocks = tiles * (kBM / kBK);
+    a.w = m->w;
+    a.m = m->mom;
+    a.v = m->vel;
+    for (int l = 0; l < kLayers; l++) a.gb[l] = m->gb[l];
+    a.loss = m->loss;
+    a.loss_out = loss;
+    a.grads = grads;
+    a.weights = m->weights;
+    a.lr = lr;
+    a.b1c = 1.f - powf(0.9f, (float)(m->step > 0 ? m->step : 1));
+    a.b2c = 1.f - powf(0.999f, (float)(m->step > 0 ? m->step : 1));
+    a.decay = wd;
+    a.update = do_update;
+    a.err = m->err_d;
+    grad_kernel<<<kGradTiles + 1, kGradThreads, kGradSmem, s>>>(a);
+    MTRY(m, cudaGetLastError());
     MTRY(m, cudaStreamSynchronize(s));
     return check_err(m);
 }
