@@ -164,14 +164,16 @@ __device__ __forceinline__ void tmem_ld16(float* v, uint32_t taddr) {
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16(a)) |
+           ((uint32_t)__bfloat16_as_ushort(__float2bfloat16(b)) << 16);
+}
+
 // 16 values of one row, as BF16, to columns c0 .. c0+15 of a K block in shared memory.
 __device__ __forceinline__ void put_row16(uint8_t* block, int row, int c0, const float* v) {
     uint32_t w[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const bf16 lo = __float2bfloat16(v[2 * i]), hi = __float2bfloat16(v[2 * i + 1]);
-        w[i] = (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
-    }
+    for (int i = 0; i < 8; i++) w[i] = pack_bf16(v[2 * i], v[2 * i + 1]);
     uint8_t* d = block + (row >> 3) * 1024 + (c0 >> 3) * 128 + (row & 7) * 16;
     *reinterpret_cast<uint4*>(d) = make_uint4(w[0], w[1], w[2], w[3]);
     *reinterpret_cast<uint4*>(d + 128) = make_uint4(w[4], w[5], w[6], w[7]);
@@ -431,6 +433,7 @@ constexpr int kGradThreads = 32 * 10;                        // 8 epilogue warps
 constexpr int kGradRing = 6;
 constexpr uint32_t kGradStage = block_bytes(kBM) + block_bytes(kGradN);
 constexpr size_t kGradSmem = 1024 + kGradRing * kGradStage;
+static_assert(kBM * (kGradN + 1) * 4 <= 48 * 1024 && 48 * 1024 + kBM * kGradN * 2 <= kGradRing * kGradStage, "the tile");
 
 struct GradArgs {
     const uint8_t* x0t;
@@ -468,14 +471,19 @@ __device__ __forceinline__ void store_weight(uint8_t* stream, int l, int r, int 
     if (l > 0) *reinterpret_cast<bf16*>(stream + product_offset(9 - l) + packed_at(kH, c, r)) = b;
 }
 
-// AdamW on parameter i with gradient gr; returns the new value.
+// AdamW with gradient gr: updates the moments, returns the new parameter.
+__device__ __forceinline__ float adamw_step(const GradArgs& g, float gr, float& m, float& v, float w, float decay) {
+    m = 0.9f * m + 0.1f * gr;
+    v = 0.999f * v + 0.001f * gr * gr;
+    return w - g.lr * ((m / g.b1c) / (sqrtf(v / g.b2c) + 1e-8f) + decay * w);
+}
+
+// The same on parameter i in place.
 __device__ __forceinline__ float adamw(const GradArgs& g, int i, float gr, float decay) {
-    const float m = 0.9f * g.m[i] + 0.1f * gr;
-    const float v = 0.999f * g.v[i] + 0.001f * gr * gr;
+    float m = g.m[i], v = g.v[i];
+    const float w = adamw_step(g, gr, m, v, g.w[i], decay);
     g.m[i] = m;
     g.v[i] = v;
-    float w = g.w[i];
-    w -= g.lr * ((m / g.b1c) / (sqrtf(v / g.b2c) + 1e-8f) + decay * w);
     g.w[i] = w;
     return w;
 }
@@ -586,19 +594,100 @@ __global__ void __launch_bounds__(kGradThreads, 1) grad_kernel(const GradArgs g)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int q = warp & 3, cg = warp >> 2;
             const int row = mt * kBM + 32 * q + lane;
+            // the ring is free: the tile goes through it, so that parameters and
+            // moments are read and written in whole lines
+            float* tile = reinterpret_cast<float*>(ring);
+            constexpr int kLd = kGradN + 1;
+            uint8_t* block = ring + 48 * 1024;
             for (int c0 = 32 * cg; c0 < 32 * cg + 32 && c0 < N; c0 += 16) {
                 float v[16];
                 tmem_ld16(v, tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)c0);
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
                     const int col = n0 + c0 + i;
-                    const int r = l == 4 ? col : row, c = l == 4 ? row : col;
-                    if (r < layer_out(l) && c < layer_in(l)) {
-                        const int at = weight_at(l) + r * layer_in(l) + c;
+                    if (l < 4) {
+                        tile[(32 * q + lane) * kLd + c0 + i] = v[i];
+                    } else if (col < COR_MLP_OUT) {
+                        const int at = weight_at(4) + col * kH + row;
                         if (g.grads) g.grads[at] = v[i];
-                        if (g.update) store_weight(g.weights, l, r, c, adamw(g, at, v[i], g.decay));
+                        if (g.update) store_weight(g.weights, 4, col, row, adamw(g, at, v[i], g.decay));
                     }
                 }
+            }
+            if (l == 0) {
+                // 128 rows of 19, contiguous
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                constexpr int kBatch = 10;
+                static_assert(256 * kBatch >= kBM * COR_MLP_IN, "one batch");
+                float m[kBatch], v[kBatch], w[kBatch];
+                const int at0 = weight_at(0) + mt * kBM * COR_MLP_IN;
+#pragma unroll
+                for (int k = 0; k < kBatch; k++) {
+                    const int e = threadIdx.x + 256 * k;
+                    if (e < kBM * COR_MLP_IN) {
+                        m[k] = g.m[at0 + e];
+                        v[k] = g.v[at0 + e];
+                        w[k] = g.w[at0 + e];
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < kBatch; k++) {
+                    const int e = threadIdx.x + 256 * k, r = e / COR_MLP_IN, c = e % COR_MLP_IN;
+                    if (e < kBM * COR_MLP_IN) {
+                        const float gr = tile[r * kLd + c];
+                        if (g.grads) g.grads[at0 + e] = gr;
+                        if (g.update) {
+                            const float nw = adamw_step(g, gr, m[k], v[k], w[k], g.decay);
+                            g.m[at0 + e] = m[k];
+                            g.v[at0 + e] = v[k];
+                            g.w[at0 + e] = nw;
+                            store_weight(g.weights, 0, mt * kBM + r, c, nw);
+                        }
+                    }
+                }
+            } else if (l < 4) {
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                // four float4 of each array in flight per thread
+                constexpr int kBatch = 4;
+                for (int e0 = threadIdx.x; e0 < kBM * kGradN / 4; e0 += 256 * kBatch) {
+                    float4 m[kBatch], v[kBatch], w[kBatch];
+                    int at[kBatch];
+#pragma unroll
+                    for (int k = 0; k < kBatch; k++) {
+                        const int e = e0 + 256 * k;
+                        at[k] = weight_at(l) + (mt * kBM + e / (kGradN / 4)) * kH + n0 + e % (kGradN / 4) * 4;
+                        m[k] = *reinterpret_cast<const float4*>(g.m + at[k]);
+                        v[k] = *reinterpret_cast<const float4*>(g.v + at[k]);
+                        w[k] = *reinterpret_cast<const float4*>(g.w + at[k]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < kBatch; k++) {
+                        const int e = e0 + 256 * k;
+                        const int tr = e / (kGradN / 4), tc = e % (kGradN / 4) * 4;
+                        const float* gr = tile + tr * kLd + tc;
+                        if (g.grads) {
+#pragma unroll
+                            for (int i = 0; i < 4; i++) g.grads[at[k] + i] = gr[i];
+                        }
+                        if (g.update) {
+                            w[k].x = adamw_step(g, gr[0], m[k].x, v[k].x, w[k].x, g.decay);
+                            w[k].y = adamw_step(g, gr[1], m[k].y, v[k].y, w[k].y, g.decay);
+                            w[k].z = adamw_step(g, gr[2], m[k].z, v[k].z, w[k].z, g.decay);
+                            w[k].w = adamw_step(g, gr[3], m[k].w, v[k].w, w[k].w, g.decay);
+                            *reinterpret_cast<float4*>(g.m + at[k]) = m[k];
+                            *reinterpret_cast<float4*>(g.v + at[k]) = v[k];
+                            *reinterpret_cast<float4*>(g.w + at[k]) = w[k];
+                            const uint2 b = make_uint2(pack_bf16(w[k].x, w[k].y), pack_bf16(w[k].z, w[k].w));
+                            *reinterpret_cast<uint2*>(g.weights + product_offset(l) +
+                                                      packed_at(kH, mt * kBM + tr, n0 + tc)) = b;
+                            *reinterpret_cast<uint2*>(block + packed_at(kBM, tr, tc)) = b;
+                        }
+                    }
+                }
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                if (g.update)
+                    put_transposed(g.weights + product_offset(9 - l), kH, n0 + 32 * cg, mt * kBM, block + 4 * cg * 128,
+                                   q, 32);
             }
         }
     }
