@@ -2,13 +2,14 @@
 // BF16 MLP whose every matrix product runs on the 5th-generation tensor cores.
 //
 // rows_kernel takes 128 rows of the batch through the whole network in one
-// launch: the activations stay in shared memory from layer to layer, and the
-// weights stream through a ring of shared-memory stages (one 64-deep K block,
-// up to 32 KB, per cp.async.bulk).  For a training step it goes on through the
-// loss and back through the layers (dZ of every layer), and leaves what the
-// weight gradients need in global memory.  grad_kernel then takes the weight
-// gradients (one CTA per 128 x 64 tile, K = the batch) and applies AdamW to
-// its tile in the epilogue.
+// launch, by a cluster of four CTAs with a quarter of every hidden layer's
+// columns each: the activations stay in the four shared memories from layer to
+// layer, and the weights stream through a ring of shared-memory stages (a 64-deep
+// K block of a CTA's columns, 8 KB, per cp.async.bulk).  For a training step it
+// goes on through the loss and back through the layers (dZ of every layer), and
+// leaves what the weight gradients need in global memory.  grad_kernel then
+// takes the weight gradients (one CTA per 128 x 64 tile, K = the batch) and
+// applies AdamW to its tile in the epilogue.
 //
 // Products: C[M][N] = A[M][K] . B[N][K]^T with A, B BF16 and K-major, C FP32 in
 // tensor memory, one tcgen05.mma (M = 128, N up to 256, K = 16) per K slice.
@@ -19,18 +20,20 @@
 // stage is one contiguous copy.  Transposed copies (for dW = dZ^T . X) come out
 // of shared memory through ldmatrix.trans, core matrix by core matrix.
 //
-// Warps 0-15 are the epilogue (warp w owns rows 32 (w % 4) .. and columns
-// 64 (w / 4) .. of the accumulator), warp 16 feeds the ring, warp 17 issues the
-// MMAs.  Waits are bounded (about 2 s of SM clock); a wait that runs out sets
+// Warps 0-15 are rows_kernel's epilogue (warp w owns rows 32 (w % 4) .. and
+// columns 16 (w / 4) .. of the accumulator), warp 16 feeds the ring, warp 17
+// issues the MMAs, warp 18 sends the CTA's columns to its peers.  Waits are bounded (about 2 s of SM clock); a wait that runs out sets
 // the error word, and every role leaves its loop, waits for its copies and
 // frees the TMEM.
 //
-// Measured: 2,664 rows forward 404 -> 58 us a call; a training step of 512
-// rows 1,150 -> 210 us.  One GEMM per launch had spent its time in
-// synchronous stages (load, fence, MMA, wait: 5 to 7 us each), in epilogues that
-// wrote rows with a stride, and in 25 launches a step.  What bounds it now is
-// the chain of the layers: the SiLU of 128 x 256 elements, about 3 us of issue
-// slots a layer, and the latency between its parts.
+// Measured: 2,664 rows forward 405 -> 43 us a call (kernel 22 us); a training
+// step of 512 rows 1,150 -> 103 us (rows_kernel 49, grad_kernel 16 us).  One
+// GEMM per launch had spent its time in synchronous stages (load, fence, MMA,
+// wait: 5 to 7 us each), in epilogues that wrote rows with a stride, and in 25
+// launches a step.  One CTA per 128 rows (without the cluster) took 38 and 111
+// us: the SiLU of 128 x 256 elements alone is 3 us of issue slots a layer.  What
+// bounds it now is the chain of the layers, about 4 us each way and layer: MMA,
+// accumulator read, SiLU, exchange.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -200,11 +203,13 @@ __device__ __forceinline__ void put_transposed(uint8_t* dst, int R, int f0, int 
     }
 }
 
-constexpr int kEpiWarps = 16, kRowsThreads = 32 * (kEpiWarps + 2);
-constexpr int kRing = 4;
-constexpr uint32_t kStageBytes = block_bytes(kH);
-constexpr uint32_t kABytes = 4 * block_bytes(kBM);
-constexpr size_t kRowsSmem = 1024 + kABytes + kRing * kStageBytes;
+constexpr int kEpiWarps = 16, kRowsThreads = 32 * (kEpiWarps + 3);
+constexpr int kSplit = 4;                        // CTAs of a cluster: 64 columns of every hidden layer each
+constexpr int kNCols = kH / kSplit;
+constexpr int kRing = 8;
+constexpr uint32_t kStageBytes = block_bytes(kNCols);
+constexpr uint32_t kABlock = block_bytes(kBM);
+constexpr size_t kRowsSmem = 1024 + (2 * kSplit + 1) * kABlock + kRing * kStageBytes;
 
 struct RowsArgs {
     const float* x;          // n x 19
@@ -225,21 +230,48 @@ struct RowsArgs {
 };
 
 struct RowsShared {
-    uint64_t full[kRing], empty[kRing], acc, a_ready;
+    uint64_t full[kRing], empty[kRing], acc;
+    uint64_t local;              // the single K block that this CTA fills itself (input, dY)
+    // K block r of exchange x, in set x % 2: this CTA's own written, or a peer's
+    // copy landed.  Two sets, as two buffers: a peer sends x + 2 only after
+    // this CTA has taken x, but it may send x + 1 before.
+    uint64_t kready[2][kSplit];
     uint32_t tmem;
 };
 static_assert(sizeof(RowsShared) <= 1024, "rows_kernel header");
 
+// Address of this CTA's shared-memory address `a` in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t peer_addr(uint32_t a, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+
+// The output of hidden product p (0 .. 3 forward, 5 .. 7 back) is exchange p or
+// p - 1, into A buffer exchange % 2; the two products before and after the
+// output layer read the single block instead.
+__device__ __forceinline__ int exchange_into(int p) { return p == 0 || p == 5 ? -1 : p < 5 ? p - 1 : p - 2; }
+__device__ __forceinline__ int exchange_out(int p) { return p < 4 ? p : p - 1; }
+
+// A cluster of four CTAs takes one tile of 128 rows: CTA r computes columns
+// 64 r .. 64 r + 63 of every hidden layer, which are K block r of the next
+// product's A, and copies them to its three peers' shared memory.  An epilogue
+// of 128 x 64 elements by 16 warps takes a quarter of what the whole width
+// does, and a weight block is a quarter of the size.  A has two buffers: a
+// peer that writes exchange x has read exchange x - 1 of this CTA, which it
+// sent after its products had read x - 2.
 template <bool TRAIN>
-__global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const RowsArgs g) {
+__global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kRowsThreads, 1) rows_kernel(const RowsArgs g) {
     extern __shared__ __align__(1024) uint8_t smem[];
     RowsShared& sh = *reinterpret_cast<RowsShared*>(smem);
-    uint8_t* sa = smem + 1024;
-    uint8_t* ring = sa + kABytes;
+    uint8_t* abuf = smem + 1024;                          // 2 x 4 K blocks
+    uint8_t* single = abuf + 2 * kSplit * kABlock;        // 1 K block
+    uint8_t* ring = single + kABlock;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.x * kBM;
+    const int rank = blockIdx.x % kSplit, tile = blockIdx.x / kSplit;
+    const int m0 = tile * kBM;
     constexpr int kLast = TRAIN ? kProducts : kFwdProducts;
-    constexpr uint32_t kCols = 256;
+    constexpr uint32_t kCols = kNCols;
 
     if (threadIdx.x == 0) {
         for (int k = 0; k < kRing; k++) {
@@ -247,7 +279,9 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const RowsArgs g)
             mbar_init(&sh.empty[k], 1);
         }
         mbar_init(&sh.acc, 1);
-        mbar_init(&sh.a_ready, 32 * kEpiWarps);
+        mbar_init(&sh.local, 32 * kEpiWarps);
+        for (int i = 0; i < 2; i++)
+            for (int r = 0; r < kSplit; r++) mbar_init(&sh.kready[i][r], r == rank ? 32 * kEpiWarps : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -256,7 +290,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const RowsArgs g)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    // every CTA's barriers are set up before a peer's copy can arrive
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = sh.tmem;
     bool ok = true;
@@ -265,14 +300,15 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const RowsArgs g)
         if (lane == 0) {
             int s = 0;
             for (int p = 0; p < kLast && ok; p++) {
-                const uint32_t bytes = block_bytes(product_n(p));
-                const uint8_t* src = g.weights + product_offset(p);
+                // the output layer's 16 rows go to every CTA; else this CTA's 64 rows
+                const uint32_t bytes = p == 4 ? block_bytes(kOutPad) : kStageBytes;
+                const uint8_t* src = g.weights + product_offset(p) + (p == 4 ? 0 : rank * kStageBytes);
                 for (int kb = 0; kb < product_blocks(p) && ok; kb++, s++) {
                     const int k = s % kRing;
                     if (s >= kRing) ok = mbar_wait(&sh.empty[k], (uint32_t)((s / kRing - 1) & 1));
                     if (!ok) break;
                     mbar_expect(&sh.full[k], bytes);
-                    bulk_load(ring + k * kStageBytes, src + (size_t)kb * bytes, bytes, &sh.full[k]);
+                    bulk_load(ring + k * kStageBytes, src + (size_t)kb * block_bytes(product_n(p)), bytes, &sh.full[k]);
                 }
             }
             if (!ok) {
@@ -286,18 +322,45 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const RowsArgs g)
         if (lane == 0) {
             int s = 0;
             for (int p = 0; p < kLast && ok; p++) {
-                const uint32_t idesc = instr_desc(kBM, product_n(p));
-                ok = mbar_wait(&sh.a_ready, (uint32_t)(p & 1));
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t idesc = instr_desc(kBM, p == 4 ? kOutPad : kNCols);
+                const int x = exchange_into(p);
+                if (x < 0) {
+                    ok = mbar_wait(&sh.local, (uint32_t)(p == 5));
+                } else {
+                    for (int r = 0; r < kSplit; r++)
+                        if (r != rank) mbar_expect(&sh.kready[x & 1][r], kABlock);
+                }
+                const uint8_t* a = x < 0 ? single : abuf + (x & 1) * kSplit * kABlock;
                 for (int kb = 0; kb < product_blocks(p) && ok; kb++, s++) {
                     const int k = s % kRing;
-                    ok = mbar_wait(&sh.full[k], (uint32_t)((s / kRing) & 1));
+                    if (x >= 0) ok = mbar_wait(&sh.kready[x & 1][kb], (uint32_t)((x >> 1) & 1));
+                    ok = ok && mbar_wait(&sh.full[k], (uint32_t)((s / kRing) & 1));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    mma_block(tmem, smem_u32(sa + kb * block_bytes(kBM)), smem_u32(ring + k * kStageBytes), idesc, kb == 0);
+                    mma_block(tmem, smem_u32(a + kb * kABlock), smem_u32(ring + k * kStageBytes), idesc, kb == 0);
                     commit_to(&sh.empty[k]);
                 }
                 if (ok) commit_to(&sh.acc);
+            }
+            if (!ok) atomicExch(g.err, 1);
+        }
+    } else if (warp == kEpiWarps + 2) {
+        if (lane == 0) {
+            // this CTA's K block to its peers
+            for (int p = 0; p + 1 < kLast && ok; p++) {
+                if (p == 4) continue;
+                const int x = exchange_out(p);
+                ok = mbar_wait(&sh.kready[x & 1][rank], (uint32_t)((x >> 1) & 1));
+                if (!ok) break;
+                const uint32_t a = smem_u32(abuf + ((x & 1) * kSplit + rank) * kABlock);
+                for (int i = 1; i < kSplit; i++) {
+                    const int r = (rank + i) % kSplit;
+                    asm volatile(
+                        "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                            peer_addr(a, r)),
+                        "r"(a), "r"(kABlock), "r"(peer_addr(smem_u32(&sh.kready[x & 1][rank]), r))
+                        : "memory");
+                }
             }
             if (!ok) atomicExch(g.err, 1);
         }
@@ -307,52 +370,32 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const RowsArgs g)
         const int gr = m0 + row;
         const bool valid = gr < g.n;
         const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16);
-        // the input: 16 columns per column group
-        {
-            float v[16];
+        const int col0 = kNCols * rank + 16 * cg;   // this warp's 16 columns of a hidden layer
+        float v[16];
+        // the input: 16 columns per column group, in every CTA
 #pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const int c = 16 * cg + i;
-                v[i] = valid && c < COR_MLP_IN ? g.x[(size_t)gr * COR_MLP_IN + c] : 0.f;
-            }
-            put_row16(sa, row, 16 * cg, v);
-            if (TRAIN) {
-                __syncwarp();
-                put_transposed(g.x0t, kInPad, 16 * cg, m0, sa + 2 * cg * 128, q, 16);
-            }
+        for (int i = 0; i < 16; i++) {
+            const int c = 16 * cg + i;
+            v[i] = valid && c < COR_MLP_IN ? g.x[(size_t)gr * COR_MLP_IN + c] : 0.f;
+        }
+        put_row16(single, row, 16 * cg, v);
+        if (TRAIN && rank == 0) {
+            __syncwarp();
+            put_transposed(g.x0t, kInPad, 16 * cg, m0, single + 2 * cg * 128, q, 16);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_arrive(&sh.a_ready);
+        mbar_arrive(&sh.local);
         for (int p = 0; p < kLast; p++) {
             ok = mbar_wait(&sh.acc, (uint32_t)(p & 1));
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint8_t* block = sa + cg * block_bytes(kBM);
-            if (p < COR_MLP_LAYERS) {
-                for (int c0 = 0; c0 < 64; c0 += 16) {
-                    float v[16];
-                    tmem_ld16(v, trow + 64 * cg + c0);
-#pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        const int c = 64 * cg + c0 + i;
-                        const float z = v[i] + g.bias[p][c];
-                        if (TRAIN) g.z[p][((size_t)blockIdx.x * kH + c) * kBM + row] = z;
-                        v[i] = silu(z);
-                    }
-                    put_row16(block, row, c0, v);
-                }
-                if (TRAIN) {
-                    __syncwarp();
-                    put_transposed(g.ht[p], kH, 64 * cg, m0, block, q, 64);
-                }
-            } else if (p == COR_MLP_LAYERS) {
+            if (p == COR_MLP_LAYERS) {
                 if (cg == 0) {
-                    float v[16];
                     tmem_ld16(v, trow);
                     const float y0 = v[0] + g.bias[4][0], y1 = v[1] + g.bias[4][1];
                     if (!TRAIN) {
-                        if (valid) {
+                        if (valid && rank == 0) {
                             g.y[2 * (size_t)gr] = y0;
                             g.y[2 * (size_t)gr + 1] = y1;
                         }
@@ -368,55 +411,78 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const RowsArgs g)
                         float d0 = scale * e0, d1 = scale * e1;
 #pragma unroll
                         for (int i = 0; i < 16; i++) v[i] = i == 0 ? d0 : i == 1 ? d1 : 0.f;
-                        put_row16(sa, row, 0, v);
+                        put_row16(single, row, 0, v);
                         v[0] = v[1] = 0.f;
-                        for (int c0 = 16; c0 < 64; c0 += 16) put_row16(sa, row, c0, v);
-                        __syncwarp();
-                        put_transposed(g.dyt, kOutPad, 0, m0, sa, q, 16);
+                        for (int c0 = 16; c0 < 64; c0 += 16) put_row16(single, row, c0, v);
+                        if (rank == 0) {
+                            __syncwarp();
+                            put_transposed(g.dyt, kOutPad, 0, m0, single, q, 16);
 #pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) {
-                            l += __shfl_xor_sync(0xffffffffu, l, o);
-                            d0 += __shfl_xor_sync(0xffffffffu, d0, o);
-                            d1 += __shfl_xor_sync(0xffffffffu, d1, o);
-                        }
-                        if (lane == 0) {
-                            atomicAdd(g.loss, l);
-                            atomicAdd(g.gb[4], d0);
-                            atomicAdd(g.gb[4] + 1, d1);
+                            for (int o = 16; o > 0; o >>= 1) {
+                                l += __shfl_xor_sync(0xffffffffu, l, o);
+                                d0 += __shfl_xor_sync(0xffffffffu, d0, o);
+                                d1 += __shfl_xor_sync(0xffffffffu, d1, o);
+                            }
+                            if (lane == 0) {
+                                atomicAdd(g.loss, l);
+                                atomicAdd(g.gb[4], d0);
+                                atomicAdd(g.gb[4] + 1, d1);
+                            }
                         }
                     }
+                }
+                if (TRAIN) {
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    mbar_arrive(&sh.local);
+                }
+                continue;
+            }
+            uint8_t* block = abuf + ((exchange_out(p) & 1) * kSplit + rank) * kABlock;
+            tmem_ld16(v, trow + 16 * cg);
+            if (p < COR_MLP_LAYERS) {
+                float z[16];
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    z[i] = v[i] + g.bias[p][col0 + i];
+                    v[i] = silu(z[i]);
+                }
+                put_row16(block, row, 16 * cg, v);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                mbar_arrive(&sh.kready[exchange_out(p) & 1][rank]);
+                if (TRAIN) {
+                    // what the way back needs, beside the next product
+#pragma unroll
+                    for (int i = 0; i < 16; i++) g.z[p][((size_t)tile * kH + col0 + i) * kBM + row] = z[i];
+                    __syncwarp();
+                    put_transposed(g.ht[p], kH, col0, m0, block + 2 * cg * 128, q, 16);
                 }
             } else {
                 const int l = kProducts - 1 - p;   // dZ of layer l + 1
-                for (int c0 = 0; c0 < 64; c0 += 16) {
-                    float v[16];
-                    tmem_ld16(v, trow + 64 * cg + c0);
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        const int c = 64 * cg + c0 + i;
-                        v[i] = v[i] * silu_grad(g.z[l][((size_t)blockIdx.x * kH + c) * kBM + row]);
-                    }
-                    put_row16(block, row, c0, v);
-                    // column sums over the warp's 32 rows: lanes 2c and 2c+1 end with column c's
-#pragma unroll
-                    for (int o = 16, m = 8; m > 0; o >>= 1, m >>= 1) {
-                        const bool up = (lane & o) != 0;
-#pragma unroll
-                        for (int i = 0; i < m; i++) {
-                            const float give = up ? v[i] : v[i + m];
-                            v[i] = (up ? v[i + m] : v[i]) + __shfl_xor_sync(0xffffffffu, give, o);
-                        }
-                    }
-                    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-                    if ((lane & 1) == 0) atomicAdd(g.gb[l] + 64 * cg + c0 + (lane >> 1), v[0]);
+                for (int i = 0; i < 16; i++)
+                    v[i] = v[i] * silu_grad(g.z[l][((size_t)tile * kH + col0 + i) * kBM + row]);
+                put_row16(block, row, 16 * cg, v);
+                if (p + 1 < kLast) {
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    mbar_arrive(&sh.kready[exchange_out(p) & 1][rank]);
                 }
+                // column sums over the warp's 32 rows: lanes 2c and 2c+1 end with column c's
+#pragma unroll
+                for (int o = 16, m = 8; m > 0; o >>= 1, m >>= 1) {
+                    const bool up = (lane & o) != 0;
+#pragma unroll
+                    for (int i = 0; i < m; i++) {
+                        const float give = up ? v[i] : v[i + m];
+                        v[i] = (up ? v[i + m] : v[i]) + __shfl_xor_sync(0xffffffffu, give, o);
+                    }
+                }
+                v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+                if ((lane & 1) == 0) atomicAdd(g.gb[l] + col0 + (lane >> 1), v[0]);
                 __syncwarp();
-                put_transposed(g.dzt[l], kH, 64 * cg, m0, block, q, 64);
-            }
-            if (p + 1 < kLast) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive(&sh.a_ready);
+                put_transposed(g.dzt[l], kH, col0, m0, block + 2 * cg * 128, q, 16);
             }
         }
         if (!ok) atomicExch(g.err, 1);
@@ -424,6 +490,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_kernel(const RowsArgs g)
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
+    // no CTA leaves while a peer's copy may still read or write shared memory
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // ---- weight gradients and AdamW ---------------------------------------------------
@@ -886,7 +954,7 @@ int cor_mlp_forward(cor_mlp* m, const float* x_dev, int32_t n, float* y_dev, voi
     cudaStream_t s = (cudaStream_t)stream;
     RowsArgs g = rows_args(m, x_dev, n);
     g.y = y_dev;
-    rows_kernel<false><<<(n + kBM - 1) / kBM, kRowsThreads, kRowsSmem, s>>>(g);
+    rows_kernel<false><<<kSplit * ((n + kBM - 1) / kBM), kRowsThreads, kRowsSmem, s>>>(g);
     MTRY(m, cudaGetLastError());
     MTRY(m, cudaStreamSynchronize(s));
     return check_err(m);
@@ -903,7 +971,7 @@ static int train(cor_mlp* m, const float* x, const float* t, int32_t n, float lr
     MTRY(m, cudaMemsetAsync(m->gb[0], 0, kGbBytes, s));
     RowsArgs g = rows_args(m, x, n);
     g.target = t;
-    rows_kernel<true><<<tiles, kRowsThreads, kRowsSmem, s>>>(g);
+    rows_kernel<true><<<kSplit * tiles, kRowsThreads, kRowsSmem, s>>>(g);
     MTRY(m, cudaGetLastError());
     if (do_update) m->step++;
     GradArgs a = {};
