@@ -44,6 +44,7 @@ struct cor_ctx {
     cudaStream_t stream = nullptr;
     char err[512] = {0};
     DevBuf jobs, trig, offsets, params, sites, status, records;
+    DevBuf f_params, f_pos, f_out, f_idx; // field batches: parameter blocks, positions, fields, block indices
     int32_t n_params = 0;                 // resident DevParams blocks (cor_upload_params)
     unsigned long long* queue = nullptr;  // work-queue counter (scratch)
     DevBuf park[2];                       // parked trajectories between generations (scratch)
@@ -154,7 +155,8 @@ extern "C" int cor_ctx_destroy(cor_ctx* ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     DevBuf* bufs[] = {&ctx->jobs,   &ctx->trig,    &ctx->offsets, &ctx->params,  &ctx->sites,
-                      &ctx->status, &ctx->records, &ctx->park[0], &ctx->park[1], &ctx->steps};
+                      &ctx->status, &ctx->records, &ctx->park[0], &ctx->park[1], &ctx->steps,
+                      &ctx->f_params, &ctx->f_pos, &ctx->f_out, &ctx->f_idx};
     if (ctx->gen) cudaFree(ctx->gen);
     if (ctx->park_count_host) cudaFreeHost(ctx->park_count_host);
     if (ctx->launches_host) cudaFreeHost(ctx->launches_host);
@@ -712,24 +714,23 @@ extern "C" int cor_field_batch(cor_ctx* ctx, cor_model_set models, const cor_mod
     if (n == 0) return COR_OK;
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
-    void *dp = nullptr, *dpos = nullptr, *dout = nullptr, *didx = nullptr;
+    // the context's own buffers: an allocation and a free a call were 45 us
     int rc = COR_OK;
     do {
-        if (cudaMalloc(&dp, sizeof(DevParams) * (size_t)n_params) != cudaSuccess ||
-            cudaMalloc(&dpos, sizeof(double) * 3 * (size_t)n) != cudaSuccess ||
-            cudaMalloc(&dout, sizeof(double) * 3 * (size_t)n) != cudaSuccess ||
-            (param_index && cudaMalloc(&didx, sizeof(int32_t) * (size_t)n) != cudaSuccess)) {
-            rc = fail(ctx, COR_ERR_NOMEM, "device allocation for the field batch");
-            break;
-        }
+        if ((rc = ensure(ctx, ctx->f_params, sizeof(DevParams) * (size_t)n_params)) != COR_OK) break;
+        if ((rc = ensure(ctx, ctx->f_pos, sizeof(double) * 3 * (size_t)n)) != COR_OK) break;
+        if ((rc = ensure(ctx, ctx->f_out, sizeof(double) * 3 * (size_t)n)) != COR_OK) break;
+        if (param_index && (rc = ensure(ctx, ctx->f_idx, sizeof(int32_t) * (size_t)n)) != COR_OK) break;
+        void *dp = ctx->f_params.p, *dpos = ctx->f_pos.p, *dout = ctx->f_out.p;
+        void* didx = param_index ? ctx->f_idx.p : nullptr;
         DevParams* hp = (DevParams*)malloc(sizeof(DevParams) * (size_t)n_params);
         if (!hp) {
             rc = fail(ctx, COR_ERR_NOMEM, "host allocation");
             break;
         }
         prepare_params(params, n_params, hp);
+        // from pageable memory: the call returns when the source has been read
         cudaMemcpyAsync(dp, hp, sizeof(DevParams) * (size_t)n_params, cudaMemcpyHostToDevice, s);
-        cudaStreamSynchronize(s);
         free(hp);
         cudaMemcpyAsync(dpos, gsm_pos, sizeof(double) * 3 * (size_t)n, cudaMemcpyHostToDevice, s);
         if (param_index) cudaMemcpyAsync(didx, param_index, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, s);
@@ -751,10 +752,6 @@ extern "C" int cor_field_batch(cor_ctx* ctx, cor_model_set models, const cor_mod
         if (e == cudaSuccess) e = cudaGetLastError();
         if (e != cudaSuccess) rc = fail(ctx, COR_ERR_CUDA, "field batch: %s", cudaGetErrorString(e));
     } while (0);
-    if (dp) cudaFree(dp);
-    if (dpos) cudaFree(dpos);
-    if (dout) cudaFree(dout);
-    if (didx) cudaFree(didx);
     return rc;
 }
 

@@ -60,7 +60,9 @@ __device__ __forceinline__ Vec3 calculate_field(const bool want, const Vec3 gsm_
         if (internal) {
             // internal_calc, src/models.c:146-160
             const Vec3 geo = gsm_to_geo(pos, p);
-            const Vec3 bg = internal_geo(geo, p);
+            Vec3 bg;
+            if constexpr (MS::external == COR_EXTERNAL_NONE && MS::crustal == 0) bg = internal_geo_plain(geo, p);
+            else bg = internal_geo(geo, p);
             const Vec3 bs = geo_to_gsm(bg, p);
             tot.x += bs.x;
             tot.y += bs.y;

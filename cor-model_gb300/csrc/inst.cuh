@@ -38,20 +38,20 @@
     }                                                                                                      \
     static cudaError_t field_##NAME(const DevParams* p, int np, const int32_t* idx, const double* pos,     \
                                     int64_t n, double* out, CrustalTables crust, cudaStream_t s) {         \
-        unsigned blocks = (unsigned)((n + 127) / 128);                                                     \
-        int64_t per_warp = 1;                                                                              \
-        if (C != 0) {                                                                                      \
-            int dev = 0, sms = 1, per_sm = 1;                                                              \
-            cudaError_t e = cudaGetDevice(&dev);                                                           \
-            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);   \
-            if (e == cudaSuccess)                                                                          \
-                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, field_kernel<MS_##NAME>, 128, 0); \
-            if (e != cudaSuccess) return e;                                                                \
-            const int64_t resident = (int64_t)sms * (per_sm > 0 ? per_sm : 1);                             \
-            per_warp = (n + 4 * resident - 1) / (4 * resident);                                            \
-            blocks = (unsigned)((n + 4 * per_warp - 1) / (4 * per_warp));                                  \
-        }                                                                                                  \
-        field_kernel<MS_##NAME><<<blocks, 128, 0, s>>>(p, np, idx, pos, n, out, crust, per_warp);          \
+        int dev = 0, sms = 1, per_sm = 1;                                                                  \
+        cudaError_t e = cudaGetDevice(&dev);                                                               \
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);       \
+        if (e == cudaSuccess)                                                                              \
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, field_kernel<MS_##NAME>, kFieldThreads, 0); \
+        if (e != cudaSuccess) return e;                                                                    \
+        const int64_t resident = (int64_t)sms * (per_sm > 0 ? per_sm : 1);                                 \
+        const int64_t per_warp = (n + 4 * resident - 1) / (4 * resident);                                  \
+        const int per_thread =                                                                             \
+            E == 0 && n >= (int64_t)sms * 2 * kFieldThreads * kFieldPerThread ? kFieldPerThread : 1;       \
+        const int64_t per_block = C != 0 ? 4 * per_warp : (int64_t)kFieldThreads * per_thread;             \
+        const unsigned blocks = (unsigned)((n + per_block - 1) / per_block);                               \
+        field_kernel<MS_##NAME><<<blocks, kFieldThreads, 0, s>>>(p, np, idx, pos, n, out, crust, per_warp, \
+                                                                 per_thread);                              \
         return cudaGetLastError();                                                                         \
     }                                                                                                      \
     static cudaError_t tables_##NAME(const T96Tables* t96, const TS05Tables* ts05) {                       \

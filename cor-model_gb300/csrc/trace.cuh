@@ -558,39 +558,87 @@ __global__ void __launch_bounds__(kTraceThreads, 1) trace_kernel(const TraceArgs
     warp_add_u64(reinterpret_cast<unsigned long long*>(&a.counters->watchdog), n_wd);
 }
 
-// calculate_field at n points.  With the crustal model, whose sum takes a whole
-// warp per point, the resident warps take per_warp points each, so
-// that no wave of blocks is left nearly empty (40,001 points in blocks of 128
-// threads, 128 points each, were two waves, the second of 9 blocks); without
-// it, a thread takes one point.
+// calculate_field at n points.  A block takes kFieldThreads x per_thread points
+// and, but for TS05, evaluates them in the order of their field_band, so that
+// a warp's points run the same branches and the same degree of the internal
+// field (a warp's time is its longest lane's).  Log-uniform over 1 to 12 R_E,
+// us a call unsorted / sorted over 128 / over 512 points: IGRF-14, 500,003
+// points 3,182 / 2,603 / 2,475; T96, 20,000 points 1,101 / 955 / 1,813 and
+// 200,000 5,934 / 5,582 / 7,049 (its warps of unlike cost leave the block's
+// slowest alone); TS05, 200,000 10,923 / 11,112 / 15,128 (its branches are
+// small).  So four points a thread with the internal field alone, where they
+// fill the SMs; else one.
+//
+// With the crustal model, whose sum takes a whole warp per point, the
+// resident warps take per_warp points each, so that no wave of blocks is left
+// nearly empty (40,001 points in blocks of 128 threads, 128 points each, were
+// two waves, the second of 9 blocks).
+constexpr int kFieldThreads = 128, kFieldPerThread = 4;
+
 template <class MS>
-__global__ void field_kernel(const DevParams* __restrict__ params, int n_params,
-                             const int32_t* __restrict__ pidx, const double* __restrict__ pos, int64_t n,
-                             double* __restrict__ out, CrustalTables crust, int64_t per_warp) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (MS::crustal == 0 && t >= n) return;
-    int64_t lo = t, hi = n;
-    if (MS::crustal != 0) {
-        lo = (t >> 5) * per_warp;
-        hi = lo + per_warp < n ? lo + per_warp : n;
-    }
-    for (int64_t i0 = lo; i0 < hi; i0 += 32) {
-        const int64_t i = MS::crustal != 0 ? i0 + (threadIdx.x & 31) : i0;
-        const bool want = i < hi;
-        int k = 0;
-        Vec3 x = {0., 0., 0.};
-        if (want) {
-            k = pidx ? pidx[i] : 0;
-            if (k < 0 || k >= n_params) k = 0;
-            x = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
+__device__ __forceinline__ void field_point(const DevParams* params, int n_params, const int32_t* pidx,
+                                            const double* pos, int64_t i, const DevParams*& par, Vec3& x) {
+    int k = pidx ? pidx[i] : 0;
+    if (k < 0 || k >= n_params) k = 0;
+    par = params + k;
+    x = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
+}
+
+template <class MS>
+__global__ void __launch_bounds__(kFieldThreads)
+    field_kernel(const DevParams* __restrict__ params, int n_params, const int32_t* __restrict__ pidx,
+                 const double* __restrict__ pos, int64_t n, double* __restrict__ out, CrustalTables crust,
+                 int64_t per_warp, int per_thread) {
+    const int tid = (int)threadIdx.x;
+    if constexpr (MS::crustal != 0) {
+        const int64_t t = (int64_t)blockIdx.x * kFieldThreads + tid;
+        const int64_t lo = (t >> 5) * per_warp, hi = lo + per_warp < n ? lo + per_warp : n;
+        for (int64_t i0 = lo; i0 < hi; i0 += 32) {
+            const int64_t i = i0 + (tid & 31);
+            const bool want = i < hi;
+            const DevParams* par = params;
+            Vec3 x = {0., 0., 0.};
+            if (want) field_point<MS>(params, n_params, pidx, pos, i, par, x);
+            const Vec3 b = calculate_field<MS>(want, x, par, crust);
+            if (want) {
+                out[3 * i] = b.x;
+                out[3 * i + 1] = b.y;
+                out[3 * i + 2] = b.z;
+            }
         }
-        const Vec3 b = calculate_field<MS>(want, x, params + k, crust);
-        if (want) {
+    } else {
+        __shared__ unsigned key[kFieldThreads * kFieldPerThread];
+        __shared__ unsigned short at[kFieldThreads * kFieldPerThread];
+        const int m = kFieldThreads * per_thread;
+        const int64_t base = (int64_t)blockIdx.x * m;
+        const int here = n - base < m ? (int)(n - base) : m;
+        constexpr bool kSort = MS::external != COR_EXTERNAL_TS05;
+        if constexpr (kSort) {
+            for (int j = tid; j < here; j += kFieldThreads) {
+                const DevParams* par;
+                Vec3 x;
+                field_point<MS>(params, n_params, pidx, pos, base + j, par, x);
+                key[j] = field_band<MS>(x, par);
+            }
+            __syncthreads();
+            for (int j = tid; j < here; j += kFieldThreads) {
+                const unsigned kj = key[j];
+                int rank = 0;
+                for (int i = 0; i < here; i++) rank += (key[i] < kj || (key[i] == kj && i < j)) ? 1 : 0;
+                at[rank] = (unsigned short)j;
+            }
+            __syncthreads();
+        }
+        for (int j = tid; j < here; j += kFieldThreads) {
+            const int64_t i = base + (kSort ? at[j] : j);
+            const DevParams* par;
+            Vec3 x;
+            field_point<MS>(params, n_params, pidx, pos, i, par, x);
+            const Vec3 b = calculate_field<MS>(true, x, par, crust);
             out[3 * i] = b.x;
             out[3 * i + 1] = b.y;
             out[3 * i + 2] = b.z;
         }
-        if (MS::crustal == 0) return;
     }
 }
 
