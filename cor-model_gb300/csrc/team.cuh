@@ -192,8 +192,12 @@ __device__ __forceinline__ int quad_advance(Lane& L, const TraceArgs& a, bool ru
 }
 
 // ---- the internal field in tasks ---------------------------------------------
-constexpr int kShTerms = 105;   // (m, n), 1 <= m <= n <= 14, at n(n-1)/2 + m - 1
+constexpr int kShTerms = 105;   // (m, n), 1 <= m <= n <= 14, at n(n-1)/2 + m - 1 in the tables
 constexpr int kShCols = 14;
+
+// Where a slot keeps term (m, m) if it goes up to n = K: column by column, as
+// the sums take the terms, without gaps.
+__device__ __forceinline__ int sh_at(const int m, const int K) { return (m - 1) * (K + 1) - m * (m - 1) / 2; }
 
 // What internal_geo keeps in registers, for one slot.
 struct ShSlot {
@@ -302,12 +306,14 @@ __device__ __forceinline__ void sh_column(ShSlot& s, const int m) {
     const int K = s.K;
     const double* __restrict__ REC = s.p->rec;
     double q = s.pmm[m - 1], zz = s.dmm[m - 1], p2 = 0., d2 = 0.;
-    int i = m * (m - 1) / 2 + m - 1;
+    int i = m * (m - 1) / 2 + m - 1, j = sh_at(m, K);
+    double next = __ldg(&REC[i]);
     for (int n = m; n <= K; n++) {
-        s.q[i] = q;
-        s.z_[i] = zz;
+        s.q[j] = q;
+        s.z_[j++] = zz;
         if (n < K) {
-            const double xk = __ldg(&REC[i]);
+            const double xk = next;
+            if (n + 1 < K) next = __ldg(&REC[i + n]);
             const double dp = sh_mad<FMA>(-xk, d2, sh_mad<FMA>(C, zz, -__dmul_rn(S, q)));
             const double pm = sh_mad<FMA>(C, q, -__dmul_rn(xk, p2));
             d2 = zz;
@@ -322,15 +328,15 @@ __device__ __forceinline__ void sh_column(ShSlot& s, const int m) {
 // The factors of term i that multiply P and dP in the three sums.
 template <bool FMA>
 __device__ __forceinline__ void sh_term(ShSlot& s, const int i) {
-    const int n = c_sh_n[i], m = i - n * (n - 1) / 2 + 1;
+    const int n = c_sh_n[i], m = i - n * (n - 1) / 2 + 1, j = sh_at(m, s.K) + n - m;
     const double an = s.pw[n - 1];
     const double sm = s.sm[m - 1], cm = s.cm[m - 1];
     const double e = __ldg(&s.p->g[i]);
     const double hh = __ldg(&s.p->h[i]);
     const double w = sh_mad<FMA>(e, sm, __dmul_rn(hh, cm));
-    s.a1[i] = s.pwn[n - 1] * w;
-    s.a2[i] = -(an * w);
-    s.a3[i] = an * sh_mad<FMA>(e, cm, -__dmul_rn(hh, sm));
+    s.a1[j] = s.pwn[n - 1] * w;
+    s.a2[j] = -(an * w);
+    s.a3[j] = an * sh_mad<FMA>(e, cm, -__dmul_rn(hh, sm));
 }
 
 // Without contraction the sums add rounded products, which are then taken
@@ -342,22 +348,33 @@ __device__ __forceinline__ void sh_product(ShSlot& s, const int i) {
     s.a3[i] = s.a3[i] * (s.pole ? z : q);
 }
 
+constexpr int kShBatch = 7;
+
 // One of the sums of internal_geo in its order: br (0), bt (1), or the share
-// of order m - 1 in bf (m = 2 .. K).
+// of order m - 1 in bf (m = 2 .. K).  The two long ones bound their phase:
+// 10,700 cycles for 105 terms when each addition waited for its own loads,
+// with the terms in the sums' order and loads ahead of them a lone IGRF
+// trajectory's step went from 42.8 us to 41.5.
 template <bool FMA>
 __device__ __forceinline__ void sh_sum(ShSlot& s, const int which) {
     const int K = s.K;
     const double* A = which == 0 ? s.a1 : which == 1 ? s.a2 : s.a3;
     const double* B = which == 1 || (which >= 2 && s.pole) ? s.z_ : s.q;
-    const int m0 = which < 2 ? 1 : which, m1 = which < 2 ? K : which;
+    const int end = which < 2 ? K * (K + 1) / 2 : which <= K ? sh_at(which + 1, K) : 0;
+    int j = which < 2 ? 0 : which <= K ? sh_at(which, K) : 0;
     double acc = 0.;
-    for (int m = m0; m <= m1; m++) {
-        int i = m * (m - 1) / 2 + m - 1;
-        for (int n = m; n <= K; n++) {
-            acc = FMA ? __fma_rn(A[i], B[i], acc) : __dadd_rn(acc, A[i]);
-            i += n;
+    // loads in batches: one at a time, each waits for the addition before it
+    for (; j + kShBatch <= end; j += kShBatch) {
+        double a[kShBatch], b[kShBatch];
+#pragma unroll
+        for (int k = 0; k < kShBatch; k++) {
+            a[k] = A[j + k];
+            if (FMA) b[k] = B[j + k];
         }
+#pragma unroll
+        for (int k = 0; k < kShBatch; k++) acc = FMA ? __fma_rn(a[k], b[k], acc) : __dadd_rn(acc, a[k]);
     }
+    for (; j < end; j++) acc = FMA ? __fma_rn(A[j], B[j], acc) : __dadd_rn(acc, A[j]);
     if (which >= 2) acc = __dmul_rn(acc, which - 1);   // rounded before it is added, in both kinds of unit
     s.sum[which] = acc;
 }
@@ -454,7 +471,7 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
         if constexpr (kT96) {
             any = true;
             if (takes(ch, 1)) {
-                if (lane < n) t96_task_b1(slots[list[lane]].t96);
+                t96_task_b1(slots[list[lane < 2 * n ? lane >> 1 : 0]].t96, lane < 2 * n);
             } else if (takes(ch, chunks(6 * n))) {
                 const int t = (int)ch * 32 + lane;
                 if (t < 6 * n) t96_task_rt(slots[list[t % n]].t96, t / n);
@@ -569,10 +586,12 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
                     else if (ch == 1) t96_task_sheet<1>(s);
                     else t96_task_sheet<2>(s);
                 }
-            } else if (takes(ch, nc ? 1 : 0)) {
-                if (lane < nc) t96_task_con(slots[lc[lane]].t96);
-            } else if (takes(ch, ni ? 1 : 0)) {
-                if (lane < ni) t96_task_inner(slots[li[lane]].t96);
+            } else if (takes(ch, chunks(5 * nc))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 5 * nc) t96_task_con(slots[lc[t % nc]].t96, t / nc);
+            } else if (takes(ch, chunks(7 * ni))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 7 * ni) t96_task_inner(slots[li[t % ni]].t96, t / ni);
             } else if (takes(ch, chunks(ncir))) {
                 const int t = (int)ch * 32 + lane;
                 if (t < 3 * nl) t96_task_circle(slots[ll[t % nl]].t96, t / nl, false);

@@ -9,7 +9,8 @@
 //            sines and cosines of the shields (36);
 //   phase 2: exponential terms of the shields (56), dipoles of the conical
 //            basis (46) and of the loops basis (21), current circles (up to
-//            14), the conical harmonics, the Region-2 sheet by component;
+//            14), the conical harmonics by order (5 each), the Region-2 sheet
+//            by component;
 //   phase 3: every sum in its order, one lane per sum and component.
 // The expressions, and what is rounded before it is added, are t96.cuh's: a
 // term whose last product the one-lane code adds with one rounding is kept as
@@ -167,7 +168,7 @@ struct T96Slot {
     double dip[kT96Dip][6];
     double lop[kT96Lop][4];
     double cir[18][3];            // 0-2 loops basis, 3-13 r2outer, 3-6 r2inner
-    double con[3], inner[3], sheet[3];
+    double con[5][3], inn[7][3], sheet[3];   // harmonics by order; inn: 5, 6 the distributed dipoles
     double shield[6][3];
     double tl[3], tc[3], cyl[3], ring[3], tail[3], tail87[2], ri[3], ro[3];
     const T96Cond* c;
@@ -213,21 +214,27 @@ static __device__ __noinline__ void t96_task_main(T96Slot& s) {
     s.sigma = sqrt(div_r(aro + axx0 + sqrt(aa * aa - c.four_asq * axx0), c.two_asq, c.r_two_asq));
 }
 
-// t96_birk1tot up to the points where its bases are taken.
-static __device__ __noinline__ void t96_task_b1(T96Slot& s) {
+// t96_birk1tot up to the points where its bases are taken, by two neighbouring
+// lanes that take one of the two arc tangents and of their sines each (the
+// whole warp calls; live: the lane's slot is evaluated).
+static __device__ __noinline__ void t96_task_b1(T96Slot& s, const bool live) {
     const double x = s.x, y = s.y, z = s.z;
+    const bool odd = threadIdx.x & 1;
+    const double an = ol_atan2(odd ? sqrt(x * x + y * y) : y, odd ? z : x);
+    const double ap = !odd && x == 0.0 && y == 0.0 ? 0.0 : an;
+    const double sn = ol_sin(odd ? ap : ap * 0.5);
+    const double pas = __shfl_sync(0xffffffffu, ap, threadIdx.x & 30);
+    const double tas = __shfl_sync(0xffffffffu, ap, threadIdx.x | 1);
+    const double sh = __shfl_sync(0xffffffffu, sn, threadIdx.x & 30);
+    const double stas = __shfl_sync(0xffffffffu, sn, threadIdx.x | 1);
+    if (!live || odd) return;
     const double tnoonn = 12.0 * 0.01745329;
     const double tnoons = 3.141592654 - tnoonn;
     const double r2 = x * x + y * y + z * z;
     const double r = sqrt(r2);
     const double r3 = r * r2;
-    double pas = 0.0;
-    if (x != 0.0 || y != 0.0) pas = ol_atan2(y, x);
-    const double tas = ol_atan2(sqrt(x * x + y * y), z);
-    const double stas = ol_sin(tas);
     double tet0 = ol_asin(stas / ol_pow((stas * stas * stas * stas * stas * stas) * (1.0 - r3) + r3, 0.1666666667));
     if (tas > 1.5707963) tet0 = 3.141592654 - tet0;
-    const double sh = ol_sin(pas * 0.5);
     const double dtet = (8.0 * 0.01745329) * (sh * sh);
     const double tr1n = tnoonn + dtet, tr1s = tnoons - dtet;
     const double t01n = tr1n - 0.034906, t01s = tr1s - 0.034906;
@@ -512,23 +519,50 @@ static __device__ __noinline__ void t96_task_circle(T96Slot& s, const int k, con
     s.cir[k][2] = b.z;
 }
 
-// The conical harmonics of condip1 (t96_r1_condip's first sum).
-static __device__ __noinline__ void t96_task_con(T96Slot& sl) {
-    constexpr double C2[5] = {6.04133, 0.305415, 0.606066E-02, 0.128379E-03, -0.179406E-04};
+// (tan t/2)^m + (cot t/2)^m of a conical harmonic and the powers below, m =
+// k + 1: the last order's powers are only added there, in one rounding.
+__device__ __forceinline__ double t96_cone_powers(const double tnh, const double cnh, const int k, double& tp,
+                                                  double& cp) {
+    tp = cp = 1.0;
+    double t1 = tnh, c1 = cnh;
+#pragma unroll
+    for (int i = 1; i < 5; i++) {
+        if (i <= k) {
+            tp = t1;
+            cp = c1;
+            t1 = __dmul_rn(tp, tnh);
+            c1 = __dmul_rn(cp, cnh);
+        }
+    }
+    return k == 4 ? __fma_rn(tp, tnh, c1) : __dadd_rn(t1, c1);
+}
+
+// Conical harmonic k + 1 of condip1 (t96_r1_condip's first sum).  The angles
+// are every order's; three quotients and the powers are its own.  All five by
+// one lane took 22,500 cycles (r2inner's, with the dipoles, 30,400) and were
+// their phase's longest tasks; by order a lone T96 trajectory's step went
+// from 62.4 us to 56.8 (with the arc tangents of t96_task_b1 by two lanes,
+// 23,200 cycles by one), 8,000 trajectories of 250 steps from 114 ms to 110.
+static __device__ __noinline__ void t96_task_con(T96Slot& sl, const int k) {
     const double x = sl.pc[0], y = sl.pc[1], z = sl.pc[2];
     const double xsm = x + 0.16;
     const double ro2 = xsm * xsm + y * y;
     const double ro = sqrt(ro2);
     const double rro = 1.0 / ro;
-    double cf[5], sf[5];
-    cf[0] = div_r(xsm, ro, rro);
-    sf[0] = div_r(y, ro, rro);
-    cf[1] = cf[0] * cf[0] - sf[0] * sf[0];
-    sf[1] = 2.0 * sf[0] * cf[0];
+    const double cf0 = div_r(xsm, ro, rro), sf0 = div_r(y, ro, rro);
+    double cf = cf0, sf = sf0;
+    if (k > 0) {
+        cf = cf0 * cf0 - sf0 * sf0;
+        sf = 2.0 * sf0 * cf0;
+    }
 #pragma unroll
     for (int m = 2; m < 5; m++) {
-        cf[m] = cf[m - 1] * cf[0] - sf[m - 1] * sf[0];
-        sf[m] = sf[m - 1] * cf[0] + cf[m - 1] * sf[0];
+        const double c1 = __fma_rn(cf, cf0, -__dmul_rn(sf, sf0));
+        const double s1 = __fma_rn(sf, cf0, __dmul_rn(cf, sf0));
+        if (m <= k) {
+            cf = c1;
+            sf = s1;
+        }
     }
     const double r2 = ro2 + z * z;
     const double r = sqrt(r2);
@@ -538,91 +572,70 @@ static __device__ __noinline__ void t96_task_con(T96Slot& sl) {
     const double tnh = sh / ch, cnh = 1.0 / tnh;
     const double ch2 = ch * ch, sh2 = sh * sh;
     const double rs = r * s;
-    double bx = 0.0, by = 0.0, bz = 0.0;
-    double tp = 1.0, cp = 1.0;  // tnh^m, cnh^m
-#pragma unroll
-    for (int m = 0; m < 5; m++) {
-        const double mn = m + 1;
-        const double tp1 = (m == 0) ? tnh : tp * tnh, cp1 = (m == 0) ? cnh : cp * cnh;
-        const double bt = mn * cf[m] / rs * (tp1 + cp1);
-        const double bf = div_r(-0.5 * mn * sf[m], r, rr) * (tp / ch2 - cp / sh2);
-        bx += C2[m] * (bt * c * cf[0] - bf * sf[0]);
-        by += C2[m] * (bt * c * sf[0] + bf * cf[0]);
-        bz += C2[m] * (-bt * s);
-        tp = tp1;
-        cp = cp1;
-    }
-    sl.con[0] = bx;
-    sl.con[1] = by;
-    sl.con[2] = bz;
+    const double mn = k + 1;
+    double tp, cp;
+    const double sum = t96_cone_powers(tnh, cnh, k, tp, cp);
+    const double bt = mn * cf / rs * sum;
+    const double bf = div_r(-0.5 * mn * sf, r, rr) * (tp / ch2 - cp / sh2);
+    sl.con[k][0] = __fma_rn(bt * c, cf0, -__dmul_rn(bf, sf0));
+    sl.con[k][1] = __fma_rn(bt * c, sf0, __dmul_rn(bf, cf0));
+    sl.con[k][2] = -bt * s;
 }
 
-// r2inner without its loops: the conical harmonics and the two distributed
-// dipoles, added as t96_r2inner adds them.
-static __device__ __noinline__ void t96_task_inner(T96Slot& sl) {
-    constexpr double CB[5] = {154.185, -2.12446, 0.601735E-01, -.153954E-02, .355077E-04};
+// Conical harmonic k + 1 of r2inner (k < 5), or its distributed dipoles (5, 6).
+static __device__ __noinline__ void t96_task_inner(T96Slot& sl, const int k) {
     const double x = sl.x, y = sl.y, z = sl.z;
-    const double ro2 = x * x + y * y;
+    double* o = sl.inn[k];
+    // a square that t96_r2inner uses in several sums, and so does not fuse
+    const double yy = __dmul_rn(y, y);
+    if (k >= 5) {
+        const double xx = k == 5 ? x - .0774 : x + .038;
+        const double x2 = __dmul_rn(xx, xx);
+        const double rho2 = __dadd_rn(x2, yy);
+        const double rho4 = rho2 * rho2;
+        if (k == 5) {
+            const double q2 = __fma_rn(z, z, rho2);
+            const double r3 = q2 * sqrt(q2);
+            o[0] = z / rho4 * __fma_rn(q2, __dadd_rn(yy, -x2), -__dmul_rn(rho2, x2)) / r3;
+            o[1] = -xx * y * z / rho4 * (2.0 * q2 + rho2) / r3;
+            o[2] = xx / r3;
+        } else {
+            o[0] = z / rho4 * __dadd_rn(yy, -x2);
+            o[1] = -2.0 * xx * y * z / rho4;
+            o[2] = xx / rho2;
+        }
+        return;
+    }
+    const double ro2 = __fma_rn(x, x, yy);
     const double ro = sqrt(ro2);
     const double rro = 1.0 / ro;
     const double cf = div_r(x, ro, rro), sf = div_r(y, ro, rro);
-    const double r2 = ro2 + z * z;
+    const double r2 = __fma_rn(z, z, ro2);
     const double r = sqrt(r2);
     const double rr = 1.0 / r;
     const double c = div_r(z, r, rr), s = div_r(ro, r, rr);
     const double ch = sqrt(0.5 * (1.0 + c)), sh = sqrt(0.5 * (1.0 - c));
-    double tnhm1 = 1.0, cnhm1 = 1.0;
     const double tnh = sh / ch, cnh = 1.0 / tnh;
     const double ch2 = ch * ch, sh2 = sh * sh;
     const double rs = r * s;
-    double cfm1 = 1.0, sfm1 = 0.0;
-    double bx = 0.0, by = 0.0, bz = 0.0;
+    double cfm = cf, sfm = sf;
 #pragma unroll
-    for (int m = 0; m < 5; m++) {
-        const double cfm = cfm1 * cf - sfm1 * sf;
-        const double sfm = cfm1 * sf + sfm1 * cf;
-        cfm1 = cfm;
-        sfm1 = sfm;
-        const double tnhm = tnhm1 * tnh, cnhm = cnhm1 * cnh;
-        const double bt = (m + 1) * cfm / rs * (tnhm + cnhm);
-        const double bf = div_r(-0.5 * (m + 1) * sfm, r, rr) * (tnhm1 / ch2 - cnhm1 / sh2);
-        tnhm1 = tnhm;
-        cnhm1 = cnhm;
-        const double cbx = bt * c * cf - bf * sf, cby = bt * c * sf + bf * cf, cbz = -bt * s;
-        if (m == 0) {
-            bx = CB[0] * cbx;
-            by = CB[0] * cby;
-            bz = CB[0] * cbz;
-        } else {
-            bx = bx + CB[m] * cbx;
-            by = by + CB[m] * cby;
-            bz = bz + CB[m] * cbz;
+    for (int m = 1; m < 5; m++) {
+        const double c1 = __fma_rn(cfm, cf, -__dmul_rn(sfm, sf));
+        const double s1 = __fma_rn(cfm, sf, __dmul_rn(sfm, cf));
+        if (m <= k) {
+            cfm = c1;
+            sfm = s1;
         }
     }
-    Vec3 d6, d7;
-    {
-        const double xx = x - .0774;
-        const double x2 = xx * xx;
-        const double rho2 = x2 + y * y;
-        const double q2 = rho2 + z * z;
-        const double r3 = q2 * sqrt(q2);
-        const double rho4 = rho2 * rho2;
-        d6.x = z / rho4 * (q2 * (y * y - x2) - rho2 * x2) / r3;
-        d6.y = -xx * y * z / rho4 * (2.0 * q2 + rho2) / r3;
-        d6.z = xx / r3;
-    }
-    {
-        const double xx = x + .038;
-        const double x2 = xx * xx;
-        const double rho2 = x2 + y * y;
-        const double rho4 = rho2 * rho2;
-        d7.x = z / rho4 * (y * y - x2);
-        d7.y = -2.0 * xx * y * z / rho4;
-        d7.z = xx / rho2;
-    }
-    sl.inner[0] = bx + 29.9996 * d6.x + 262.886 * d7.x;
-    sl.inner[1] = by + 29.9996 * d6.y + 262.886 * d7.y;
-    sl.inner[2] = bz + 29.9996 * d6.z + 262.886 * d7.z;
+    double tp, cp;
+    const double sum = t96_cone_powers(tnh, cnh, k, tp, cp);
+    const double mn = k + 1;
+    const double bt = mn * cfm / rs * sum;
+    const double bf = div_r(-0.5 * mn * sfm, r, rr) * (tp / ch2 - cp / sh2);
+    o[0] = __fma_rn(bt * c, cf, -__dmul_rn(bf, sf));
+    o[1] = __fma_rn(bt * c, sf, __dmul_rn(bf, cf));
+    o[2] = -bt * s;
 }
 
 // Component C of t96_r2sheet.
@@ -732,7 +745,10 @@ static __device__ const double g_con_c2[37] = {
     -0.661373E-02, 0.249201E-02, 0.343978E-01};
 
 __device__ __forceinline__ void t96_sum_con(T96Slot& s, const int c) {
-    double b = s.con[c];
+    constexpr double C2[5] = {6.04133, 0.305415, 0.606066E-02, 0.128379E-03, -0.179406E-04};
+    double b = 0.0;
+#pragma unroll
+    for (int m = 0; m < 5; m++) b += C2[m] * s.con[m][c];
     const int ax = g_dip_at[0][c], ay = g_dip_at[1][c], az = g_dip_at[2][c];
     for (int i = 0; i < 9; i++) {
         const double(*d)[6] = &s.dip[4 * i];
@@ -843,9 +859,15 @@ static __device__ __noinline__ void t96_sum_outer(T96Slot& s) {
 
 static __device__ __noinline__ void t96_sum_inner(T96Slot& s) {
     const Vec3 d8 = t96_loops_of(&s.cir[3], 0);
-    s.ri[0] = s.inner[0] + 99.9132 * d8.x;
-    s.ri[1] = s.inner[1] + 99.9132 * d8.y;
-    s.ri[2] = s.inner[2] + 99.9132 * d8.z;
+    constexpr double CB[5] = {154.185, -2.12446, 0.601735E-01, -.153954E-02, .355077E-04};
+    const double(*h)[3] = s.inn;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        double b = __fma_rn(CB[0], h[0][c], __dmul_rn(CB[1], h[1][c]));
+#pragma unroll
+        for (int m = 2; m < 5; m++) b = b + CB[m] * h[m][c];
+        s.ri[c] = b + 29.9996 * h[5][c] + 262.886 * h[6][c] + 99.9132 * comp(d8, c);
+    }
 }
 
 // r2_birk's mix of the sub-fields of its band.
