@@ -303,40 +303,41 @@ static const ModelOps* find_ops(const cor_model_set& m) {
 // Whether `live` trajectories run by teams (team.cuh) instead of one to a
 // lane: up to half of the lanes of cap_blocks scan blocks.  Below that the
 // lanes' own code leaves sub-partitions idle or lanes of a warp waiting for
-// the longest; above it their throughput is the higher one.  IGRF-14, ms by
-// lanes / by teams: 400 trajectories 331 / 109, 8,000 243 / 86, 20,000
-// 286 / 178, 40,000 375 / 325 (291 when the teams take over at half the
-// lanes), 91,200 562 / 666 (487).  With T96, limit 1,000 steps: 400
-// trajectories 432 / 63, 2,000 484 / 92; limit 250: 8,000 103 / 110, 20,000
-// 291 / 187, 66,000 (the tail by teams) 629 / 497.  With TS05: 3,573
-// trajectories, limit 400, 607 / 172; limit 100: 8,000 143 / 84, 20,000
-// 235 / 153.
+// the longest; above it their throughput is the higher one.  IGRF-14, limit
+// 1,000 steps, ms by lanes / by teams: 8,000 trajectories 199 / 81, 12,000
+// 209 / 114, 20,000 246 / 181 (173 when the teams take over at half the
+// lanes).  With T96, limit 250: 4,000 272 / 88, 12,000 173 / 132, 16,000
+// 192 / 168, 20,000 - / 215 (183).  With TS05, limit 100: 12,000 113 / 84,
+// 16,000 122 / 113.
 static bool team_takes(const ModelOps* ops, uint64_t live, uint64_t cap_blocks) {
     return ops->launch_team && 2 * live <= cap_blocks * (uint64_t)kTraceThreads;
 }
 
 // The same for a field batch of n points, where every lane does the same
-// amount of work: up to a sixth of the lanes, with TS05 (whose tasks fill a
-// team best) up to half.  T96, us by lanes / by teams (the call's allocations
-// and copies included): 1 point 403 / 114, 1,000 614 / 184, 5,000 625 / 433,
-// 8,000 639 / 736; IGRF-14: 1 116 / 83, 2,664 177 / 127, 8,000 177 / 184;
-// TS05: 1 979 / 188, 2,664 1,085 / 364, 12,000 1,110 / 985, 20,000
-// 1,989 / 1,603.
+// amount of work: up to a sixth of the lanes, with T96 up to a quarter, with
+// TS05 (whose tasks fill a team best) up to three quarters.  us by lanes / by
+// teams (the call's copies included): IGRF-14, 5,000 points 146 / 131, 8,000
+// 151 / 138, 12,000 147 / 178; T96, 1,000 560 / 165, 5,000 598 / 285, 8,000
+// 581 / 411, 12,000 598 / 615; TS05, 12,000 1,077 / 850, 16,000
+// 1,090 / 1,110, 20,000 1,955 / 1,372, 30,000 2,357 / 2,132.
 static bool team_takes_field(const ModelOps* ops, cor_model_set models, uint64_t n, int sms) {
-    const uint64_t share = models.external_model == COR_EXTERNAL_TS05 ? 2 : 6;
-    return ops->launch_team_field && share * n <= (uint64_t)sms * (uint64_t)kTraceThreads;
+    const uint64_t lanes = (uint64_t)sms * (uint64_t)kTraceThreads;
+    const uint64_t most = models.external_model == COR_EXTERNAL_TS05  ? lanes / 4 * 3
+                          : models.external_model == COR_EXTERNAL_T96 ? lanes / 4
+                                                                      : lanes / 6;
+    return ops->launch_team_field && n <= most;
 }
 
 // Slots per block and blocks of a team launch: as many blocks as are resident
 // before a block takes a second slot (a lone trajectory's step is the
-// shortest), at most kTeamSlots slots.
+// shortest), at most the set's kTeamSlotsOf.
 static int team_shape(cor_ctx* ctx, const ModelOps* ops, uint64_t live, int* slots, unsigned* blocks) {
-    int per_sm = 0;
-    CUDA_TRY(ctx, ops->team_occupancy(kTeamSlots, &per_sm));
+    int per_sm = 0, most = 1;
+    CUDA_TRY(ctx, ops->team_occupancy(&most, &per_sm));
     if (per_sm < 1) per_sm = 1;
     const uint64_t cap = (uint64_t)per_sm * (uint64_t)ctx->sms;
     uint64_t n = (live + cap - 1) / cap;
-    if (n > (uint64_t)kTeamSlots) n = kTeamSlots;
+    if (n > (uint64_t)most) n = most;
     const uint64_t b = (live + n - 1) / n;
     *slots = (int)n;
     *blocks = (unsigned)(b < cap ? b : cap);

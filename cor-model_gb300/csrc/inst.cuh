@@ -69,8 +69,9 @@
     }                                                                                                      \
     template <class MS, bool TEAM = MS::crustal == 0>                                                      \
     struct Team_##NAME {                                                                                   \
-        static cudaError_t occ(int n_slots, int* n) {                                                      \
-            const size_t smem = (size_t)n_slots * sizeof(TeamSlot<MS>);                                    \
+        static cudaError_t occ(int* n_slots, int* n) {                                                     \
+            *n_slots = kTeamSlotsOf<MS>;                                                                   \
+            const size_t smem = (size_t)*n_slots * sizeof(TeamSlot<MS>);                                   \
             cudaError_t e = cudaFuncSetAttribute(team_trace_kernel<MS>,                                    \
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
             if (e != cudaSuccess) return e;                                                                \
@@ -81,7 +82,7 @@
             cudaError_t e = cudaFuncSetAttribute(team_trace_kernel<MS>,                                    \
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
             if (e != cudaSuccess) return e;                                                                \
-            team_trace_kernel<MS><<<blocks, kTeamThreads, smem, s>>>(a, n_slots);                          \
+            team_trace_kernel<MS><<<blocks, team_threads(n_slots), smem, s>>>(a, n_slots);                 \
             return cudaGetLastError();                                                                     \
         }                                                                                                  \
         static cudaError_t field(const DevParams* p, int np, const int32_t* idx, const double* pos, int64_t n, \
@@ -90,7 +91,7 @@
             cudaError_t e = cudaFuncSetAttribute(team_field_kernel<MS>,                                    \
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
             if (e != cudaSuccess) return e;                                                                \
-            team_field_kernel<MS><<<blocks, kTeamThreads, smem, s>>>(p, np, idx, pos, n, out, n_slots);    \
+            team_field_kernel<MS><<<blocks, team_threads(n_slots), smem, s>>>(p, np, idx, pos, n, out, n_slots);\
             return cudaGetLastError();                                                                     \
         }                                                                                                  \
         static constexpr auto occ_ptr = &occ;                                                              \

@@ -23,8 +23,9 @@ struct ModelOps {
     cudaError_t (*stream_occupancy)(int* blocks_per_sm);
     cudaError_t (*launch_stream)(const StreamArgs& a, unsigned blocks, cudaStream_t s);
     // the scan by teams (team.cuh): blocks of n_slots trajectories each; null
-    // for sets without it
-    cudaError_t (*team_occupancy)(int n_slots, int* blocks_per_sm);
+    // for sets without it.  team_occupancy: the most slots a block can have, and
+    // how many such blocks an SM holds.
+    cudaError_t (*team_occupancy)(int* n_slots, int* blocks_per_sm);
     cudaError_t (*launch_team)(const TraceArgs& a, int n_slots, unsigned blocks, cudaStream_t s);
     // launch_field by teams
     cudaError_t (*launch_team_field)(const DevParams* params, int n_params, const int32_t* pidx, const double* pos,

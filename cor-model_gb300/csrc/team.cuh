@@ -1,6 +1,6 @@
-// team.cuh -- block-cooperative trajectory steps: a block of four warps holds
-// a few trajectories ("slots") and spreads every field evaluation over all of
-// its threads.
+// team.cuh -- block-cooperative trajectory steps: a block of eight warps holds
+// up to 32 trajectories ("slots") and spreads every field evaluation over all
+// of its threads.
 //
 // An FP64 warp instruction holds its sub-partition for 64 cycles however many
 // lanes are active, four sub-partitions together retire one per 19 cycles, and
@@ -20,10 +20,10 @@
 // not move by a bit.
 //
 // Measured (IGRF-14): a lone trajectory's accepted step 126 us by one lane,
-// 43 us by a team; one site of 400 rigidities, limit 2,500 steps, 331-507 ms
-// and 109 ms; 8,000 trajectories, limit 1,000 steps, 243 ms and 86 ms.  The
-// step is bound by the quads' trials (about 115 FP64 instructions each, 3.3
-// per step) and the 105-term sums.
+// 41 us by a team; one site of 400 rigidities, limit 2,500 steps, 331-507 ms
+// and 104 ms; 8,000 trajectories, limit 1,000 steps, 243 ms and 81 ms.  A lone
+// step is bound by the quad's trials (about 115 FP64 instructions each, 3.3
+// per step) and the 105-term sums, a full block by the FP64 pipe.
 #pragma once
 
 #include <type_traits>
@@ -40,9 +40,17 @@ __device__ __forceinline__ double comp(const Vec3 v, const int c) { return c == 
 
 namespace cor {
 
-constexpr int kTeamThreads = 128;
+constexpr int kTeamThreads = 256;
 constexpr int kTeamWarps = kTeamThreads / 32;
-constexpr int kTeamSlots = 8;   // at most: one warp's quads (16 slots were no faster)
+constexpr int kTeamSlots = 32;                 // one bit each in a warp's masks
+constexpr int kTeamSharedBytes = 224 * 1024;   // of 227 KB, TeamShared besides
+
+// Threads of a block of n slots: eight warps, or six for a few slots, whose
+// warps mostly find the chunk counters run out (1,000 T96 steps of one
+// trajectory 58.4 ms with eight, 56.4 with six; 400 trajectories at three
+// slots each 60.6 and 58.6; at 13 slots and more six are 3-5 % slower).
+constexpr int team_threads(const int n_slots) { return n_slots <= 4 ? 192 : kTeamThreads; }
+static_assert(6 * kTeamSlots <= kTeamThreads && 6 * 4 <= team_threads(4), "team_field's last phase is one pass");
 constexpr unsigned kFull = 0xffffffffu;
 
 // ---- quad helpers ---------------------------------------------------------
@@ -453,6 +461,22 @@ struct TeamSlot : TeamSlotBody<MS> {
     double pad[1 + (sizeof(TeamSlotBody<MS>) / 8) % 2];
 };
 
+// Slots per block, at most.  With an external model as many as shared memory
+// holds (19 with T96, 29 with TS05): most kinds of task are a few per slot, a
+// chunk of them costs its 32 lanes whether they are filled or not, and blocks
+// of 128 threads and 8 slots, two to an SM, filled 8 to 24 (3,573 TS05
+// trajectories of 400 steps 173 ms with those, 135 with one block of 16
+// slots, 96 with 24; 8,000 T96 trajectories of 250 steps 110, 94 and, with 18
+// slots, 81).  The internal field alone has enough terms to fill its chunks,
+// and two blocks of 16 slots overlap one's steps with the other's fields
+// (8,000 trajectories of 1,000 steps: 81 ms; one block of 32 slots 96, two of
+// 12 106).
+template <class MS>
+constexpr int kTeamSlotsOf = MS::external == 0 ? 16
+                             : kTeamSharedBytes / (int)sizeof(TeamSlot<MS>) < kTeamSlots
+                                 ? kTeamSharedBytes / (int)sizeof(TeamSlot<MS>)
+                                 : kTeamSlots;
+
 // The field of the slots in `mask` (not 0), from what the quads wrote.  All
 // threads of the block; the phases are separated by block barriers, and
 // within one the warps take chunks of 32 tasks, the longest kinds first.
@@ -470,8 +494,9 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
         bool any = false;
         if constexpr (kT96) {
             any = true;
-            if (takes(ch, 1)) {
-                t96_task_b1(slots[list[lane < 2 * n ? lane >> 1 : 0]].t96, lane < 2 * n);
+            if (takes(ch, chunks(2 * n))) {
+                const int t = (int)ch * 32 + lane;
+                t96_task_b1(slots[list[t < 2 * n ? t >> 1 : 0]].t96, t < 2 * n);
             } else if (takes(ch, chunks(6 * n))) {
                 const int t = (int)ch * 32 + lane;
                 if (t < 6 * n) t96_task_rt(slots[list[t % n]].t96, t / n);
@@ -502,10 +527,12 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
                     TS05Slot& s = slots[list[lane]].ts05;
                     put3(s.cf, ts05_shlcar3x3(s.x, s.y, s.z));
                 }
-            } else if (takes(ch, 1)) {
-                if (lane < 2 * n) ts05_task_birk(slots[list[lane >> 1]].ts05, lane & 1);
-            } else if (takes(ch, 1)) {
-                if (lane < 2 * n) ts05_task_symm(slots[list[lane >> 1]].ts05, lane & 1);
+            } else if (takes(ch, chunks(2 * n))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 2 * n) ts05_task_birk(slots[list[t >> 1]].ts05, t & 1);
+            } else if (takes(ch, chunks(2 * n))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 2 * n) ts05_task_symm(slots[list[t >> 1]].ts05, t & 1);
             } else if (takes(ch, 1)) {
                 if (lane < n) ts05_task_quad(slots[list[lane]].ts05);
             } else if (takes(ch, 1)) {
@@ -619,12 +646,15 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
             } else if (takes(ch, chunks(4 * nc))) {
                 const int t = (int)ch * 32 + lane;
                 if (t < 4 * nc) ts05_task_ap(slots[lc[t % nc]].ts05, 1, t / nc);
-            } else if (takes(ch, nc ? 1 : 0)) {
-                if (lane < 3 * nc) ts05_task_br(slots[lc[lane % nc]].ts05, lane / nc);
-            } else if (takes(ch, nc ? 1 : 0)) {
-                if (lane < 3 * nc) ts05_task_bt(slots[lc[lane % nc]].ts05, lane / nc);
-            } else if (takes(ch, nc ? 1 : 0)) {
-                if (lane < 2 * nc) ts05_task_disk(slots[lc[lane >> 1]].ts05, lane & 1);
+            } else if (takes(ch, chunks(3 * nc))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 3 * nc) ts05_task_br(slots[lc[t % nc]].ts05, t / nc);
+            } else if (takes(ch, chunks(3 * nc))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 3 * nc) ts05_task_bt(slots[lc[t % nc]].ts05, t / nc);
+            } else if (takes(ch, chunks(2 * nc))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 2 * nc) ts05_task_disk(slots[lc[t >> 1]].ts05, t & 1);
             } else if (takes(ch, chunks(4 * nc))) {
                 const int t = (int)ch * 32 + lane;
                 if (t < 4 * nc) ts05_task_ap(slots[lc[t % nc]].ts05, 0, t / nc);
@@ -691,8 +721,9 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
         bool any = false;
         if constexpr (kSh) {
             any = true;
-            if (takes(ch, 1)) {
-                if (lane < 2 * n) sh_sum<kFma<MS>>(slots[list[lane >> 1]].sh, lane & 1);
+            if (takes(ch, chunks(2 * n))) {
+                const int t = (int)ch * 32 + lane;
+                if (t < 2 * n) sh_sum<kFma<MS>>(slots[list[t >> 1]].sh, t & 1);
             } else if (takes(ch, chunks(n * (kShCols - 1)))) {
                 const int t = (int)ch * 32 + lane;
                 if (t < n * (kShCols - 1)) sh_sum<kFma<MS>>(slots[list[t % n]].sh, 2 + t / n);
@@ -706,10 +737,12 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
                 if (takes(ch, chunks(50 * nc))) {
                     const int t = (int)ch * 32 + lane;
                     if (t < 50 * nc) ts05_task_exp(slots[lc[t % nc]].ts05, t / nc);
-                } else if (takes(ch, nc ? 1 : 0)) {
-                    if (lane < 2 * nc) ts05_end_birk(slots[lc[lane >> 1]].ts05, lane & 1);
-                } else if (takes(ch, nc ? 1 : 0)) {
-                    if (lane < 2 * nc) ts05_end_symm(slots[lc[lane >> 1]].ts05, lane & 1);
+                } else if (takes(ch, chunks(2 * nc))) {
+                    const int t = (int)ch * 32 + lane;
+                    if (t < 2 * nc) ts05_end_birk(slots[lc[t >> 1]].ts05, t & 1);
+                } else if (takes(ch, chunks(2 * nc))) {
+                    const int t = (int)ch * 32 + lane;
+                    if (t < 2 * nc) ts05_end_symm(slots[lc[t >> 1]].ts05, t & 1);
                 } else if (takes(ch, nc ? 1 : 0)) {
                     if (lane < nc) ts05_end_quad(slots[lc[lane]].ts05);
                 } else {
@@ -720,10 +753,12 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
         if constexpr (kT96) {
             if (!any) {
                 any = true;
-                if (takes(ch, nc ? 1 : 0)) {
-                    if (lane < 3 * nc) t96_sum_con(slots[lc[lane % nc]].t96, lane / nc);
-                } else if (takes(ch, nl ? 1 : 0)) {
-                    if (lane < 3 * nl) t96_sum_loops(slots[ll[lane % nl]].t96, lane / nl);
+                if (takes(ch, chunks(3 * nc))) {
+                    const int t = (int)ch * 32 + lane;
+                    if (t < 3 * nc) t96_sum_con(slots[lc[t % nc]].t96, t / nc);
+                } else if (takes(ch, chunks(3 * nl))) {
+                    const int t = (int)ch * 32 + lane;
+                    if (t < 3 * nl) t96_sum_loops(slots[ll[t % nl]].t96, t / nl);
                 } else if (takes(ch, no ? 1 : 0)) {
                     if (lane < no) t96_sum_outer(slots[lo[lane]].t96);
                 } else if (takes(ch, ni ? 1 : 0)) {
@@ -736,8 +771,9 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
                     }
                 } else if (takes(ch, 1)) {
                     if (lane < n) t96_sum_t87(slots[list[lane]].t96);
-                } else if (takes(ch, 1)) {
-                    if (lane < 3 * n) t96_sum_cyl(slots[list[lane % n]].t96, lane / n);
+                } else if (takes(ch, chunks(3 * n))) {
+                    const int t = (int)ch * 32 + lane;
+                    if (t < 3 * n) t96_sum_cyl(slots[list[t % n]].t96, t / n);
                 } else if (takes(ch, chunks(6 * n))) {
                     const int t = (int)ch * 32 + lane;
                     if (t < 6 * n) {
@@ -754,7 +790,7 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
     }
     __syncthreads();
     if constexpr (kTS05) {
-        const int t = (int)threadIdx.x;   // one pass: at most 6 kTeamSlots tasks
+        const int t = (int)threadIdx.x;   // one pass: at most 6 tasks per slot
         if (t < 6 * nc) {
             const int k = t / nc;
             ts05_sum5(slots[lc[t % nc]].ts05, k / 3, k % 3);
@@ -850,7 +886,7 @@ __global__ void __launch_bounds__(kTeamThreads)
 }
 
 // The scan by teams: one generation, as trace_kernel's.  `n_slots` (at most
-// kTeamSlots) trajectories per block.
+// kTeamSlotsOf<MS>) trajectories per block.
 
 template <class MS>
 __global__ void __launch_bounds__(kTeamThreads) team_trace_kernel(const TraceArgs a, const int n_slots) {
