@@ -20,9 +20,9 @@
 // not move by a bit.
 //
 // Measured (IGRF-14): a lone trajectory's accepted step 126 us by one lane,
-// 41 us by a team; one site of 400 rigidities, limit 2,500 steps, 331-507 ms
-// and 104 ms; 8,000 trajectories, limit 1,000 steps, 243 ms and 81 ms.  A lone
-// step is bound by the quad's trials (about 115 FP64 instructions each, 3.3
+// 39.6 us by a team; one site of 400 rigidities, limit 2,500 steps, 331-507 ms
+// and 100 ms; 8,000 trajectories, limit 1,000 steps, 243 ms and 79 ms.  A lone
+// step is bound by the quad's trials (about 110 FP64 instructions each, 3.9
 // per step) and the 105-term sums, a full block by the FP64 pipe.
 #pragma once
 
@@ -96,6 +96,19 @@ __device__ __forceinline__ Vec3 quad_rk_position(const double h, const Vec3 v, c
     return quad_gather(rk_position_1(h, comp(v, c), comp(x, c)));
 }
 
+// One component of geo_to_gsm and gsm_to_geo: the quad's lanes take one each
+// and gather.  With the end of the internal field and the turn's two scalar
+// products split the same way, a lone trajectory's step went from 41.5 us to
+// 39.6 (IGRF-14) and from 57.2 to 52.9 (T96).
+__device__ __forceinline__ double gsm_comp(const Vec3 g, const cor_model_params* __restrict__ p, const int c) {
+    const double* a = c == 0 ? p->a1 : c == 1 ? p->a2 : p->a3;
+    return __ldg(&a[0]) * g.x + __ldg(&a[1]) * g.y + __ldg(&a[2]) * g.z;
+}
+
+__device__ __forceinline__ double geo_comp(const Vec3 s, const cor_model_params* __restrict__ p, const int c) {
+    return __ldg(&p->a1[c]) * s.x + __ldg(&p->a2[c]) * s.y + __ldg(&p->a3[c]) * s.z;
+}
+
 // t / nk0 for nk0 = nk1 2^k, given r1 = RN(1 / nk1): the quotient by nk1 in
 // three operations, then an exact shift of its exponent, where both are
 // normal numbers (else the division itself).
@@ -115,7 +128,7 @@ __device__ __forceinline__ int quad_advance(Lane& L, const TraceArgs& a, bool ru
     const int q = threadIdx.x & 3, c = q == 3 ? 2 : q;
     const double zn = run ? L.job->zn : 1.;
     const int nk1 = run ? L.job->nk1 : 1;
-    const cor_model_params* __restrict__ p = run ? &L.par->p : nullptr;
+    const cor_model_params* __restrict__ p = run ? &L.par->p : &a.params->p;
     // per trajectory and per step what the trials share; h = t / (nk1 2^k) is
     // the correctly rounded t / nk1 scaled by a power of two
     const double dq = 1.E-09 * zn * kQ, tb = fabs(zn) * kQ * L.b, r1 = 1. / nk1;
@@ -132,6 +145,10 @@ __device__ __forceinline__ int quad_advance(Lane& L, const TraceArgs& a, bool ru
             const double t = quad_get(td, 0), d = quad_get(td, 2);
             const double hh = gyro_step(t, nk1, r1, L.nk0);
             const Vec3 n = quad_rk_velocity(hh, d, L.field, L.vel, c);
+            // |n|^2 by lanes 0, 1 and the cosine's numerator by lanes 2, 3
+            const Vec3 w = q < 2 ? n : L.vel;
+            const double nw = n.x * w.x + n.y * w.y + n.z * w.z;
+            const double n2 = quad_get(nw, 0), nv0 = quad_get(nw, 2);
             if (trial) {
                 L.step++;
                 if (vc > 1.) {
@@ -140,9 +157,8 @@ __device__ __forceinline__ int quad_advance(Lane& L, const TraceArgs& a, bool ru
                 } else {
                     const double vprev = L.v;
                     L.trials++;
-                    L.v = sqrt(n.x * n.x + n.y * n.y + n.z * n.z);
-                    const bool reject =
-                        turn_rejects(a, n.x * L.vel.x + n.y * L.vel.y + n.z * L.vel.z, L.v * vprev);
+                    L.v = sqrt(n2);
+                    const bool reject = turn_rejects(a, nv0, L.v * vprev);
                     if (reject && L.nk0 <= 50000) {
                         L.nk0 *= 2;
                         L.step--;
@@ -156,9 +172,9 @@ __device__ __forceinline__ int quad_advance(Lane& L, const TraceArgs& a, bool ru
             __syncwarp();
         }
         const Vec3 np = quad_rk_position(h, L.vel, L.pos, c);
+        const Vec3 gsm = quad_gather(gsm_comp(np, p, c));
         if (run) {
             const double rr = sqrt(np.x * np.x + np.y * np.y + np.z * np.z);
-            const Vec3 gsm = geo_to_gsm(np, p);
             const double pax = div_c(DIVRE(gsm.x) + 25.3, 36.08, 1. / 36.08);
             const double paz = DIVRE2(gsm.y * gsm.y + gsm.z * gsm.z);
             const double r = DIVRE(rr);
@@ -387,9 +403,9 @@ __device__ __forceinline__ void sh_sum(ShSlot& s, const int which) {
     s.sum[which] = acc;
 }
 
-// The end of internal_geo, by the quad.
+// The end of internal_geo, by the quad: component c.
 template <bool FMA>
-__device__ __forceinline__ Vec3 sh_finish(const ShSlot& s) {
+__device__ __forceinline__ double sh_finish(const ShSlot& s, const int c) {
     const double br = s.sum[0], bt = s.sum[1], C = s.C, S = s.S, cf = s.cf, sf = s.sf;
     double bf = 0., bphi;
 #pragma unroll
@@ -404,11 +420,8 @@ __device__ __forceinline__ Vec3 sh_finish(const ShSlot& s) {
         bphi = bf / S;
     }
     const double he = sh_mad<FMA>(br, S, __dmul_rn(bt, C));
-    Vec3 b;
-    b.x = sh_mad<FMA>(he, cf, -__dmul_rn(bphi, sf));
-    b.y = sh_mad<FMA>(he, sf, __dmul_rn(bphi, cf));
-    b.z = sh_mad<FMA>(br, C, -__dmul_rn(bt, S));
-    return b;
+    return sh_mad<FMA>(c < 2 ? he : br, c == 0 ? cf : c == 1 ? sf : C,
+                       __dmul_rn(c < 2 ? bphi : bt, c == 0 ? -sf : c == 1 ? cf : -S));
 }
 
 // ---- the block's task loop ----------------------------------------------------
@@ -800,15 +813,14 @@ __device__ __forceinline__ void team_field(TeamShared& ts, TeamSlot<MS>* slots, 
     if (threadIdx.x == 0) ts.next[2] = ts.next[3] = 0;
 }
 
-// What a quad writes for its slot before team_field (all lanes of the warp
-// call; need: the quad's slot is evaluated) and reads after it.
+// What a quad writes for its slot before team_field and reads after it (all
+// lanes of the warp call, with any par; need: the quad's slot is evaluated).
 template <class MS>
 __device__ __forceinline__ void team_begin(TeamSlot<MS>& s, const Vec3 pos, const DevParams* par, const bool need) {
     if constexpr (MS::internal != 0) {
-        Vec3 geo = {1., 0., 0.};
-        if (need) geo = gsm_to_geo(pos, &par->p);
-        __syncwarp();
-        quad_sh_geometry(s.sh, geo, need ? &par->p : nullptr, need);
+        const int q = threadIdx.x & 3, c = q == 3 ? 2 : q;
+        const Vec3 geo = quad_gather(geo_comp(pos, &par->p, c));
+        quad_sh_geometry(s.sh, need ? geo : Vec3{1., 0., 0.}, need ? &par->p : nullptr, need);
     }
     if constexpr (MS::external == COR_EXTERNAL_T96) {
         if (need && (threadIdx.x & 3) == 0) t96_slot_start(s.t96, par->t96, pos);
@@ -820,28 +832,25 @@ __device__ __forceinline__ void team_begin(TeamSlot<MS>& s, const Vec3 pos, cons
 }
 
 template <class MS>
-__device__ __forceinline__ Vec3 team_end(const TeamSlot<MS>& s, const DevParams* par) {
+__device__ __forceinline__ Vec3 team_end(const TeamSlot<MS>& s, const DevParams* par, const bool need) {
     const cor_model_params* p = &par->p;
-    Vec3 tot = {0., 0., 0.};
+    const int q = threadIdx.x & 3, c = q == 3 ? 2 : q;
+    double tot = 0.;
     if constexpr (MS::internal != 0) {
-        const Vec3 bs = geo_to_gsm(sh_finish<kFma<MS>>(s.sh), p);
-        tot.x += bs.x;
-        tot.y += bs.y;
-        tot.z += bs.z;
+        double b = 0.;
+        if (need) b = sh_finish<kFma<MS>>(s.sh, c);
+        __syncwarp();
+        tot += gsm_comp(quad_gather(b), p, c);
     }
     if constexpr (MS::external == COR_EXTERNAL_T96) {
-        const Vec3 b = t96_slot_end(s.t96);
-        tot.x += b.x;
-        tot.y += b.y;
-        tot.z += b.z;
+        if (need) tot += comp(t96_slot_end(s.t96), c);
+        __syncwarp();
     }
     if constexpr (MS::external == COR_EXTERNAL_TS05) {
-        const Vec3 b = ts05_slot_end(s.ts05);
-        tot.x += b.x;
-        tot.y += b.y;
-        tot.z += b.z;
+        if (need) tot += comp(ts05_slot_end(s.ts05), c);
+        __syncwarp();
     }
-    return gsm_to_geo(tot, p);
+    return quad_gather(geo_comp(quad_gather(tot), p, c));
 }
 
 // The field at n points by teams (field_kernel's arguments): block b takes
@@ -859,7 +868,8 @@ __global__ void __launch_bounds__(kTeamThreads)
         const int64_t i = i0 + slot;
         const bool need = slot < n_slots && i < n;
         const DevParams* par = params;
-        if (__any_sync(kFull, need)) {
+        const bool warp_need = __any_sync(kFull, need);
+        if (warp_need) {
             Vec3 x = {0., 0., 0.};
             if (need) {
                 const int k = pidx ? pidx[i] : 0;
@@ -873,15 +883,14 @@ __global__ void __launch_bounds__(kTeamThreads)
         const int m = left < n_slots ? (int)left : n_slots;
         __syncthreads();
         team_field<MS>(ts, slots, m == 32 ? kFull : (1u << m) - 1u);
-        if (need) {
-            const Vec3 b = team_end<MS>(slots[slot], par);
-            if ((tid & 3) == 0) {
+        if (warp_need) {
+            const Vec3 b = team_end<MS>(slots[slot < n_slots ? slot : 0], par, need);
+            if (need && (tid & 3) == 0) {
                 out[3 * i] = b.x;
                 out[3 * i + 1] = b.y;
                 out[3 * i + 2] = b.z;
             }
         }
-        __syncwarp();
     }
 }
 
@@ -902,6 +911,7 @@ __global__ void __launch_bounds__(kTeamThreads) team_trace_kernel(const TraceArg
     L.b = 1.;
     L.nk0 = 1;
     L.vel = L.pos = L.field = L.gsm = Vec3{0., 0., 0.};
+    L.par = a.params;
     bool has = false, done = slot >= n_slots;
     unsigned long long n_steps = 0, n_trials = 0, n_traj = 0, n_wd = 0;
     const bool rig_major = a.rig_major && (!a.grid_ok || *(volatile const unsigned int*)a.grid_ok != 0u);
@@ -972,11 +982,14 @@ __global__ void __launch_bounds__(kTeamThreads) team_trace_kernel(const TraceArg
             continue;
         }
         team_field<MS>(ts, slots, mask);
-        if (need) {
-            L.field = team_end<MS>(slots[slot], L.par);
-            L.b = 1.E-09 * sqrt(L.field.x * L.field.x + L.field.y * L.field.y + L.field.z * L.field.z);
+        if (warp_need) {
+            const Vec3 f = team_end<MS>(slots[slot < n_slots ? slot : 0], L.par, need);
+            if (need) {
+                L.field = f;
+                L.b = 1.E-09 * sqrt(L.field.x * L.field.x + L.field.y * L.field.y + L.field.z * L.field.z);
+            }
+            __syncwarp();
         }
-        __syncwarp();
     }
     warp_add_u64(reinterpret_cast<unsigned long long*>(&a.counters->accepted_steps), n_steps);
     warp_add_u64(reinterpret_cast<unsigned long long*>(&a.counters->trials), n_trials);
