@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kTraceThreads, 1) stream_kernel(const StreamAr
         bool need_field = false, need_reduce = false;
         int red_j = 0;
         if (has) {
-            const int st = lane_advance(L, a);
+            const int st = lane_advance<kPlain<MS>>(L, a);
             if (st == 0) {
                 need_field = true;
             } else {

@@ -64,6 +64,7 @@ __device__ __forceinline__ Vec3 quad_gather(const double v) {
 
 // rk_velocity with one component per lane: stage k's cross product needs the
 // two other components of the stage velocity, which the quad exchanges.
+template <bool PLAIN>
 __device__ __forceinline__ Vec3 quad_rk_velocity(const double h, const double d, const Vec3 f, const Vec3 v,
                                                  const int c) {
     const int c1 = c == 2 ? 0 : c + 1, c2 = c == 0 ? 2 : c - 1;
@@ -75,16 +76,16 @@ __device__ __forceinline__ Vec3 quad_rk_velocity(const double h, const double d,
     const double s2 = vc + DIV3(a1);
     OTHERS(s2);
     const double a2 = CROSS(s2p, s2q);
-    const double s3 = vc + DIV25(4. * a1 + 6. * a2);
+    const double s3 = rk_3<PLAIN>(vc, a1, a2);
     OTHERS(s3);
     const double a3 = CROSS(s3p, s3q);
-    const double s4 = vc + DIV4(a1 - 12. * a2 + 15. * a3);
+    const double s4 = rk_4<PLAIN>(vc, a1, a2, a3);
     OTHERS(s4);
     const double a4 = CROSS(s4p, s4q);
-    const double s5 = vc + DIV81(6. * a1 + 90. * a2 - 50. * a3 + 8. * a4);
+    const double s5 = rk_5<PLAIN>(vc, a1, a2, a3, a4);
     OTHERS(s5);
     const double a5 = CROSS(s5p, s5q);
-    const double s6 = vc + DIV75(6. * a1 + 36. * a2 + 10. * a3 + 8. * a4);
+    const double s6 = rk_6<PLAIN>(vc, a1, a2, a3, a4);
     OTHERS(s6);
     const double a6 = CROSS(s6p, s6q);
 #undef CROSS
@@ -92,8 +93,9 @@ __device__ __forceinline__ Vec3 quad_rk_velocity(const double h, const double d,
     return quad_gather(vc + DIV192(23. * a1 + 125. * a3 - 81. * a5 + 125. * a6));
 }
 
+template <bool PLAIN>
 __device__ __forceinline__ Vec3 quad_rk_position(const double h, const Vec3 v, const Vec3 x, const int c) {
-    return quad_gather(rk_position_1(h, comp(v, c), comp(x, c)));
+    return quad_gather(rk_position_1<PLAIN>(h, comp(v, c), comp(x, c)));
 }
 
 // One component of geo_to_gsm and gsm_to_geo: the quad's lanes take one each
@@ -124,6 +126,7 @@ __device__ __forceinline__ double gyro_step(const double t, const int nk1, const
 // calls it, `run` says whether the lane's quad holds a trajectory.  The trial
 // loop runs while any quad of the warp has a trial to make, with the others'
 // lanes computing on without effect.  Returns the class of run lanes' quads.
+template <bool PLAIN>
 __device__ __forceinline__ int quad_advance(Lane& L, const TraceArgs& a, bool run) {
     const int q = threadIdx.x & 3, c = q == 3 ? 2 : q;
     const double zn = run ? L.job->zn : 1.;
@@ -144,7 +147,7 @@ __device__ __forceinline__ int quad_advance(Lane& L, const TraceArgs& a, bool ru
             const double td = (q < 2 ? 2. * kPi * hm : dq) / (q < 2 ? tb : hm);
             const double t = quad_get(td, 0), d = quad_get(td, 2);
             const double hh = gyro_step(t, nk1, r1, L.nk0);
-            const Vec3 n = quad_rk_velocity(hh, d, L.field, L.vel, c);
+            const Vec3 n = quad_rk_velocity<PLAIN>(hh, d, L.field, L.vel, c);
             // |n|^2 by lanes 0, 1 and the cosine's numerator by lanes 2, 3
             const Vec3 w = q < 2 ? n : L.vel;
             const double nw = n.x * w.x + n.y * w.y + n.z * w.z;
@@ -171,7 +174,7 @@ __device__ __forceinline__ int quad_advance(Lane& L, const TraceArgs& a, bool ru
             }
             __syncwarp();
         }
-        const Vec3 np = quad_rk_position(h, L.vel, L.pos, c);
+        const Vec3 np = quad_rk_position<PLAIN>(h, L.vel, L.pos, c);
         const Vec3 gsm = quad_gather(gsm_comp(np, p, c));
         if (run) {
             const double rr = sqrt(np.x * np.x + np.y * np.y + np.z * np.z);
@@ -918,7 +921,7 @@ __global__ void __launch_bounds__(kTeamThreads) team_trace_kernel(const TraceArg
     for (;;) {
         bool need = false;
         if (__any_sync(kFull, has)) {
-            const int st = quad_advance(L, a, has);
+            const int st = quad_advance<kPlain<MS>>(L, a, has);
             if (has) {
                 if (st == 0) {
                     need = true;

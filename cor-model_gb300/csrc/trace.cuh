@@ -102,6 +102,10 @@ __device__ __forceinline__ int find_job(const uint64_t* __restrict__ off, int n_
     return lo;
 }
 
+// The sets whose units are compiled without FMA contraction.
+template <class MS>
+constexpr bool kPlain = MS::external == 0 && MS::crustal == 0;
+
 // Per-lane trajectory state.
 struct Lane {
     Vec3 pos, vel, field, gsm;
@@ -244,19 +248,23 @@ __device__ __forceinline__ bool turn_rejects(const TraceArgs& a, const double do
 // with the field evaluation left to the caller.  Bounded: at most 10
 // turn-angle halvings (nk0 <= 50000) plus at most 30 boundary halvings
 // (nk0 < 2^30) per step.
+template <bool PLAIN = false>
 __device__ __forceinline__ int lane_advance(Lane& L, const TraceArgs& a) {
     const double zn = L.job->zn;
     const int nk1 = L.job->nk1;
+    // every trial of the step divides by it (with an external model, whose
+    // kernels are short of registers, its reciprocal costs what it gives)
+    const double tb = fabs(zn) * kQ * L.b, rtb = PLAIN ? 1. / tb : 0.;
     for (;;) {
         L.step++;
         const double vc = DIVC(L.v);
         if (vc > 1.) return COR_TRAJ_SUPERLUM;  // :48-54
         const double hm = a.mass / sqrt(1. - vc * vc);
-        const double t = (2. * kPi * hm) / (fabs(zn) * kQ * L.b);
+        const double t = PLAIN ? div_r(2. * kPi * hm, tb, rtb) : (2. * kPi * hm) / tb;
         const double h = t / L.nk0;
         const double d = (1.E-09 * zn * kQ) / hm;
         const double vprev = L.v;
-        const Vec3 nv = rk_velocity(h, d, L.field, L.vel);
+        const Vec3 nv = rk_velocity<PLAIN>(h, d, L.field, L.vel);
         L.trials++;
         L.v = sqrt(nv.x * nv.x + nv.y * nv.y + nv.z * nv.z);
         const bool reject = turn_rejects(a, nv.x * L.vel.x + nv.y * L.vel.y + nv.z * L.vel.z, L.v * vprev);
@@ -265,7 +273,7 @@ __device__ __forceinline__ int lane_advance(Lane& L, const TraceArgs& a) {
             L.step--;
             continue;
         }
-        const Vec3 np = rk_position(h, L.vel, L.pos);
+        const Vec3 np = rk_position<PLAIN>(h, L.vel, L.pos);
         const double rr = sqrt(np.x * np.x + np.y * np.y + np.z * np.z);  // car_to_sph radius
         const Vec3 gsm = geo_to_gsm(np, &L.par->p);
         const double pax = div_c(DIVRE(gsm.x) + 25.3, 36.08, 1. / 36.08);
@@ -466,7 +474,7 @@ __global__ void __launch_bounds__(kTraceThreads, 1) trace_kernel(const TraceArgs
     for (;;) {
         bool need_field = false;
         if (has) {
-            const int st = lane_advance(L, a);
+            const int st = lane_advance<kPlain<MS>>(L, a);
             if (st == 0) {
                 need_field = true;
                 if (a.step_records && L.step <= a.step_cap) {
