@@ -328,6 +328,18 @@ static bool team_takes_field(const ModelOps* ops, cor_model_set models, uint64_t
     return ops->launch_team_field && n <= most;
 }
 
+// Whether a first generation of `live` trajectories runs in blocks of half the
+// threads, two to an SM: IGRF-14 alone, from two trajectories a lane on.  A
+// block's warps wait for its slowest one before each field, and with two
+// blocks the other's warps have the FP64 pipe meanwhile.  ms in whole blocks /
+// in halves: 60,000 trajectories 315-324 / 331-348 (the lanes end in fewer,
+// longer rounds), 76,000 375-388 / 352-362, 91,200 451-466 / 423-435, 200,000
+// of 300 steps 503 / 463.  T96's warps are less alike in a block of four
+// (120,000 455 / 479), TS05's are alike anyway (90,000 553 / 551).
+static bool use_halves(const ModelOps* ops, uint64_t live, uint64_t cap_blocks) {
+    return ops->launch_halves && live >= 2 * cap_blocks * (uint64_t)kTraceThreads;
+}
+
 // Slots per block and blocks of a team launch: as many blocks as are resident
 // before a block takes a second slot (a lone trajectory's step is the
 // shortest), at most the set's kTeamSlotsOf.
@@ -387,7 +399,12 @@ static int launch_trace(cor_ctx* ctx, const ModelOps* ops, TraceArgs a, cudaStre
             CUDA_TRY(ctx, ops->launch_team(a, slots, team_blocks, s));
         } else {
             NvtxRange r(g == 0 ? "cor: scan generation 0" : "cor: scan generation (regrouped)");
-            CUDA_TRY(ctx, ops->launch_generation(a, (unsigned)blocks, s));
+            if (g == 0 && a.allow_park && use_halves(ops, live, cap_blocks)) {
+                a.active_threads = kTraceThreads / 2;   // as many lanes and warps in all as whole blocks have
+                CUDA_TRY(ctx, ops->launch_halves(a, (unsigned)(2 * blocks), s));
+            } else {
+                CUDA_TRY(ctx, ops->launch_generation(a, (unsigned)blocks, s));
+            }
         }
         ctx->generations = g + 1;
         if (!a.allow_park) break;

@@ -9,17 +9,17 @@
     namespace cor {                                                                                        \
     using MS_##NAME = ModelSet<I, E, C>;                                                                   \
     static cudaError_t occ_##NAME(int* n) {                                                                \
-        cudaError_t e = cudaFuncSetAttribute(trace_kernel<MS_##NAME>,                                      \
+        cudaError_t e = cudaFuncSetAttribute(trace_kernel<MS_##NAME, kTraceThreads>,                       \
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRegroupSmem); \
         if (e != cudaSuccess) return e;                                                                    \
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, trace_kernel<MS_##NAME>, kTraceThreads,    \
-                                                             kRegroupSmem);                                \
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, trace_kernel<MS_##NAME, kTraceThreads>,    \
+                                                             kTraceThreads, kRegroupSmem);                 \
     }                                                                                                      \
     static cudaError_t gen_##NAME(const TraceArgs& a, unsigned blocks, cudaStream_t s) {                   \
-        cudaError_t e = cudaFuncSetAttribute(trace_kernel<MS_##NAME>,                                      \
+        cudaError_t e = cudaFuncSetAttribute(trace_kernel<MS_##NAME, kTraceThreads>,                       \
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRegroupSmem); \
         if (e != cudaSuccess) return e;                                                                    \
-        trace_kernel<MS_##NAME><<<blocks, kTraceThreads, kRegroupSmem, s>>>(a);                            \
+        trace_kernel<MS_##NAME, kTraceThreads><<<blocks, kTraceThreads, kRegroupSmem, s>>>(a);             \
         return cudaGetLastError();                                                                         \
     }                                                                                                      \
     static cudaError_t socc_##NAME(int* n) {                                                               \
@@ -104,7 +104,25 @@
         static constexpr std::nullptr_t run_ptr = nullptr;                                                 \
         static constexpr std::nullptr_t field_ptr = nullptr;                                               \
     };                                                                                                     \
+    template <class MS, bool HALVES = kPlain<MS>>                                                          \
+    struct Halves_##NAME {                                                                                 \
+        static cudaError_t run(const TraceArgs& a, unsigned blocks, cudaStream_t s) {                      \
+            constexpr int T = kTraceThreads / 2;                                                           \
+            constexpr size_t smem = sizeof(RegroupScratchOf<T>);                                           \
+            cudaError_t e = cudaFuncSetAttribute(trace_kernel<MS, T>,                                      \
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+            if (e != cudaSuccess) return e;                                                                \
+            trace_kernel<MS, T><<<blocks, T, smem, s>>>(a);                                                \
+            return cudaGetLastError();                                                                     \
+        }                                                                                                  \
+        static constexpr auto ptr = &run;                                                                  \
+    };                                                                                                     \
+    template <class MS>                                                                                    \
+    struct Halves_##NAME<MS, false> {                                                                      \
+        static constexpr std::nullptr_t ptr = nullptr;                                                     \
+    };                                                                                                     \
     const ModelOps ops_##NAME = {I * 100 + E * 10 + C, occ_##NAME, gen_##NAME, field_##NAME, tables_##NAME, \
                                  socc_##NAME, stream_##NAME, Team_##NAME<MS_##NAME>::occ_ptr,               \
-                                 Team_##NAME<MS_##NAME>::run_ptr, Team_##NAME<MS_##NAME>::field_ptr};       \
+                                 Team_##NAME<MS_##NAME>::run_ptr, Team_##NAME<MS_##NAME>::field_ptr,         \
+                                 Halves_##NAME<MS_##NAME>::ptr};                                           \
     }

@@ -30,6 +30,8 @@ struct ModelOps {
     // launch_field by teams
     cudaError_t (*launch_team_field)(const DevParams* params, int n_params, const int32_t* pidx, const double* pos,
                                      int64_t n, double* out, int n_slots, unsigned blocks, cudaStream_t s);
+    // launch_generation in blocks of half the threads; null for sets without it
+    cudaError_t (*launch_halves)(const TraceArgs& a, unsigned blocks, cudaStream_t s);
 };
 
 extern const ModelOps ops_igrf, ops_igrf_t96, ops_t96, ops_igrf_ts05, ops_ts05, ops_crustal;

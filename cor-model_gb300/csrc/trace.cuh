@@ -358,12 +358,14 @@ struct LaneMove {
 static_assert(sizeof(LaneMove) == 200, "LaneMove layout");
 
 // Dynamic shared memory of the trace and stream kernels (regroup_lanes).
-struct RegroupScratch {
-    LaneMove mv[kTraceThreads];
-    unsigned key[kTraceThreads];
-    unsigned short at[kTraceThreads];   // the threads that take part, in thread order
-    unsigned warp_live[kTraceWarps];
+template <int THREADS>
+struct RegroupScratchOf {
+    LaneMove mv[THREADS];
+    unsigned key[THREADS];
+    unsigned short at[THREADS];   // the threads that take part, in thread order
+    unsigned warp_live[THREADS / 32];
 };
+using RegroupScratch = RegroupScratchOf<kTraceThreads>;
 constexpr size_t kRegroupSmem = sizeof(RegroupScratch);
 
 // Block-wide: the threads that take part (part: they hold a trajectory whose
@@ -375,8 +377,8 @@ constexpr size_t kRegroupSmem = sizeof(RegroupScratch);
 // the thread it ends on.  JobCopy: L.job points at the thread's own copy of
 // the scan's job (my_job), which then takes the arriving trajectory's zn and
 // nk1.  All threads of the block call this.
-template <bool JobCopy>
-__device__ __forceinline__ void regroup_lanes(RegroupScratch& sc, const bool part, const unsigned key, Lane& L,
+template <bool JobCopy, int THREADS>
+__device__ __forceinline__ void regroup_lanes(RegroupScratchOf<THREADS>& sc, const bool part, const unsigned key, Lane& L,
                                               cor_scan_job* my_job, unsigned& slot, unsigned long long& seq,
                                               const int tid) {
     const int lane = tid & 31, warp = tid >> 5;
@@ -390,7 +392,7 @@ __device__ __forceinline__ void regroup_lanes(RegroupScratch& sc, const bool par
     int rank = 0;
     if (part) {
         // keys of the threads that do not take part are above every real key
-        for (int j = 0; j < kTraceThreads; j++) {
+        for (int j = 0; j < THREADS; j++) {
             const unsigned kj = sc.key[j];
             rank += (kj < key || (kj == key && j < tid)) ? 1 : 0;
         }
@@ -462,10 +464,11 @@ __device__ __forceinline__ void regroup_lanes(RegroupScratch& sc, const bool par
 // warps have parked -- writes its live trajectories to the park list and leaves;
 // the host then launches the next generation sized to the parked count,
 // which restores them densely (the regroup step).
-template <class MS>
-__global__ void __launch_bounds__(kTraceThreads, 1) trace_kernel(const TraceArgs a) {
+// THREADS: kTraceThreads, or half of it for two blocks to an SM (use_halves).
+template <class MS, int THREADS>
+__global__ void __launch_bounds__(THREADS, kTraceThreads / THREADS) trace_kernel(const TraceArgs a) {
     extern __shared__ __align__(16) unsigned char s_dyn[];
-    RegroupScratch& sc = *reinterpret_cast<RegroupScratch*>(s_dyn);
+    RegroupScratchOf<THREADS>& sc = *reinterpret_cast<RegroupScratchOf<THREADS>*>(s_dyn);
     Lane L;
     bool has = false, done = threadIdx.x >= a.active_threads;
     unsigned long long n_steps = 0, n_trials = 0, n_traj = 0, n_wd = 0;
@@ -520,8 +523,8 @@ __global__ void __launch_bounds__(kTraceThreads, 1) trace_kernel(const TraceArgs
         // block-wide decisions: every thread of the block takes the same
         // branch (threads beyond active_threads are done from the start)
         const int n_done = __syncthreads_count(done);
-        if (n_done == kTraceThreads) break;
-        if (a.allow_park && n_done > kTraceThreads - (int)a.active_threads) {
+        if (n_done == THREADS) break;
+        if (a.allow_park && n_done > THREADS - (int)a.active_threads) {
             const int n_live = __syncthreads_count(has);
             unsigned pw = 0;
             if (threadIdx.x == 0) pw = *((volatile unsigned int*)&a.gen->parked_warps);

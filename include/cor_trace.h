@@ -230,8 +230,11 @@ int cor_upload_params(cor_ctx *ctx, const cor_model_params *params, int32_t n_pa
  * park_below lanes per warp are live (0..32; default 16), or once half of the
  * generation's warps have parked; at most max_generations generations run
  * (1..1024; default 48; 1 = never regroup), and a generation with at most
- * min_park live trajectories (default 256) runs them to the end.  Results
- * do not depend on these settings, only the time does. */
+ * min_park live trajectories (default 256) runs them to the end.  A generation
+ * of at most half as many trajectories as the GPU's scan blocks have lanes runs
+ * by teams, each block sharing every step of its trajectories among all of its
+ * threads, to the end as well (not with the crustal model).  Results do not
+ * depend on these settings, only the time does. */
 int cor_ctx_set_regroup(cor_ctx *ctx, int32_t park_below, int32_t max_generations, int64_t min_park);
 
 /* Diagnostics of the last scan on this context (no counterpart in the
@@ -258,7 +261,8 @@ int cor_ctx_set_queue_order(cor_ctx *ctx, int32_t rigidity_major);
  * kernel of cor_trace_batch, cor_trace_batch_device(_noalloc) and
  * cor_trace_steps regroups its trajectories by the branches of the field
  * code their positions take, so that a warp's lanes run the same sub-models;
- * 0: never.  Results do not depend on it (a stream takes the same choice from
+ * 0: never.  Generations that run by teams have nothing to regroup.  Results do
+ * not depend on it (a stream takes the same choice from
  * cor_stream_config.sort_lanes).  Other values give COR_ERR_INVALID.  No
  * counterpart in the reference (its OpenMP threads run one trajectory each,
  * src/trajectory.c:11). */
