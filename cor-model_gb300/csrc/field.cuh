@@ -102,20 +102,23 @@ __device__ __forceinline__ Vec3 calculate_field(const bool want, const Vec3 gsm_
 // field (r2_birk's xksi bands, lib/t96/t96.c:1265-1314), whose outer, sheet
 // and inner fields dominate the divergent work; then, for every model set,
 // the radius in whole R_E (the internal field's degree and T96/TS05's inner
-// structures change with it) and |z|/r in twelfths (latitude bands).
+// structures change with it) and |z|/r in twelfths (latitude bands).  In single
+// precision, whose pipe is idle here: in FP64 it took 1-2 % of a step (66,000
+// streamed T96 trajectories 425 ms with that, 417 with this; 91,200 IGRF-14
+// ones 437 and 435).  Region-1's bases as a further part of the key changed
+// nothing (419, 423).
 template <class MS>
 __device__ __forceinline__ unsigned field_band(const Vec3 gsm_pos, const DevParams* __restrict__ dp) {
     constexpr double kInvRe = 1.0 / kRe;
-    const double x = gsm_pos.x * kInvRe, y = gsm_pos.y * kInvRe, z = gsm_pos.z * kInvRe;
-    const double r = sqrt(x * x + y * y + z * z);
-    const unsigned ri = r < 31.0 ? (unsigned)r : 31u;
-    const double zr = r > 0.0 ? fabs(z) / r : 0.0;
-    const unsigned lat = zr < 1.0 ? (unsigned)(zr * 12.0) : 12u;
+    const float x = (float)(gsm_pos.x * kInvRe), y = (float)(gsm_pos.y * kInvRe), z = (float)(gsm_pos.z * kInvRe);
+    const float r = sqrtf(x * x + y * y + z * z);
+    const unsigned ri = r < 31.0f ? (unsigned)r : 31u;
+    const float zr = r > 0.0f ? fabsf(z) / r : 0.0f;
+    const unsigned lat = zr < 1.0f ? (unsigned)(zr * 12.0f) : 12u;
     unsigned band = 0;
     if constexpr (MS::external == COR_EXTERNAL_T96) {
-        const double xa = dp->t96.xappa;
-        const double xks = t96_xksi(x * xa, y * xa, z * xa);
-        band = xks < -0.045 ? 0u : xks < -0.015 ? 1u : xks < 0.015 ? 2u : xks < 0.045 ? 3u : 4u;
+        const float xa = (float)dp->t96.xappa;
+        band = t96_band(x * xa, y * xa, z * xa);
     }
     return (band << 9) | (ri << 4) | lat;
 }

@@ -679,6 +679,24 @@ __device__ __forceinline__ double t96_xksi(const double x, const double y, const
     return (fg2 / fgh32) - (th * th);
 }
 
+// t96_xksi's band of r2_birk in single precision, for field_band: about 150 FP64
+// operations less per step, of some 11,400.
+__device__ __forceinline__ unsigned t96_band(const float x, const float y, const float z) {
+    const float r = sqrtf(x * x + y * y + z * z), rr = 1.0f / r;
+    const float xr = x * rr, yr = y * rr, zr = z * rr;
+    const float pr = r >= 1.21563f ? sqrtf((r - 1.21563f) * (r - 1.21563f) + 7.50937f * 7.50937f) - 7.50937f : 0.0f;
+    const float f = x + pr * (0.305662f - 0.383593f * xr + 0.2677733f * xr * xr - 0.097656f * yr * yr - 0.636034f * zr * zr);
+    const float g = y + pr * (-0.359862f * yr + 0.424706f * xr * yr);
+    const float h = z + pr * (-0.126366f * zr + 0.292578f * xr * zr);
+    const float fg2 = f * f + g * g, sq = sqrtf(fg2 + h * h);
+    float xks = -1.0f;
+    if (fg2 >= 1.0e-5f) {
+        const float th = sinf(0.3665191f + 0.5f * 0.09599309f * (1.0f - f / sqrtf(fg2)));
+        xks = fg2 / (sq * sq * sq) - th * th;
+    }
+    return xks < -0.045f ? 0u : xks < -0.015f ? 1u : xks < 0.015f ? 2u : xks < 0.045f ? 3u : 4u;
+}
+
 __device__ __forceinline__ double t96_tksi(const double xk, const double x0, const double dx) {
     const double tdz3 = 2.0 * dx * dx * dx;
     if (xk - x0 < -dx) return 0.0;
