@@ -83,7 +83,10 @@ struct NvtxRange {
     NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+// Records why a call failed and returns its code.  A runtime error is taken
+// off the thread with that, or the next launch would find it and report it again.
 static int fail(cor_ctx* ctx, int code, const char* fmt, ...) {
+    if (code == COR_ERR_CUDA || code == COR_ERR_NOMEM) cudaGetLastError();
     if (ctx) {
         va_list ap;
         va_start(ap, fmt);
@@ -717,6 +720,48 @@ extern "C" int cor_trace_steps(cor_ctx* ctx, const cor_batch_req* req, cor_batch
     return COR_OK;
 }
 
+// A field batch on the context's stream, in the context's own buffers (an
+// allocation and a free a call were 45 us).  The output buffer outlives the
+// call: every copy and launch is checked, since after one that failed it holds
+// an earlier call's fields.
+static int field_run(cor_ctx* ctx, const cor_model_set& models, const cor_model_params* params, int32_t n_params,
+                     const int32_t* param_index, const double* gsm_pos, int64_t n, double* geo_field) {
+    cudaStream_t s = ctx->stream;
+    int rc;
+    if ((rc = ensure(ctx, ctx->f_params, sizeof(DevParams) * (size_t)n_params)) != COR_OK) return rc;
+    if ((rc = ensure(ctx, ctx->f_pos, sizeof(double) * 3 * (size_t)n)) != COR_OK) return rc;
+    if ((rc = ensure(ctx, ctx->f_out, sizeof(double) * 3 * (size_t)n)) != COR_OK) return rc;
+    if (param_index && (rc = ensure(ctx, ctx->f_idx, sizeof(int32_t) * (size_t)n)) != COR_OK) return rc;
+    const DevParams* dp = (const DevParams*)ctx->f_params.p;
+    const double* dpos = (const double*)ctx->f_pos.p;
+    const int32_t* didx = param_index ? (const int32_t*)ctx->f_idx.p : nullptr;
+    double* dout = (double*)ctx->f_out.p;
+    DevParams* hp = (DevParams*)malloc(sizeof(DevParams) * (size_t)n_params);
+    if (!hp) return fail(ctx, COR_ERR_NOMEM, "host allocation");
+    prepare_params(params, n_params, hp);
+    // from pageable memory: the call returns when the source has been read
+    const cudaError_t e =
+        cudaMemcpyAsync(ctx->f_params.p, hp, sizeof(DevParams) * (size_t)n_params, cudaMemcpyHostToDevice, s);
+    free(hp);
+    CUDA_TRY(ctx, e);
+    CUDA_TRY(ctx, cudaMemcpyAsync(ctx->f_pos.p, gsm_pos, sizeof(double) * 3 * (size_t)n, cudaMemcpyHostToDevice, s));
+    if (param_index)
+        CUDA_TRY(ctx, cudaMemcpyAsync(ctx->f_idx.p, param_index, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, s));
+    CrustalTables crust;
+    if ((rc = crustal_tables(ctx, models, &crust)) != COR_OK) return rc;
+    const ModelOps* ops = find_ops(models);
+    if (team_takes_field(ops, models, (uint64_t)n, ctx->sms)) {
+        int slots = 1;
+        unsigned blocks = 1;
+        if ((rc = team_shape(ctx, ops, (uint64_t)n, &slots, &blocks)) != COR_OK) return rc;
+        CUDA_TRY(ctx, ops->launch_team_field(dp, n_params, didx, dpos, n, dout, slots, blocks, s));
+    } else {
+        CUDA_TRY(ctx, ops->launch_field(dp, n_params, didx, dpos, n, dout, crust, s));
+    }
+    CUDA_TRY(ctx, cudaMemcpyAsync(geo_field, dout, sizeof(double) * 3 * (size_t)n, cudaMemcpyDeviceToHost, s));
+    return COR_OK;
+}
+
 extern "C" int cor_field_batch(cor_ctx* ctx, cor_model_set models, const cor_model_params* params, int32_t n_params,
                                const int32_t* param_index, const double* gsm_pos, int64_t n, double* geo_field) {
     NvtxRange nvtx_range("cor_field_batch");
@@ -731,46 +776,11 @@ extern "C" int cor_field_batch(cor_ctx* ctx, cor_model_set models, const cor_mod
             return fail(ctx, COR_ERR_INVALID, "point %lld: param_index %d out of range", (long long)i, param_index[i]);
     if (n == 0) return COR_OK;
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    cudaStream_t s = ctx->stream;
-    // the context's own buffers: an allocation and a free a call were 45 us
-    int rc = COR_OK;
-    do {
-        if ((rc = ensure(ctx, ctx->f_params, sizeof(DevParams) * (size_t)n_params)) != COR_OK) break;
-        if ((rc = ensure(ctx, ctx->f_pos, sizeof(double) * 3 * (size_t)n)) != COR_OK) break;
-        if ((rc = ensure(ctx, ctx->f_out, sizeof(double) * 3 * (size_t)n)) != COR_OK) break;
-        if (param_index && (rc = ensure(ctx, ctx->f_idx, sizeof(int32_t) * (size_t)n)) != COR_OK) break;
-        void *dp = ctx->f_params.p, *dpos = ctx->f_pos.p, *dout = ctx->f_out.p;
-        void* didx = param_index ? ctx->f_idx.p : nullptr;
-        DevParams* hp = (DevParams*)malloc(sizeof(DevParams) * (size_t)n_params);
-        if (!hp) {
-            rc = fail(ctx, COR_ERR_NOMEM, "host allocation");
-            break;
-        }
-        prepare_params(params, n_params, hp);
-        // from pageable memory: the call returns when the source has been read
-        cudaMemcpyAsync(dp, hp, sizeof(DevParams) * (size_t)n_params, cudaMemcpyHostToDevice, s);
-        free(hp);
-        cudaMemcpyAsync(dpos, gsm_pos, sizeof(double) * 3 * (size_t)n, cudaMemcpyHostToDevice, s);
-        if (param_index) cudaMemcpyAsync(didx, param_index, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, s);
-        CrustalTables crust;
-        if ((rc = crustal_tables(ctx, models, &crust)) != COR_OK) break;
-        const ModelOps* ops = find_ops(models);
-        int slots = 1;
-        unsigned blocks = 1;
-        if (team_takes_field(ops, models, (uint64_t)n, ctx->sms)) {
-            if ((rc = team_shape(ctx, ops, (uint64_t)n, &slots, &blocks)) != COR_OK) break;
-            ops->launch_team_field((const DevParams*)dp, n_params, (const int32_t*)didx, (const double*)dpos, n,
-                                   (double*)dout, slots, blocks, s);
-        } else {
-            ops->launch_field((const DevParams*)dp, n_params, (const int32_t*)didx, (const double*)dpos, n,
-                              (double*)dout, crust, s);
-        }
-        cudaMemcpyAsync(geo_field, dout, sizeof(double) * 3 * (size_t)n, cudaMemcpyDeviceToHost, s);
-        cudaError_t e = cudaStreamSynchronize(s);
-        if (e == cudaSuccess) e = cudaGetLastError();
-        if (e != cudaSuccess) rc = fail(ctx, COR_ERR_CUDA, "field batch: %s", cudaGetErrorString(e));
-    } while (0);
-    return rc;
+    const int rc = field_run(ctx, models, params, n_params, param_index, gsm_pos, n, geo_field);
+    const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    if (rc != COR_OK) return rc;
+    CUDA_TRY(ctx, e);
+    return COR_OK;
 }
 
 // ---- FP64 peak probe -------------------------------------------------------

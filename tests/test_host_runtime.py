@@ -1,0 +1,106 @@
+"""The host side of libcortrace over a stand-in for the CUDA runtime
+(tests/host_runtime/fake_cudart.cpp), on the CPU: what it reports when a
+launch or a copy fails, how long it keeps what an asynchronous copy reads, and
+what calls of other threads can change.  Kernels do nothing here."""
+from __future__ import annotations
+
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+import build_lib
+import cortrace as ct
+
+SRC = os.path.join(ROOT, "tests", "host_runtime", "fake_cudart.cpp")
+ERR_NOMEM, ERR_CUDA = -2, -3
+TIME7 = [2020, 6, 21, 173, 12, 0, 0]
+PARMOD = [3.0, -40.0, 2.0, -5.0, 0.5, 0.4, 0.3, 0.5, 0.3, 0.6]
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    if shutil.which("g++") is None:
+        pytest.skip("no g++")
+    build_lib.build()
+    so = str(tmp_path_factory.mktemp("host_runtime") / "libcortrace_host.so")
+    objs = [os.path.join(build_lib.BUILD, s + ".o") for s in build_lib.CU_SOURCES + build_lib.LIB_C_SOURCES]
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build_lib.nvcc()))), "include")
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-g", "-fPIC", "-shared", "-pthread", f"-I{cuda}", SRC, *objs,
+                        "-o", so, "-Wl,-Bsymbolic", "-Wl,--wrap=free", "-lm", "-ldl"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+    was, ct._lib = ct._lib, None
+    lib = ct.load(so)
+    lib.fake_fail_launch.argtypes = [C.c_char_p]
+    lib.fake_fail_call.argtypes = [C.c_char_p, C.c_int]
+    lib.fake_limits_set.argtypes = [C.c_char_p]
+    lib.fake_launch.argtypes = [C.c_int, C.c_char_p, C.c_int, C.POINTER(C.c_uint), C.POINTER(C.c_uint),
+                                C.POINTER(C.c_uint64)]
+    yield lib
+    lib.fake_reset()
+    ct._lib = was
+
+
+@pytest.fixture()
+def host(fake):
+    fake.fake_reset()
+    yield fake
+    fake.fake_reset()
+
+
+def params(external=ct.EXTERNAL_NONE):
+    return ct.internal_setup("igrf14", TIME7, parmod=PARMOD if external else None)
+
+
+def points(n):
+    return np.tile(np.array([[3.0, 1.0, 2.0]]) * ct.DEF_RE, (n, 1))
+
+
+# a team call and one point to a lane, for every model set
+FIELD_CALLS = [(m, n) for m in [(1, 0, 0), (1, 1, 0), (0, 1, 0), (1, 2, 0), (0, 2, 0)] for n in (5, 40000)] + \
+    [((1, 1, 1), 5)]
+
+
+@pytest.mark.parametrize("models,n", FIELD_CALLS)
+def test_field_launch_that_fails_is_reported(host, models, n):
+    """cor_field_batch keeps its output buffer between calls: a launch that
+    fails must not hand out the fields of the call before."""
+    with ct.Context(0) as ctx:
+        m = ct.model_set(*models)
+        ctx.field_batch(points(n), params(1), m)
+        host.fake_fail_launch(b"field_kernel")
+        with pytest.raises(ct.CorError) as e:
+            ctx.field_batch(points(n), params(1), m)
+        assert e.value.code == ERR_CUDA
+        host.fake_fail_launch(b"")
+        ctx.field_batch(points(n), params(1), m)
+
+
+@pytest.mark.parametrize("nth", [1, 2, 3, 4])
+def test_field_copy_that_fails_is_reported(host, nth):
+    """Parameters, positions, parameter indices, fields."""
+    with ct.Context(0) as ctx:
+        idx = np.zeros(7, np.int32)
+        ctx.field_batch(points(7), params(), param_index=idx)
+        host.fake_fail_call(b"cudaMemcpyAsync", nth)
+        with pytest.raises(ct.CorError) as e:
+            ctx.field_batch(points(7), params(), param_index=idx)
+        assert e.value.code == ERR_CUDA
+
+
+def test_error_of_one_call_is_not_the_next_ones(host):
+    """A call that found no memory has reported it; the next one is itself again."""
+    jobs = ct.make_job(50.0, 15.0, rig=1.0, rk=5.0, dele=1.0)
+    with ct.Context(0) as ctx:
+        for call in (lambda: ctx.field_batch(points(7), params()), lambda: ctx.trace_batch(jobs, params()),
+                     lambda: ctx.upload_crustal(np.ones(6), np.ones(6), 3)):
+            host.fake_fail_call(b"cudaMalloc", 1)
+            with pytest.raises(ct.CorError) as e:
+                call()
+            assert e.value.code == ERR_NOMEM
+            ctx.field_batch(points(7), params(), ct.model_set(ct.INTERNAL_SH, ct.EXTERNAL_T96))
+            call()
