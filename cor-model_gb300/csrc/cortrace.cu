@@ -723,9 +723,11 @@ extern "C" int cor_trace_steps(cor_ctx* ctx, const cor_batch_req* req, cor_batch
 // A field batch on the context's stream, in the context's own buffers (an
 // allocation and a free a call were 45 us).  The output buffer outlives the
 // call: every copy and launch is checked, since after one that failed it holds
-// an earlier call's fields.
-static int field_run(cor_ctx* ctx, const cor_model_set& models, const cor_model_params* params, int32_t n_params,
-                     const int32_t* param_index, const double* gsm_pos, int64_t n, double* geo_field) {
+// an earlier call's fields.  On return, copies from and to all four host arrays
+// may be pending: a copy from pageable memory need not be staged where the GPU
+// reads it through the host's page tables, as GB300's does.
+static int field_queue(cor_ctx* ctx, const cor_model_set& models, const DevParams* params, int32_t n_params,
+                       const int32_t* param_index, const double* gsm_pos, int64_t n, double* geo_field) {
     cudaStream_t s = ctx->stream;
     int rc;
     if ((rc = ensure(ctx, ctx->f_params, sizeof(DevParams) * (size_t)n_params)) != COR_OK) return rc;
@@ -736,14 +738,7 @@ static int field_run(cor_ctx* ctx, const cor_model_set& models, const cor_model_
     const double* dpos = (const double*)ctx->f_pos.p;
     const int32_t* didx = param_index ? (const int32_t*)ctx->f_idx.p : nullptr;
     double* dout = (double*)ctx->f_out.p;
-    DevParams* hp = (DevParams*)malloc(sizeof(DevParams) * (size_t)n_params);
-    if (!hp) return fail(ctx, COR_ERR_NOMEM, "host allocation");
-    prepare_params(params, n_params, hp);
-    // from pageable memory: the call returns when the source has been read
-    const cudaError_t e =
-        cudaMemcpyAsync(ctx->f_params.p, hp, sizeof(DevParams) * (size_t)n_params, cudaMemcpyHostToDevice, s);
-    free(hp);
-    CUDA_TRY(ctx, e);
+    CUDA_TRY(ctx, cudaMemcpyAsync(ctx->f_params.p, params, sizeof(DevParams) * (size_t)n_params, cudaMemcpyHostToDevice, s));
     CUDA_TRY(ctx, cudaMemcpyAsync(ctx->f_pos.p, gsm_pos, sizeof(double) * 3 * (size_t)n, cudaMemcpyHostToDevice, s));
     if (param_index)
         CUDA_TRY(ctx, cudaMemcpyAsync(ctx->f_idx.p, param_index, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, s));
@@ -776,8 +771,13 @@ extern "C" int cor_field_batch(cor_ctx* ctx, cor_model_set models, const cor_mod
             return fail(ctx, COR_ERR_INVALID, "point %lld: param_index %d out of range", (long long)i, param_index[i]);
     if (n == 0) return COR_OK;
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    const int rc = field_run(ctx, models, params, n_params, param_index, gsm_pos, n, geo_field);
+    DevParams* hp = (DevParams*)malloc(sizeof(DevParams) * (size_t)n_params);
+    if (!hp) return fail(ctx, COR_ERR_NOMEM, "host allocation");
+    prepare_params(params, n_params, hp);
+    const int rc = field_queue(ctx, models, hp, n_params, param_index, gsm_pos, n, geo_field);
+    // also after a failure: copies may be pending from hp and the caller's arrays
     const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    free(hp);
     if (rc != COR_OK) return rc;
     CUDA_TRY(ctx, e);
     return COR_OK;

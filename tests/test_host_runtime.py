@@ -104,3 +104,27 @@ def test_error_of_one_call_is_not_the_next_ones(host):
             assert e.value.code == ERR_NOMEM
             ctx.field_batch(points(7), params(), ct.model_set(ct.INTERNAL_SH, ct.EXTERNAL_T96))
             call()
+
+
+@pytest.mark.parametrize("n,n_params", [(1, 1), (7, 3), (40000, 1)])
+def test_field_parameters_outlive_their_copy(host, n, n_params):
+    """The runtime may read a pageable source at any time before the stream is
+    waited for: nothing a queued copy reads is freed before."""
+    with ct.Context(0) as ctx:
+        for models in [(1, 0, 0), (1, 1, 0), (1, 2, 0), (1, 0, 1)]:
+            ctx.field_batch(points(n), np.repeat(params(1), n_params), ct.model_set(*models))
+            assert host.fake_freed_pending() == 0 and host.fake_pending() == 0
+
+
+@pytest.mark.parametrize("call", ["cudaMalloc", "cudaOccupancy", "cudaFuncSetAttribute", "cudaMemcpyAsync"])
+@pytest.mark.parametrize("nth", range(1, 5))
+@pytest.mark.parametrize("models", [(1, 0, 0), (1, 1, 0), (1, 0, 1)])
+def test_field_call_that_fails_leaves_no_copy_behind(host, call, nth, models):
+    """Whatever fails, no copy from or to the caller's arrays is pending afterwards."""
+    with ct.Context(0) as ctx:
+        host.fake_fail_call(call.encode(), nth)
+        try:
+            ctx.field_batch(points(7), params(1), ct.model_set(*models), param_index=np.zeros(7, np.int32))
+        except ct.CorError as e:
+            assert e.code in (ERR_CUDA, ERR_NOMEM)
+        assert host.fake_pending() == 0 and host.fake_freed_pending() == 0
