@@ -69,27 +69,30 @@
     }                                                                                                      \
     template <class MS, bool TEAM = MS::crustal == 0>                                                      \
     struct Team_##NAME {                                                                                   \
+        /* the functions' limit is the device's, not the context's: every call of every thread sets the  */\
+        /* same one, that of the most slots, whatever its own launch needs                               */\
+        static constexpr size_t kLimit = kTeamSlotsOf<MS> * sizeof(TeamSlot<MS>);                          \
+        template <class F>                                                                                 \
+        static cudaError_t limit(F* kernel) {                                                              \
+            return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLimit); \
+        }                                                                                                  \
         static cudaError_t occ(int* n_slots, int* n) {                                                     \
             *n_slots = kTeamSlotsOf<MS>;                                                                   \
-            const size_t smem = (size_t)*n_slots * sizeof(TeamSlot<MS>);                                   \
-            cudaError_t e = cudaFuncSetAttribute(team_trace_kernel<MS>,                                    \
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+            const cudaError_t e = limit(team_trace_kernel<MS>);                                            \
             if (e != cudaSuccess) return e;                                                                \
-            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, team_trace_kernel<MS>, kTeamThreads, smem); \
+            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, team_trace_kernel<MS>, kTeamThreads, kLimit);\
         }                                                                                                  \
         static cudaError_t run(const TraceArgs& a, int n_slots, unsigned blocks, cudaStream_t s) {         \
             const size_t smem = (size_t)n_slots * sizeof(TeamSlot<MS>);                                    \
-            cudaError_t e = cudaFuncSetAttribute(team_trace_kernel<MS>,                                    \
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+            const cudaError_t e = limit(team_trace_kernel<MS>);                                            \
             if (e != cudaSuccess) return e;                                                                \
             team_trace_kernel<MS><<<blocks, team_threads(n_slots), smem, s>>>(a, n_slots);                 \
             return cudaGetLastError();                                                                     \
         }                                                                                                  \
-        static cudaError_t field(const DevParams* p, int np, const int32_t* idx, const double* pos, int64_t n, \
+        static cudaError_t field(const DevParams* p, int np, const int32_t* idx, const double* pos, int64_t n,\
                                  double* out, int n_slots, unsigned blocks, cudaStream_t s) {              \
             const size_t smem = (size_t)n_slots * sizeof(TeamSlot<MS>);                                    \
-            cudaError_t e = cudaFuncSetAttribute(team_field_kernel<MS>,                                    \
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+            const cudaError_t e = limit(team_field_kernel<MS>);                                            \
             if (e != cudaSuccess) return e;                                                                \
             team_field_kernel<MS><<<blocks, team_threads(n_slots), smem, s>>>(p, np, idx, pos, n, out, n_slots);\
             return cudaGetLastError();                                                                     \

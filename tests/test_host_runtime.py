@@ -128,3 +128,37 @@ def test_field_call_that_fails_leaves_no_copy_behind(host, call, nth, models):
         except ct.CorError as e:
             assert e.code in (ERR_CUDA, ERR_NOMEM)
         assert host.fake_pending() == 0 and host.fake_freed_pending() == 0
+
+
+TEAM_SETS = [(1, 0, 0), (1, 1, 0), (0, 1, 0), (1, 2, 0), (0, 2, 0)]
+
+
+def scan(ctx, n, models):
+    jobs = ct.make_job(50.0, 15.0, rig=1.0, rk=1.0 + 0.01 * (n - 1), dele=0.01)
+    return ctx.trace_batch(jobs, params(1), ct.model_set(*models), step_limit=10)
+
+
+@pytest.mark.parametrize("models", TEAM_SETS)
+def test_calls_of_other_threads_do_not_change_a_launch(host, models):
+    """The limit of dynamic shared memory belongs to a function on the device,
+    and contexts of other threads make calls of other sizes: whatever they set
+    between this call's set-up and its launch must leave room for it.  Here the
+    other thread's call runs right after each setting, with the least shared
+    memory a call can take."""
+    with ct.Context(0) as a, ct.Context(0) as b:
+        m = ct.model_set(*models)
+        for mine in (lambda: a.field_batch(points(2000), params(1), m), lambda: scan(a, 2000, models)):
+            inside = []
+
+            def other(_name):
+                if not inside:
+                    inside.append(1)
+                    b.field_batch(points(1), params(1), m)
+                    scan(b, 1, models)
+                    inside.pop()
+            hook = C.CFUNCTYPE(None, C.c_char_p)(other)
+            host.fake_after_attribute(hook)
+            mine()
+            host.fake_after_attribute(None)
+    for f in (b"team_trace_kernel", b"team_field_kernel"):
+        assert host.fake_limits_set(f) == 1
