@@ -46,6 +46,7 @@
 
 #include "cor_trace.h"
 #include "cor_window.h"
+#include "mlp_schedule.h"
 
 namespace mlp {
 
@@ -69,10 +70,7 @@ __host__ __device__ constexpr size_t packed_at(int rows, int r, int k) {
 }
 
 // ---- the weight stream of rows_kernel ------------------------------------------
-// Products in order: layers 1 .. 5 forward, then back through W5^T, W4^T, W3^T, W2^T.
-constexpr int kFwdProducts = 5, kProducts = 9;
 __host__ __device__ constexpr int product_n(int p) { return p == 4 ? kOutPad : kH; }
-__host__ __device__ constexpr int product_blocks(int p) { return p == 0 || p == 5 ? 1 : 4; }
 __host__ __device__ constexpr size_t product_bytes(int p) { return (size_t)product_blocks(p) * block_bytes(product_n(p)); }
 __host__ __device__ constexpr size_t product_offset(int p) {
     size_t o = 0;
@@ -247,19 +245,15 @@ __device__ __forceinline__ uint32_t peer_addr(uint32_t a, int rank) {
     return r;
 }
 
-// The output of hidden product p (0 .. 3 forward, 5 .. 7 back) is exchange p or
-// p - 1, into A buffer exchange % 2; the two products before and after the
-// output layer read the single block instead.
-__device__ __forceinline__ int exchange_into(int p) { return p == 0 || p == 5 ? -1 : p < 5 ? p - 1 : p - 2; }
-__device__ __forceinline__ int exchange_out(int p) { return p < 4 ? p : p - 1; }
-
 // A cluster of four CTAs takes one tile of 128 rows: CTA r computes columns
 // 64 r .. 64 r + 63 of every hidden layer, which are K block r of the next
 // product's A, and copies them to its three peers' shared memory.  An epilogue
 // of 128 x 64 elements by 16 warps takes a quarter of what the whole width
 // does, and a weight block is a quarter of the size.  A has two buffers: a
 // peer that writes exchange x has read exchange x - 1 of this CTA, which it
-// sent after its products had read x - 2.
+// sent after its products had read x - 2.  There is one accumulator: a product
+// begins when this CTA's own blocks are complete, so its epilogue has read the
+// product before (waits_for; tests/test_network_order.py checks both).
 template <bool TRAIN>
 __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kRowsThreads, 1) rows_kernel(const RowsArgs g) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -333,7 +327,8 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kRowsThreads, 1
                 const uint8_t* a = x < 0 ? single : abuf + (x & 1) * kSplit * kABlock;
                 for (int kb = 0; kb < product_blocks(p) && ok; kb++, s++) {
                     const int k = s % kRing;
-                    if (x >= 0) ok = mbar_wait(&sh.kready[x & 1][kb], (uint32_t)((x >> 1) & 1));
+                    for (int b = 0; x >= 0 && b < kBlocks && ok; b++)
+                        if (waits_for(kSplit, rank, kb, b)) ok = mbar_wait(&sh.kready[x & 1][b], (uint32_t)((x >> 1) & 1));
                     ok = ok && mbar_wait(&sh.full[k], (uint32_t)((s / kRing) & 1));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
