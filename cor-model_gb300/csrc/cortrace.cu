@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "device_share.h"
 #include "model_ops.h"
 #include "reduce_kernels.cuh"
 #include "model_prep.h"
@@ -423,6 +424,7 @@ static int launch_trace(cor_ctx* ctx, const ModelOps* ops, TraceArgs a, cudaStre
 }
 
 static int launch_scan(cor_ctx* ctx, const TraceArgs& a, cor_model_set models, cor_site_result* sites, cudaStream_t s) {
+    const ShareHold hold(ctx->device);
     CUDA_TRY(ctx, cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), s));
     CUDA_TRY(ctx, cudaMemsetAsync(a.counters, 0, sizeof(cor_counters), s));
     unsigned long long checks = 0;
@@ -1349,12 +1351,18 @@ static int stream_error(cor_stream* s) {
     return COR_OK;
 }
 
+// The launch has ended, or is known to have.
+static void stream_ended(cor_stream* s) {
+    if (s->running) share_release(s->ctx->device);
+    s->running = false;
+}
+
 // Lets the running launch finish every published segment, then waits for it.
 static int stream_stop(cor_stream* s) {
     if (!s->running) return COR_OK;
     __atomic_store_n(&s->ctl_h->stop_at, s->published, __ATOMIC_RELEASE);
     const cudaError_t e = cudaStreamSynchronize(s->ks);
-    s->running = false;
+    stream_ended(s);
     if (e != cudaSuccess) return fail(s->ctx, COR_ERR_CUDA, "stream kernel: %s", cudaGetErrorString(e));
     return stream_error(s);
 }
@@ -1396,9 +1404,12 @@ static int stream_launch(cor_stream* s, unsigned long long stop_at) {
     s->args.first_seq = (unsigned long long)s->first_seq;
     s->args.first_index = s->first_index;
     CUDA_TRY(ctx, cudaEventRecord(s->ev0, s->ks));
-    CUDA_TRY(ctx, s->ops->launch_stream(s->args, s->blocks, s->ks));
-    CUDA_TRY(ctx, cudaEventRecord(s->ev1, s->ks));
+    share_hold(ctx->device, true);
+    const cudaError_t launched = s->ops->launch_stream(s->args, s->blocks, s->ks);
+    if (launched != cudaSuccess) share_release(ctx->device);
+    CUDA_TRY(ctx, launched);
     s->running = true;
+    CUDA_TRY(ctx, cudaEventRecord(s->ev1, s->ks));
     s->timed = true;
     return COR_OK;
 }
@@ -1652,7 +1663,7 @@ extern "C" int cor_stream_wait(cor_stream* s, int64_t ticket, int32_t timeout_ms
         if (s->running) {
             const cudaError_t e = cudaStreamQuery(s->ks);
             if (e == cudaSuccess) {
-                s->running = false;
+                stream_ended(s);
                 if (__atomic_load_n(&s->done_h[slot].seq1, __ATOMIC_ACQUIRE) == (unsigned long long)ticket + 1) break;
                 return fail(ctx, COR_ERR_CUDA, "stream kernel ended before segment %lld completed", (long long)ticket);
             }

@@ -3,9 +3,10 @@
 //
 // rows_kernel takes 128 rows of the batch through the whole network in one
 // launch, by a cluster of four CTAs with a quarter of every hidden layer's
-// columns each: the activations stay in the four shared memories from layer to
-// layer, and the weights stream through a ring of shared-memory stages (a 64-deep
-// K block of a CTA's columns, 8 KB, per cp.async.bulk).  For a training step it
+// columns each (or by one CTA, beside a scan stream: device_share.h): the
+// activations stay in the shared memories from layer to layer, and the weights
+// stream through a ring of shared-memory stages (a 64-deep K block of a CTA's
+// columns, 8 KB, per cp.async.bulk).  For a training step it
 // goes on through the loss and back through the layers (dZ of every layer), and
 // leaves what the weight gradients need in global memory.  grad_kernel then
 // takes the weight gradients (one CTA per 128 x 64 tile, K = the batch) and
@@ -46,6 +47,7 @@
 
 #include "cor_trace.h"
 #include "cor_window.h"
+#include "device_share.h"
 #include "mlp_schedule.h"
 
 namespace mlp {
@@ -202,12 +204,21 @@ __device__ __forceinline__ void put_transposed(uint8_t* dst, int R, int f0, int 
 }
 
 constexpr int kEpiWarps = 16, kRowsThreads = 32 * (kEpiWarps + 3);
-constexpr int kSplit = 4;                        // CTAs of a cluster: 64 columns of every hidden layer each
-constexpr int kNCols = kH / kSplit;
-constexpr int kRing = 8;
-constexpr uint32_t kStageBytes = block_bytes(kNCols);
 constexpr uint32_t kABlock = block_bytes(kBM);
-constexpr size_t kRowsSmem = 1024 + (2 * kSplit + 1) * kABlock + kRing * kStageBytes;
+
+// The two forms of rows_kernel: a tile of 128 rows by a cluster of four CTAs,
+// with 64 columns of every hidden layer each, or by one.
+template <int SPLIT>
+struct Form {
+    static constexpr int kOwn = kBlocks / SPLIT;   // K blocks of a hidden layer that a CTA computes
+    static constexpr int kCols = kH / SPLIT;
+    static constexpr int kSets = a_sets(SPLIT);
+    static constexpr int kRing = SPLIT == 1 ? 4 : 8;
+    static constexpr uint32_t kStage = block_bytes(kCols);
+    static constexpr size_t kSmem = 1024 + (kSets * kBlocks + 1) * kABlock + kRing * kStage;
+};
+constexpr int kSplit = 4;
+constexpr int kMaxRing = 8;
 
 struct RowsArgs {
     const float* x;          // n x 19
@@ -228,12 +239,12 @@ struct RowsArgs {
 };
 
 struct RowsShared {
-    uint64_t full[kRing], empty[kRing], acc;
+    uint64_t full[kMaxRing], empty[kMaxRing], acc;
     uint64_t local;              // the single K block that this CTA fills itself (input, dY)
-    // K block r of exchange x, in set x % 2: this CTA's own written, or a peer's
-    // copy landed.  Two sets, as two buffers: a peer sends x + 2 only after
-    // this CTA has taken x, but it may send x + 1 before.
-    uint64_t kready[2][kSplit];
+    // K block b of exchange x, in set x % kSets: this CTA's own written, or a
+    // peer's copy landed.  As many sets as buffers: a peer sends x + 2 only
+    // after this CTA has taken x, but it may send x + 1 before.
+    uint64_t kready[2][kBlocks];
     uint32_t tmem;
 };
 static_assert(sizeof(RowsShared) <= 1024, "rows_kernel header");
@@ -245,6 +256,15 @@ __device__ __forceinline__ uint32_t peer_addr(uint32_t a, int rank) {
     return r;
 }
 
+// A barrier of the CTAs of one tile.
+template <int SPLIT>
+__device__ __forceinline__ void tile_sync() {
+    if constexpr (SPLIT > 1)
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else
+        __syncthreads();
+}
+
 // A cluster of four CTAs takes one tile of 128 rows: CTA r computes columns
 // 64 r .. 64 r + 63 of every hidden layer, which are K block r of the next
 // product's A, and copies them to its three peers' shared memory.  An epilogue
@@ -254,18 +274,25 @@ __device__ __forceinline__ uint32_t peer_addr(uint32_t a, int rank) {
 // sent after its products had read x - 2.  There is one accumulator: a product
 // begins when this CTA's own blocks are complete, so its epilogue has read the
 // product before (waits_for; tests/test_network_order.py checks both).
-template <bool TRAIN>
-__global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kRowsThreads, 1) rows_kernel(const RowsArgs g) {
+//
+// SPLIT = 1: one CTA takes a tile alone, the same sums in the same order (the
+// bits are the same), on any one SM.  A cluster needs four whole SMs of one GPC
+// at a time, which a device that a scan stream holds does not have
+// (device_share.h).
+template <int SPLIT, bool TRAIN>
+__global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(kRowsThreads, 1) rows_kernel(const RowsArgs g) {
+    using F = Form<SPLIT>;
+    constexpr int kRing = F::kRing, kSets = F::kSets;
     extern __shared__ __align__(1024) uint8_t smem[];
     RowsShared& sh = *reinterpret_cast<RowsShared*>(smem);
-    uint8_t* abuf = smem + 1024;                          // 2 x 4 K blocks
-    uint8_t* single = abuf + 2 * kSplit * kABlock;        // 1 K block
+    uint8_t* abuf = smem + 1024;                          // kSets x 4 K blocks
+    uint8_t* single = abuf + kSets * kBlocks * kABlock;   // 1 K block
     uint8_t* ring = single + kABlock;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rank = blockIdx.x % kSplit, tile = blockIdx.x / kSplit;
+    const int rank = blockIdx.x % SPLIT, tile = blockIdx.x / SPLIT;
     const int m0 = tile * kBM;
     constexpr int kLast = TRAIN ? kProducts : kFwdProducts;
-    constexpr uint32_t kCols = kNCols;
+    constexpr uint32_t kCols = F::kCols;
 
     if (threadIdx.x == 0) {
         for (int k = 0; k < kRing; k++) {
@@ -274,8 +301,9 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kRowsThreads, 1
         }
         mbar_init(&sh.acc, 1);
         mbar_init(&sh.local, 32 * kEpiWarps);
-        for (int i = 0; i < 2; i++)
-            for (int r = 0; r < kSplit; r++) mbar_init(&sh.kready[i][r], r == rank ? 32 * kEpiWarps : 1);
+        for (int i = 0; i < kSets; i++)
+            for (int b = 0; b < kBlocks; b++)
+                mbar_init(&sh.kready[i][b], block_owner(SPLIT, b) == rank ? 32 * kEpiWarps : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -285,7 +313,7 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kRowsThreads, 1
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     // every CTA's barriers are set up before a peer's copy can arrive
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    tile_sync<SPLIT>();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = sh.tmem;
     bool ok = true;
@@ -294,15 +322,15 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kRowsThreads, 1
         if (lane == 0) {
             int s = 0;
             for (int p = 0; p < kLast && ok; p++) {
-                // the output layer's 16 rows go to every CTA; else this CTA's 64 rows
-                const uint32_t bytes = p == 4 ? block_bytes(kOutPad) : kStageBytes;
-                const uint8_t* src = g.weights + product_offset(p) + (p == 4 ? 0 : rank * kStageBytes);
+                // the output layer's 16 rows go to every CTA; else this CTA's rows
+                const uint32_t bytes = p == 4 ? block_bytes(kOutPad) : F::kStage;
+                const uint8_t* src = g.weights + product_offset(p) + (p == 4 ? 0 : rank * F::kStage);
                 for (int kb = 0; kb < product_blocks(p) && ok; kb++, s++) {
                     const int k = s % kRing;
                     if (s >= kRing) ok = mbar_wait(&sh.empty[k], (uint32_t)((s / kRing - 1) & 1));
                     if (!ok) break;
                     mbar_expect(&sh.full[k], bytes);
-                    bulk_load(ring + k * kStageBytes, src + (size_t)kb * block_bytes(product_n(p)), bytes, &sh.full[k]);
+                    bulk_load(ring + k * F::kStage, src + (size_t)kb * block_bytes(product_n(p)), bytes, &sh.full[k]);
                 }
             }
             if (!ok) {
@@ -316,23 +344,24 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kRowsThreads, 1
         if (lane == 0) {
             int s = 0;
             for (int p = 0; p < kLast && ok; p++) {
-                const uint32_t idesc = instr_desc(kBM, p == 4 ? kOutPad : kNCols);
+                const uint32_t idesc = instr_desc(kBM, p == 4 ? kOutPad : F::kCols);
                 const int x = exchange_into(p);
                 if (x < 0) {
                     ok = mbar_wait(&sh.local, (uint32_t)(p == 5));
                 } else {
-                    for (int r = 0; r < kSplit; r++)
-                        if (r != rank) mbar_expect(&sh.kready[x & 1][r], kABlock);
+                    for (int b = 0; b < kBlocks; b++)
+                        if (block_owner(SPLIT, b) != rank) mbar_expect(&sh.kready[x % kSets][b], kABlock);
                 }
-                const uint8_t* a = x < 0 ? single : abuf + (x & 1) * kSplit * kABlock;
+                const uint8_t* a = x < 0 ? single : abuf + (x % kSets) * kBlocks * kABlock;
                 for (int kb = 0; kb < product_blocks(p) && ok; kb++, s++) {
                     const int k = s % kRing;
                     for (int b = 0; x >= 0 && b < kBlocks && ok; b++)
-                        if (waits_for(kSplit, rank, kb, b)) ok = mbar_wait(&sh.kready[x & 1][b], (uint32_t)((x >> 1) & 1));
+                        if (waits_for(SPLIT, rank, kb, b))
+                            ok = mbar_wait(&sh.kready[x % kSets][b], (uint32_t)((x / kSets) & 1));
                     ok = ok && mbar_wait(&sh.full[k], (uint32_t)((s / kRing) & 1));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    mma_block(tmem, smem_u32(a + kb * kABlock), smem_u32(ring + k * kStageBytes), idesc, kb == 0);
+                    mma_block(tmem, smem_u32(a + kb * kABlock), smem_u32(ring + k * F::kStage), idesc, kb == 0);
                     commit_to(&sh.empty[k]);
                 }
                 if (ok) commit_to(&sh.acc);
@@ -340,20 +369,21 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kRowsThreads, 1
             if (!ok) atomicExch(g.err, 1);
         }
     } else if (warp == kEpiWarps + 2) {
-        if (lane == 0) {
+        if (SPLIT > 1 && lane == 0) {
+            static_assert(SPLIT == 1 || F::kOwn == 1, "one block to send");
             // this CTA's K block to its peers
             for (int p = 0; p + 1 < kLast && ok; p++) {
                 if (p == 4) continue;
                 const int x = exchange_out(p);
-                ok = mbar_wait(&sh.kready[x & 1][rank], (uint32_t)((x >> 1) & 1));
+                ok = mbar_wait(&sh.kready[x % kSets][rank], (uint32_t)((x / kSets) & 1));
                 if (!ok) break;
-                const uint32_t a = smem_u32(abuf + ((x & 1) * kSplit + rank) * kABlock);
-                for (int i = 1; i < kSplit; i++) {
-                    const int r = (rank + i) % kSplit;
+                const uint32_t a = smem_u32(abuf + ((x % kSets) * kBlocks + rank) * kABlock);
+                for (int i = 1; i < SPLIT; i++) {
+                    const int r = (rank + i) % SPLIT;
                     asm volatile(
                         "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                             peer_addr(a, r)),
-                        "r"(a), "r"(kABlock), "r"(peer_addr(smem_u32(&sh.kready[x & 1][rank]), r))
+                        "r"(a), "r"(kABlock), "r"(peer_addr(smem_u32(&sh.kready[x % kSets][rank]), r))
                         : "memory");
                 }
             }
@@ -365,7 +395,6 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kRowsThreads, 1
         const int gr = m0 + row;
         const bool valid = gr < g.n;
         const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16);
-        const int col0 = kNCols * rank + 16 * cg;   // this warp's 16 columns of a hidden layer
         float v[16];
         // the input: 16 columns per column group, in every CTA
 #pragma unroll
@@ -433,51 +462,57 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kRowsThreads, 1
                 }
                 continue;
             }
-            uint8_t* block = abuf + ((exchange_out(p) & 1) * kSplit + rank) * kABlock;
-            tmem_ld16(v, trow + 16 * cg);
-            if (p < COR_MLP_LAYERS) {
-                float z[16];
+            const int set = exchange_out(p) % kSets;
+#pragma unroll 1
+            for (int j = 0; j < F::kOwn; j++) {
+                const int kb = rank * F::kOwn + j;
+                const int col0 = 64 * kb + 16 * cg;   // this warp's 16 columns of the block
+                uint8_t* block = abuf + (set * kBlocks + kb) * kABlock;
+                tmem_ld16(v, trow + 64 * j + 16 * cg);
+                if (p < COR_MLP_LAYERS) {
+                    float z[16];
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    z[i] = v[i] + g.bias[p][col0 + i];
-                    v[i] = silu(z[i]);
-                }
-                put_row16(block, row, 16 * cg, v);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                mbar_arrive(&sh.kready[exchange_out(p) & 1][rank]);
-                if (TRAIN) {
-                    // what the way back needs, beside the next product
-#pragma unroll
-                    for (int i = 0; i < 16; i++) g.z[p][((size_t)tile * kH + col0 + i) * kBM + row] = z[i];
-                    __syncwarp();
-                    put_transposed(g.ht[p], kH, col0, m0, block + 2 * cg * 128, q, 16);
-                }
-            } else {
-                const int l = kProducts - 1 - p;   // dZ of layer l + 1
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    v[i] = v[i] * silu_grad(g.z[l][((size_t)tile * kH + col0 + i) * kBM + row]);
-                put_row16(block, row, 16 * cg, v);
-                if (p + 1 < kLast) {
+                    for (int i = 0; i < 16; i++) {
+                        z[i] = v[i] + g.bias[p][col0 + i];
+                        v[i] = silu(z[i]);
+                    }
+                    put_row16(block, row, 16 * cg, v);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    mbar_arrive(&sh.kready[exchange_out(p) & 1][rank]);
-                }
-                // column sums over the warp's 32 rows: lanes 2c and 2c+1 end with column c's
+                    mbar_arrive(&sh.kready[set][kb]);
+                    if (TRAIN) {
+                        // what the way back needs, beside the next product
 #pragma unroll
-                for (int o = 16, m = 8; m > 0; o >>= 1, m >>= 1) {
-                    const bool up = (lane & o) != 0;
-#pragma unroll
-                    for (int i = 0; i < m; i++) {
-                        const float give = up ? v[i] : v[i + m];
-                        v[i] = (up ? v[i + m] : v[i]) + __shfl_xor_sync(0xffffffffu, give, o);
+                        for (int i = 0; i < 16; i++) g.z[p][((size_t)tile * kH + col0 + i) * kBM + row] = z[i];
+                        __syncwarp();
+                        put_transposed(g.ht[p], kH, col0, m0, block + 2 * cg * 128, q, 16);
                     }
+                } else {
+                    const int l = kProducts - 1 - p;   // dZ of layer l + 1
+#pragma unroll
+                    for (int i = 0; i < 16; i++)
+                        v[i] = v[i] * silu_grad(g.z[l][((size_t)tile * kH + col0 + i) * kBM + row]);
+                    put_row16(block, row, 16 * cg, v);
+                    if (p + 1 < kLast) {
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        mbar_arrive(&sh.kready[set][kb]);
+                    }
+                    // column sums over the warp's 32 rows: lanes 2c and 2c+1 end with column c's
+#pragma unroll
+                    for (int o = 16, m = 8; m > 0; o >>= 1, m >>= 1) {
+                        const bool up = (lane & o) != 0;
+#pragma unroll
+                        for (int i = 0; i < m; i++) {
+                            const float give = up ? v[i] : v[i + m];
+                            v[i] = (up ? v[i + m] : v[i]) + __shfl_xor_sync(0xffffffffu, give, o);
+                        }
+                    }
+                    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+                    if ((lane & 1) == 0) atomicAdd(g.gb[l] + col0 + (lane >> 1), v[0]);
+                    __syncwarp();
+                    put_transposed(g.dzt[l], kH, col0, m0, block + 2 * cg * 128, q, 16);
                 }
-                v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-                if ((lane & 1) == 0) atomicAdd(g.gb[l] + col0 + (lane >> 1), v[0]);
-                __syncwarp();
-                put_transposed(g.dzt[l], kH, col0, m0, block + 2 * cg * 128, q, 16);
             }
         }
         if (!ok) atomicExch(g.err, 1);
@@ -486,7 +521,7 @@ __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kRowsThreads, 1
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
     // no CTA leaves while a peer's copy may still read or write shared memory
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    tile_sync<SPLIT>();
 }
 
 // ---- weight gradients and AdamW ---------------------------------------------------
@@ -788,6 +823,7 @@ struct cor_mlp {
     float* loss;
     float* z[COR_MLP_LAYERS];
     uint8_t *x0t, *ht[COR_MLP_LAYERS], *dzt[COR_MLP_LAYERS], *dyt;
+    bool can_cluster = false;   // the device (or this process's part of it) can place a cluster of rows_kernel
     int* err_h = nullptr;       // mapped: set by a wait that ran out
     int* err_d = nullptr;
 };
@@ -829,6 +865,41 @@ static RowsArgs rows_args(const cor_mlp* m, const float* x, int n) {
     g.loss = m->loss;
     g.err = m->err_d;
     return g;
+}
+
+template <int SPLIT, bool TRAIN>
+static bool set_rows_limit() {
+    return cudaFuncSetAttribute(rows_kernel<SPLIT, TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)Form<SPLIT>::kSmem) == cudaSuccess;
+}
+static bool set_rows_limits() {
+    return set_rows_limit<1, false>() && set_rows_limit<1, true>() && set_rows_limit<kSplit, false>() &&
+           set_rows_limit<kSplit, true>();
+}
+
+// Whether the current device, or this process's part of it, has room for a cluster at all.
+static bool cluster_fits() {
+    cudaLaunchAttribute dims = {};
+    dims.id = cudaLaunchAttributeClusterDimension;
+    dims.val.clusterDim = {kSplit, 1, 1};
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(kSplit);
+    c.blockDim = dim3(kRowsThreads);
+    c.dynamicSmemBytes = Form<kSplit>::kSmem;
+    c.attrs = &dims;
+    c.numAttrs = 1;
+    int n = 0;
+    const bool ok = cudaOccupancyMaxActiveClusters(&n, rows_kernel<kSplit, true>, &c) == cudaSuccess && n > 0;
+    cudaGetLastError();
+    return ok;
+}
+
+template <bool TRAIN>
+static cudaError_t launch_rows(const RowsArgs& g, bool clusters, cudaStream_t s) {
+    const int tiles = (g.n + kBM - 1) / kBM;
+    if (clusters) rows_kernel<kSplit, TRAIN><<<kSplit * tiles, kRowsThreads, Form<kSplit>::kSmem, s>>>(g);
+    else rows_kernel<1, TRAIN><<<tiles, kRowsThreads, Form<1>::kSmem, s>>>(g);
+    return cudaGetLastError();
 }
 
 static int check_err(cor_mlp* m) {
@@ -893,10 +964,7 @@ int cor_mlp_create(int device, int32_t max_batch, cor_mlp** out) {
     if (cudaMemset(m->block, 0, ogb + kGbBytes) != cudaSuccess ||
         cudaHostAlloc((void**)&m->err_h, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer((void**)&m->err_d, m->err_h, 0) != cudaSuccess ||
-        cudaFuncSetAttribute(rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem) !=
-            cudaSuccess ||
+        !set_rows_limits() ||
         cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGradSmem) != cudaSuccess ||
         cudaDeviceSynchronize() != cudaSuccess) {
         cudaFree(m->block);
@@ -904,6 +972,7 @@ int cor_mlp_create(int device, int32_t max_batch, cor_mlp** out) {
         delete m;
         return COR_ERR_CUDA;
     }
+    m->can_cluster = cluster_fits();
     *m->err_h = 0;
     *out = m;
     return COR_OK;
@@ -949,8 +1018,8 @@ int cor_mlp_forward(cor_mlp* m, const float* x_dev, int32_t n, float* y_dev, voi
     cudaStream_t s = (cudaStream_t)stream;
     RowsArgs g = rows_args(m, x_dev, n);
     g.y = y_dev;
-    rows_kernel<false><<<kSplit * ((n + kBM - 1) / kBM), kRowsThreads, kRowsSmem, s>>>(g);
-    MTRY(m, cudaGetLastError());
+    const cor::NetworkTurn turn(m->device, m->can_cluster);   // until the call has waited for its kernel
+    MTRY(m, launch_rows<false>(g, turn.clusters, s));
     MTRY(m, cudaStreamSynchronize(s));
     return check_err(m);
 }
@@ -966,8 +1035,8 @@ static int train(cor_mlp* m, const float* x, const float* t, int32_t n, float lr
     MTRY(m, cudaMemsetAsync(m->gb[0], 0, kGbBytes, s));
     RowsArgs g = rows_args(m, x, n);
     g.target = t;
-    rows_kernel<true><<<kSplit * tiles, kRowsThreads, kRowsSmem, s>>>(g);
-    MTRY(m, cudaGetLastError());
+    const cor::NetworkTurn turn(m->device, m->can_cluster);
+    MTRY(m, launch_rows<true>(g, turn.clusters, s));
     if (do_update) m->step++;
     GradArgs a = {};
     a.x0t = m->x0t;

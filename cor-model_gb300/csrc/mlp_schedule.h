@@ -6,7 +6,7 @@
 // A cluster of `split` CTAs takes a tile of rows.  A hidden layer's output is
 // exchanged as the four K blocks of the next product's A operand: each CTA
 // computes kBlocks / split of them and copies them to its peers.  A CTA has one
-// accumulator, and room for two exchanges (they alternate).
+// accumulator.
 #pragma once
 
 #ifdef __CUDACC__
@@ -24,10 +24,14 @@ constexpr int kFwdProducts = 5, kProducts = 9;
 MLP_HD constexpr int product_blocks(int p) { return p == 0 || p == 5 ? 1 : kBlocks; }
 
 // The output of hidden product p (0 .. 3 forward, 5 .. 7 back) is exchange p or
-// p - 1, into A buffer exchange % 2; the two products before and after the
+// p - 1, into A buffer exchange % a_sets; the two products before and after the
 // output layer read the single block that every CTA fills itself.
 MLP_HD constexpr int exchange_into(int p) { return p == 0 || p == 5 ? -1 : p < 5 ? p - 1 : p - 2; }
 MLP_HD constexpr int exchange_out(int p) { return p < 4 ? p : p - 1; }
+
+// Exchanges that a CTA has room for.  Peers write theirs while this CTA may
+// still read the one before; a CTA alone writes after its own product.
+MLP_HD constexpr int a_sets(int split) { return split == 1 ? 1 : 2; }
 
 MLP_HD constexpr int block_owner(int split, int block) { return block / (kBlocks / split); }
 

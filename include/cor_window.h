@@ -10,6 +10,11 @@
  * Weights and activations are BF16 on the tensor cores (tcgen05.mma, FP32
  * accumulation in tensor memory); FP32 master weights, AdamW.
  *
+ * The calls run on whatever SMs are free.  On a free device four SMs share a
+ * tile of 128 samples; while a scan stream is launched in this process, or a
+ * batch scan runs, one SM takes a tile alone (the same sums, the same bits), so
+ * that one reserved SM (cor_stream_config.reserve_sms) is enough to finish.
+ *
  * Parameters travel as one FP32 array in this order: W1[256][19], b1[256],
  * W2[256][256], b2[256], W3[256][256], b3[256], W4[256][256], b4[256],
  * W5[2][256], b5[2]  (W[out][in], y = W x + b).

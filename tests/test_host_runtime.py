@@ -162,3 +162,128 @@ def test_calls_of_other_threads_do_not_change_a_launch(host, models):
             host.fake_after_attribute(None)
     for f in (b"team_trace_kernel", b"team_field_kernel"):
         assert host.fake_limits_set(f) == 1
+
+
+class Network:
+    """A window network over the stand-in runtime; rows: the forms its calls launched."""
+
+    def __init__(self, host, max_batch=512):
+        import window
+        self.lib, self.host = window._bind(host), host
+        self.h = C.c_void_p()
+        assert self.lib.cor_mlp_create(0, max_batch, C.byref(self.h)) == 0
+        self.x = np.zeros((max_batch, window.N_IN), np.float32)
+        self.y = np.zeros((max_batch, window.N_OUT), np.float32)
+        self.out = np.zeros(window.N_PARAMS + 1, np.float32)
+
+    def forward(self, n=300):
+        return self._form(self.lib.cor_mlp_forward(self.h, self.x.ctypes.data, n, self.y.ctypes.data, None), n)
+
+    def train(self, n=300):
+        return self._form(self.lib.cor_mlp_train_step(self.h, self.x.ctypes.data, self.y.ctypes.data, n, 1e-3, 0.0,
+                                                      self.out.ctypes.data, None, None), n)
+
+    def _form(self, rc, n):
+        assert rc == 0
+        name, grid = [(k, g) for k, g in launched(self.host) if "rows_kernel" in k][-1]
+        split = 4 if "ILi4E" in name else 1
+        assert grid == split * ((n + 127) // 128)
+        return split
+
+    def close(self):
+        self.lib.cor_mlp_destroy(self.h)
+
+
+def launched(host):
+    name, g, b, m = C.create_string_buffer(512), C.c_uint(), C.c_uint(), C.c_uint64()
+    out = []
+    for i in range(host.fake_launch_count()):
+        host.fake_launch(i, name, 512, C.byref(g), C.byref(b), C.byref(m))
+        out.append((name.value.decode(), g.value))
+    return out
+
+
+def small_stream(ctx):
+    return ct.Stream(ctx, ct.model_set(), slots=2, max_jobs=4, max_trajectories=64, max_params=1, fixed_params=1,
+                     pool_params=8, reserve_sms=2)
+
+
+@pytest.fixture()
+def net(host):
+    n = Network(host)
+    yield n
+    n.close()
+
+
+JOB = dict(rig=1.0, rk=5.0, dele=1.0)
+
+
+def test_network_beside_a_stream_needs_no_cluster(host, net):
+    """A scan stream leaves a network reserve_sms SMs (include/cor_trace.h): too
+    few to place clusters of four CTAs until it is drained."""
+    with ct.Context(0) as ctx, small_stream(ctx) as st:
+        assert (net.forward(), net.train()) == (4, 4)
+        for _ in range(2):
+            st.submit(ct.make_job(50.0, 15.0, **JOB), params())
+            assert (net.forward(), net.train()) == (1, 1)
+            st.drain()
+            assert (net.forward(), net.train()) == (4, 4)
+        host.fake_fail_launch(b"stream_kernel")
+        with pytest.raises(ct.CorError):
+            st.submit(ct.make_job(50.0, 15.0, **JOB), params())
+        assert net.forward() == 4
+        host.fake_fail_launch(b"")
+
+
+def test_network_beside_a_batch_scan_needs_no_cluster(host, net):
+    """Nor does it wait for four SMs at a time behind the blocks of another thread's scan."""
+    forms = []
+    busy = []
+
+    def waiting():
+        if not busy:
+            busy.append(1)
+            forms.append(net.forward())
+            busy.pop()
+    hook = C.CFUNCTYPE(None)(waiting)
+    with ct.Context(0) as ctx:
+        host.fake_during_wait(hook)
+        ctx.trace_batch(ct.make_job(50.0, 15.0, **JOB), params())
+        host.fake_during_wait(None)
+    assert 1 in forms and net.forward() == 4
+
+
+@pytest.mark.parametrize("depends", [False, True])
+def test_stream_launch_waits_for_clusters(host, net, depends):
+    """A stream that starts in another thread while a network call runs in
+    clusters lets them finish first; but not for ever, in case the network call
+    waits for what the stream is to do."""
+    import threading
+    seen, started, threads = [], threading.Event(), []
+    with ct.Context(0) as ctx, small_stream(ctx) as st:
+        def start():
+            st.submit(ct.make_job(50.0, 15.0, **JOB), params())
+            started.set()
+
+        def waiting():
+            if threads:
+                return
+            threads.append(threading.Thread(target=start))
+            threads[0].start()
+            started.wait(20.0 if depends else 0.3)
+            seen.append(any("stream_kernel" in k for k, _ in launched(host)))
+        hook = C.CFUNCTYPE(None)(waiting)
+        host.fake_during_wait(hook)
+        net.forward()
+        threads[0].join()
+        host.fake_during_wait(None)
+        assert seen == [depends] and started.is_set()
+        assert net.forward() == 1
+
+
+def test_network_where_no_cluster_fits(host):
+    """A part of a GPU with fewer than four SMs."""
+    host.fake_fail_call(b"cudaOccupancyMaxActiveClusters", 1)
+    net = Network(host)
+    assert (net.forward(), net.train()) == (1, 1)
+    net.close()

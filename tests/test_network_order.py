@@ -24,7 +24,7 @@ def schedule(tmp_path_factory):
     src = os.path.join(ROOT, "tests", "network_order", "print_schedule.cpp")
     r = subprocess.run(["g++", "-std=c++17", src, "-o", exe], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-2000:]
-    s = {"product": [], "owner": {}, "waits": {}}
+    s = {"product": [], "owner": {}, "waits": {}, "sets": {}}
     for ln in subprocess.run([exe], capture_output=True, text=True, check=True).stdout.splitlines():
         k, *v = ln.split()
         v = [int(x) for x in v]
@@ -32,6 +32,8 @@ def schedule(tmp_path_factory):
             s["fwd"], s["all"] = v
         elif k == "product":
             s["product"].append(tuple(v))
+        elif k == "sets":
+            s["sets"][v[0]] = v[1]
         elif k == "owner":
             s["owner"][v[0], v[1]] = v[2]
         else:
@@ -161,13 +163,10 @@ def conflicts(s, split, train, waits, sets):
     return bad
 
 
-FORMS = [(4, 2)]   # CTAs of a cluster, exchanges there is room for
-
-
-@pytest.mark.parametrize("split,sets", FORMS)
+@pytest.mark.parametrize("split", [1, 4])   # CTAs of a cluster
 @pytest.mark.parametrize("train", [False, True])
-def test_every_read_comes_before_the_next_write(schedule, split, sets, train):
-    assert conflicts(schedule, split, train, lambda c, kb: schedule["waits"][split, c, kb], sets) == []
+def test_every_read_comes_before_the_next_write(schedule, split, train):
+    assert conflicts(schedule, split, train, lambda c, kb: schedule["waits"][split, c, kb], schedule["sets"][split]) == []
 
 
 @pytest.mark.parametrize("train", [False, True])
@@ -179,3 +178,5 @@ def test_the_model_finds_a_missing_wait(schedule, train):
     assert {a[1] for a, _ in bad if a[0] == "read"} == {1, 2, 3}
     bad = conflicts(schedule, 4, train, lambda c, kb: schedule["waits"][4, c, kb], 1)
     assert any(a[0] == "done" and b[0] == "send" for a, b in bad)
+    # a CTA alone, too, waits for all of its blocks before the first product
+    assert conflicts(schedule, 1, train, lambda c, kb: [kb], 1)
