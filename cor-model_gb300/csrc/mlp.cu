@@ -586,6 +586,22 @@ __device__ __forceinline__ float adamw(const GradArgs& g, int i, float gr, float
     return w;
 }
 
+// Whether `ok` holds for all 256 threads of grad_kernel's epilogue.  Each warp's
+// wait has a limit of its own: what one of them found is not what the others
+// did, and the barriers below count on all of them.
+__device__ __forceinline__ bool epilogue_agrees(bool ok) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.and.pred q, 1, 256, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)ok)
+        : "memory");
+    return r != 0;
+}
+
 // One tile of a weight gradient (blocks 0 .. kGradTiles - 1), or the biases (the last block).
 __global__ void __launch_bounds__(kGradThreads, 1) grad_kernel(const GradArgs g) {
     if (blockIdx.x == kGradTiles) {
@@ -684,8 +700,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grad_kernel(const GradArgs g)
             else atomicExch(g.err, 1);
         }
     } else {
-        ok = mbar_wait(&accb, 0);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = epilogue_agrees(mbar_wait(&accb, 0));
         if (!ok) {
             atomicExch(g.err, 1);
         } else {

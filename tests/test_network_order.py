@@ -180,3 +180,20 @@ def test_the_model_finds_a_missing_wait(schedule, train):
     assert any(a[0] == "done" and b[0] == "send" for a, b in bad)
     # a CTA alone, too, waits for all of its blocks before the first product
     assert conflicts(schedule, 1, train, lambda c, kb: [kb], 1)
+
+
+def test_weight_gradient_epilogue_decides_as_one():
+    """grad_kernel's epilogue warps wait with a limit each and meet at a barrier
+    of all 256 threads: whether to go on has to be one decision, taken by a
+    barrier of the same threads, or warps whose wait ran out would leave the
+    others at theirs."""
+    with open(os.path.join(ROOT, "cor-model_gb300", "csrc", "mlp.cu")) as f:
+        src = f.read()
+    kernel = src[src.index("grad_kernel(const GradArgs g) {"):src.index("// Every weight into its BF16 copies")]
+    waits = kernel.index("mbar_wait(&accb")
+    assert 0 <= kernel.rindex("epilogue_agrees(", 0, waits + 1) < waits < kernel.index("bar.sync 1")
+    helper = src[src.index("bool epilogue_agrees"):src.index("// One tile of a weight gradient")]
+    assert "bar.red.and.pred q, 1, 256, p" in helper and "kGradThreads = 32 * 10" in src
+    # the row kernel's warps share no barrier between their waits
+    rows = src[src.index("rows_kernel(const RowsArgs g) {"):src.index("// ---- weight gradients and AdamW")]
+    assert "bar.sync" not in rows and "bar.red" not in rows
