@@ -23,9 +23,9 @@
 //
 // Warps 0-15 are rows_kernel's epilogue (warp w owns rows 32 (w % 4) .. and
 // columns 16 (w / 4) .. of the accumulator), warp 16 feeds the ring, warp 17
-// issues the MMAs, warp 18 sends the CTA's columns to its peers.  Waits are bounded (about 2 s of SM clock); a wait that runs out sets
-// the error word, and every role leaves its loop, waits for its copies and
-// frees the TMEM.
+// issues the MMAs, warp 18 sends the CTA's columns to its peers.  Waits are
+// bounded (about 2 s of SM clock); a wait that runs out sets the error word, every
+// role leaves its loop, and the tile waits out what it issued and frees the TMEM.
 //
 // Measured: 2,664 rows forward 405 -> 43 us a call (kernel 22 us); a training
 // step of 512 rows 1,150 -> 103 us (rows_kernel 49, grad_kernel 16 us).  One
@@ -110,6 +110,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
         if (ok) return true;
         if (clock64() - t0 > kWaitCycles) return false;
     }
+}
+
+// After a wait that ran out: copies and products that were issued and that
+// nobody waits for any more end within microseconds.
+constexpr long long kSettleCycles = 20000000ll;   // about 10 ms
+__device__ __forceinline__ void settle() {
+    const long long t0 = clock64();
+    while (clock64() - t0 < kSettleCycles) {}
 }
 
 __device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
@@ -246,6 +254,7 @@ struct RowsShared {
     // after this CTA has taken x, but it may send x + 1 before.
     uint64_t kready[2][kBlocks];
     uint32_t tmem;
+    uint32_t failed;             // a CTA of the tile gave up
 };
 static_assert(sizeof(RowsShared) <= 1024, "rows_kernel header");
 
@@ -301,6 +310,7 @@ __global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(kRowsThreads, 1)
         }
         mbar_init(&sh.acc, 1);
         mbar_init(&sh.local, 32 * kEpiWarps);
+        sh.failed = 0;
         for (int i = 0; i < kSets; i++)
             for (int b = 0; b < kBlocks; b++)
                 mbar_init(&sh.kready[i][b], block_owner(SPLIT, b) == rank ? 32 * kEpiWarps : 1);
@@ -518,10 +528,18 @@ __global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(kRowsThreads, 1)
         if (!ok) atomicExch(g.err, 1);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
-    // no CTA leaves while a peer's copy may still read or write shared memory
+    const int failed = __syncthreads_or(!ok);
+    if (failed && threadIdx.x < SPLIT)
+        asm volatile("st.shared::cluster.u32 [%0], 1;" ::"r"(peer_addr(smem_u32(&sh.failed), threadIdx.x)) : "memory");
+    __syncwarp();
+    // no CTA leaves while a peer's copy may still read or write shared memory:
+    // where all went well, every copy was waited for; else they are waited out
     tile_sync<SPLIT>();
+    if (*(volatile uint32_t*)&sh.failed) {
+        settle();
+        tile_sync<SPLIT>();
+    }
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
 }
 
 // ---- weight gradients and AdamW ---------------------------------------------------
@@ -805,7 +823,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) grad_kernel(const GradArgs g)
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    if (__syncthreads_or(!ok)) settle();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
 }
 

@@ -197,3 +197,21 @@ def test_weight_gradient_epilogue_decides_as_one():
     # the row kernel's warps share no barrier between their waits
     rows = src[src.index("rows_kernel(const RowsArgs g) {"):src.index("// ---- weight gradients and AdamW")]
     assert "bar.sync" not in rows and "bar.red" not in rows
+
+
+def test_a_tile_that_gave_up_waits_out_what_it_issued():
+    """Where a wait ran out, copies to and from the peers and products into the
+    accumulator may be in flight that nobody waits for any more: every CTA of the
+    tile hears of it before it leaves, lets them end, and frees its tensor
+    memory after that."""
+    with open(os.path.join(ROOT, "cor-model_gb300", "csrc", "mlp.cu")) as f:
+        src = f.read()
+    rows = src[src.index("rows_kernel(const RowsArgs g) {"):src.index("// ---- weight gradients and AdamW")]
+    steps = ["sh.failed = 0;", "tile_sync<SPLIT>();", "__syncthreads_or(!ok)", "st.shared::cluster.u32", "tile_sync<SPLIT>();",
+             "sh.failed)", "settle();", "tile_sync<SPLIT>();", "tcgen05.dealloc"]
+    at = 0
+    for k in steps:
+        at = rows.index(k, at) + len(k)
+    assert "tile_sync" not in rows[at:]
+    grad = src[src.index("grad_kernel(const GradArgs g) {"):src.index("// Every weight into its BF16 copies")]
+    assert grad.index("__syncthreads_or(!ok)") < grad.index("settle();") < grad.index("tcgen05.dealloc")
