@@ -253,14 +253,21 @@ __device__ __forceinline__ int lane_advance(Lane& L, const TraceArgs& a) {
     const double zn = L.job->zn;
     const int nk1 = L.job->nk1;
     // every trial of the step divides by it (with an external model, whose
-    // kernels are short of registers, its reciprocal costs what it gives)
+    // kernels are short of registers, its reciprocal costs what it gives).  The
+    // reciprocal stands for the division where neither of the two is at the end
+    // of the doubles' range -- no field, or one out of range -- and the mass is
+    // finite
     const double tb = fabs(zn) * kQ * L.b, rtb = PLAIN ? 1. / tb : 0.;
+    const bool in_range = PLAIN && (unsigned)((to_bits(tb) >> 52) - 0x100) < 0x600u;
     for (;;) {
         L.step++;
         const double vc = DIVC(L.v);
-        if (vc > 1.) return COR_TRAJ_SUPERLUM;  // :48-54
+        const bool by_reciprocal = in_range && vc < 1.;
+        if (!by_reciprocal && vc > 1.) return COR_TRAJ_SUPERLUM;  // :48-54
         const double hm = a.mass / sqrt(1. - vc * vc);
-        const double t = PLAIN ? div_r(2. * kPi * hm, tb, rtb) : (2. * kPi * hm) / tb;
+        double t;
+        if (by_reciprocal) t = div_r(2. * kPi * hm, tb, rtb);
+        else t = (2. * kPi * hm) / tb;
         const double h = t / L.nk0;
         const double d = (1.E-09 * zn * kQ) / hm;
         const double vprev = L.v;
