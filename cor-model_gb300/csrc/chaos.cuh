@@ -39,10 +39,12 @@ constexpr double kChaosReKm = 6371.2;              // lib/chaos/chaos.h:6
 constexpr double kChaos2Pi = 6.283185307179586;    // lib/chaos/chaos.h:7
 constexpr double kChaosPi = 3.141592653589793;     // lib/chaos/chaos.h:8
 
-// Device tables of the crustal model.  g, h, k1, k2 are packed lower
-// triangles (index n(n+1)/2 + m); kd holds k per degree.  n_first is the
-// first degree with a non-zero coefficient: lower degrees add exactly +0 to
-// sums that are +0, so their terms are skipped (their rows are still built).
+// Tables of the crustal model, as crustal_block (model_prep.h) lays them out.
+// The kernels read kd, k per degree, and behind it the terms by order; g, h, k1
+// and k2, packed lower triangles (index n(n+1)/2 + m) that the terms are built
+// from, stay on the host (null on the device).  n_first is the first degree with
+// a non-zero coefficient: lower degrees add exactly +0 to sums that are +0, so
+// their terms are skipped (their rows are still built).
 // The kernels of sets with a crustal model choose the internal and external
 // models at run time (the crustal sum dwarfs the dispatch), from `internal`
 // and `external` (COR_INTERNAL_*, COR_EXTERNAL_*).

@@ -57,7 +57,7 @@ struct cor_ctx {
     double gen_ms[1024];                  // host wall time of each generation
     std::chrono::steady_clock::time_point gen_t0;
     cor_counters* counters = nullptr;
-    double* crust = nullptr;              // crustal tables: g, h, k1, k2 (packed), kd
+    double* crust = nullptr;              // crustal tables (crustal_block from kd on)
     int crust_nmax = 0;
     int crust_n_first = 0;
     int rig_major = 1;                    // queue order for uniform grids (cor_ctx_set_queue_order)
@@ -460,11 +460,13 @@ static int launch_scan(cor_ctx* ctx, const TraceArgs& a, cor_model_set models, c
 }
 
 // ---- crustal model tables --------------------------------------------------
-// One device block, built on the host by crustal_block (model_prep.h).
+// One device block: what the kernels read of the block that crustal_block
+// (model_prep.h) builds, kd and the terms by order.
 static int upload_crustal(cor_ctx* ctx, const double* g, const double* h, int32_t nmax) {
     if (nmax < 2 || nmax > kChaosMaxN)
         return fail(ctx, COR_ERR_RANGE, "crustal table nmax %d outside [2, %d]", nmax, kChaosMaxN);
     const size_t total = crustal_block_size(nmax);
+    const size_t first = 4 * ((size_t)nmax * (size_t)(nmax + 1) / 2), on_device = total - first;
     double* host = (double*)calloc(total, sizeof(double));
     if (!host) return fail(ctx, COR_ERR_NOMEM, "host allocation");
     const int n_first = crustal_block(g, h, nmax, host);
@@ -472,9 +474,9 @@ static int upload_crustal(cor_ctx* ctx, const double* g, const double* h, int32_
     double* dev = nullptr;
     do {
         cudaError_t e = cudaSetDevice(ctx->device);
-        if (e == cudaSuccess) e = cudaMalloc(&dev, sizeof(double) * total);
+        if (e == cudaSuccess) e = cudaMalloc(&dev, sizeof(double) * on_device);
         if (e != cudaSuccess) { rc = fail(ctx, COR_ERR_NOMEM, "crustal table: %s", cudaGetErrorString(e)); break; }
-        e = cudaMemcpyAsync(dev, host, sizeof(double) * total, cudaMemcpyHostToDevice, ctx->stream);
+        e = cudaMemcpyAsync(dev, host + first, sizeof(double) * on_device, cudaMemcpyHostToDevice, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) { rc = fail(ctx, COR_ERR_CUDA, "crustal table: %s", cudaGetErrorString(e)); break; }
         if (ctx->crust) cudaFree(ctx->crust);
@@ -497,12 +499,7 @@ static int crustal_tables(cor_ctx* ctx, const cor_model_set& m, CrustalTables* t
         const int rc = upload_crustal(ctx, cor_chaos716.g, cor_chaos716.h, cor_chaos716.nmax);
         if (rc != COR_OK) return rc;
     }
-    const size_t nt = (size_t)ctx->crust_nmax * (size_t)(ctx->crust_nmax + 1) / 2;
-    t->g = ctx->crust;
-    t->h = ctx->crust + nt;
-    t->k1 = ctx->crust + 2 * nt;
-    t->k2 = ctx->crust + 3 * nt;
-    t->kd = ctx->crust + 4 * nt;
+    t->kd = ctx->crust;
     t->nmax = ctx->crust_nmax;
     t->n_first = ctx->crust_n_first;
     t->internal = m.internal_model;

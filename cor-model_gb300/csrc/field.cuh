@@ -104,9 +104,9 @@ __device__ __forceinline__ Vec3 calculate_field(const bool want, const Vec3 gsm_
 // the radius in whole R_E (the internal field's degree and T96/TS05's inner
 // structures change with it) and |z|/r in twelfths (latitude bands).  In single
 // precision, whose pipe is idle here: in FP64 it took 1-2 % of a step (66,000
-// streamed T96 trajectories 425 ms with that, 417 with this; 91,200 IGRF-14
-// ones 437 and 435).  Region-1's bases as a further part of the key changed
-// nothing (419, 423).
+// streamed T96 trajectories, three times in turn: 426, 427 and 437 ms with that,
+// 422, 419 and 432 with this; 91,200 IGRF-14 ones 0.5 % less, within their
+// spread).  Region-1's bases as a further part of the key changed nothing.
 template <class MS>
 __device__ __forceinline__ unsigned field_band(const Vec3 gsm_pos, const DevParams* __restrict__ dp) {
     constexpr double kInvRe = 1.0 / kRe;

@@ -235,11 +235,10 @@ static void prepare_params(const cor_model_params* in, int32_t n, DevParams* out
 // The crustal model's tables, as one block: g, h, k1, k2 (packed lower
 // triangles of nmax(nmax+1)/2 entries each), then kd (nmax entries).  k1, k2
 // and kd are the recursion factors of lib/chaos/chaos.c:163-180, computed with
-// its expressions.  Then, for the device, the same by order (chaos_columns):
-// per term k1, k2, g, h, g m, h m (the products the sums start with), column
-// by column, and -(n + 1) per degree.  `host` holds crustal_block_size(nmax)
-// zeroed doubles.  Returns the first degree with a non-zero coefficient (nmax
-// if none).
+// its expressions.  Then, for chaos_geo_warp, the same by order: per term k1,
+// k2, g, h, g m, h m (the products the sums start with), column by column, and
+// -(n + 1) per degree.  `host` holds crustal_block_size(nmax) zeroed doubles.
+// Returns the first degree with a non-zero coefficient (nmax if none).
 static size_t crustal_block_size(int32_t nmax) {
     const size_t nt = (size_t)nmax * (size_t)(nmax + 1) / 2;
     return 4 * nt + (size_t)((nmax + 1) & ~1) + 6 * nt + (size_t)nmax;
