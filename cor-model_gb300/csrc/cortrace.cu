@@ -346,13 +346,18 @@ static bool use_halves(const ModelOps* ops, uint64_t live, uint64_t cap_blocks) 
 
 // Slots per block and blocks of a team launch: as many blocks as are resident
 // before a block takes a second slot (a lone trajectory's step is the
-// shortest), at most the set's kTeamSlotsOf.
+// shortest), at most the set's kTeamSlotsOf.  Beside a scan stream, full blocks:
+// they take turns on its reserved SMs.  ms for trajectories of 100 steps on two
+// of them, by one lane each / one to a block / full blocks: IGRF-14, 20
+// trajectories 12.2 / 18.1 / 4.2, 100 24 / 90 / 10, 400 84 / 182 / 36, 2,000 275 /
+// 225 / 123; T96, 100 75 / 170 / 30, 2,000 844 / 447 / 392; TS05, 100 189 / 607 /
+// 49, 2,000 2,092 / 884 / 654.
 static int team_shape(cor_ctx* ctx, const ModelOps* ops, uint64_t live, int* slots, unsigned* blocks) {
     int per_sm = 0, most = 1;
     CUDA_TRY(ctx, ops->team_occupancy(&most, &per_sm));
     if (per_sm < 1) per_sm = 1;
     const uint64_t cap = (uint64_t)per_sm * (uint64_t)ctx->sms;
-    uint64_t n = (live + cap - 1) / cap;
+    uint64_t n = share_has_stream(ctx->device) ? live : (live + cap - 1) / cap;
     if (n > (uint64_t)most) n = most;
     const uint64_t b = (live + n - 1) / n;
     *slots = (int)n;
@@ -1350,7 +1355,7 @@ static int stream_error(cor_stream* s) {
 
 // The launch has ended, or is known to have.
 static void stream_ended(cor_stream* s) {
-    if (s->running) share_release(s->ctx->device);
+    if (s->running) share_stream_end(s->ctx->device);
     s->running = false;
 }
 
@@ -1401,9 +1406,9 @@ static int stream_launch(cor_stream* s, unsigned long long stop_at) {
     s->args.first_seq = (unsigned long long)s->first_seq;
     s->args.first_index = s->first_index;
     CUDA_TRY(ctx, cudaEventRecord(s->ev0, s->ks));
-    share_hold(ctx->device, true);
+    share_stream_begin(ctx->device);
     const cudaError_t launched = s->ops->launch_stream(s->args, s->blocks, s->ks);
-    if (launched != cudaSuccess) share_release(ctx->device);
+    if (launched != cudaSuccess) share_stream_end(ctx->device);
     CUDA_TRY(ctx, launched);
     s->running = true;
     CUDA_TRY(ctx, cudaEventRecord(s->ev1, s->ks));

@@ -11,6 +11,10 @@
 // launch its kernel waits for the network calls that run in the other form.
 // That wait is bounded: a network call may itself be queued behind work of the
 // caller's that only ends after the stream has been fed.
+//
+// Team launches (team.cuh) ask for streams too: few trajectories are spread over
+// as many blocks as a free device has room for, but beside a stream those blocks
+// would take turns on the reserved SMs.
 #pragma once
 
 #include <chrono>
@@ -23,6 +27,7 @@ struct DeviceShare {
     std::mutex mu;
     std::condition_variable none;   // no network call in clusters
     int holders = 0;                // scan streams launched, batch scans running
+    int streams = 0;                // of these, the streams
     int clusters = 0;               // network calls running in clusters
 };
 
@@ -34,24 +39,39 @@ __attribute__((visibility("hidden"))) inline DeviceShare& device_share(int devic
     return all[(unsigned)device % kShareDevices];
 }
 
-inline void share_hold(int device, bool wait_for_clusters) {
+// A stream that is about to launch its kernel, and one whose launch has ended.
+inline void share_stream_begin(int device) {
     DeviceShare& d = device_share(device);
     std::unique_lock<std::mutex> l(d.mu);
     d.holders++;
-    if (wait_for_clusters) d.none.wait_for(l, std::chrono::seconds(2), [&] { return d.clusters == 0; });
+    d.streams++;
+    d.none.wait_for(l, std::chrono::seconds(2), [&] { return d.clusters == 0; });
 }
 
-inline void share_release(int device) {
+inline void share_stream_end(int device) {
     DeviceShare& d = device_share(device);
     std::lock_guard<std::mutex> l(d.mu);
     d.holders--;
+    d.streams--;
+}
+
+inline bool share_has_stream(int device) {
+    DeviceShare& d = device_share(device);
+    std::lock_guard<std::mutex> l(d.mu);
+    return d.streams > 0;
 }
 
 // A batch scan, for as long as the object lives.  (It ends by itself: it waits for nobody.)
 struct ShareHold {
-    const int device;
-    explicit ShareHold(int dev) : device(dev) { share_hold(dev, false); }
-    ~ShareHold() { share_release(device); }
+    DeviceShare& d;
+    explicit ShareHold(int device) : d(device_share(device)) {
+        std::lock_guard<std::mutex> l(d.mu);
+        d.holders++;
+    }
+    ~ShareHold() {
+        std::lock_guard<std::mutex> l(d.mu);
+        d.holders--;
+    }
     ShareHold(const ShareHold&) = delete;
     ShareHold& operator=(const ShareHold&) = delete;
 };

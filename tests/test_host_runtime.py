@@ -287,3 +287,22 @@ def test_network_where_no_cluster_fits(host):
     net = Network(host)
     assert (net.forward(), net.train()) == (1, 1)
     net.close()
+
+
+@pytest.mark.parametrize("models", TEAM_SETS)
+@pytest.mark.parametrize("n", [1, 20, 400])
+def test_teams_beside_a_stream_are_full(host, models, n):
+    """A free device takes a trajectory or a point to a block while it has room
+    for the blocks; on the SMs that a stream reserves they would run one after
+    the other."""
+    with ct.Context(0) as a, ct.Context(0) as b, small_stream(a) as st:
+        def blocks():
+            scan(b, n, models)
+            b.field_batch(points(n), params(1), ct.model_set(*models))
+            return [g for k, g in launched(host) if "team_" in k][-2:]
+        free = blocks()
+        st.submit(ct.make_job(50.0, 15.0, **JOB), params())
+        beside = blocks()
+        st.drain()
+        assert blocks() == free and min(free) >= min(n, 100)
+        assert max(beside) <= (n + 15) // 16        # 16 slots, the fewest of a full block
