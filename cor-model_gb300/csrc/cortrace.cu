@@ -65,6 +65,7 @@ struct cor_ctx {
     int park_below = 16;                  // regroup settings (cor_ctx_set_regroup)
     int max_generations = 48;
     uint64_t min_park = 256;
+    unsigned loaded = 0;                  // bit k: the kernels of kModelOps[k] are loaded (load_set)
     DevBuf steps;                         // trajectory dump: per-step records (cor_trace_steps)
     cor_step_record* step_dev = nullptr;  // set only while cor_trace_steps runs
     uint32_t step_cap = 0;
@@ -116,6 +117,8 @@ static int ensure(cor_ctx* ctx, DevBuf& b, size_t bytes) {
     return COR_OK;
 }
 
+static const ModelOps* const kModelOps[] = {&ops_igrf, &ops_igrf_t96, &ops_t96, &ops_igrf_ts05, &ops_ts05, &ops_crustal};
+
 extern "C" int cor_ctx_create(int device, cor_ctx** out) {
     if (!out) return COR_ERR_INVALID;
     *out = nullptr;
@@ -141,8 +144,7 @@ extern "C" int cor_ctx_create(int device, cor_ctx** out) {
         t96_tables(&tt);
         TS05Tables t5;
         ts05_tables(&t5);
-        const ModelOps* all[] = {&ops_igrf, &ops_igrf_t96, &ops_t96, &ops_igrf_ts05, &ops_ts05, &ops_crustal};
-        for (const ModelOps* o : all)
+        for (const ModelOps* o : kModelOps)
             if (o->upload_tables(&tt, &t5) != cudaSuccess) rc = COR_ERR_CUDA;
         if (rc != COR_OK) break;
     } while (0);
@@ -288,10 +290,23 @@ static bool model_set_ok(const cor_model_set& m) {
 static const ModelOps* find_ops(const cor_model_set& m) {
     if (m.crustal_model != COR_CRUSTAL_NONE) return &ops_crustal;
     const int key = m.internal_model * 100 + m.external_model * 10 + m.crustal_model;
-    static const ModelOps* const all[] = {&ops_igrf, &ops_igrf_t96, &ops_t96, &ops_igrf_ts05, &ops_ts05};
-    for (const ModelOps* o : all)
+    for (const ModelOps* o : kModelOps)
         if (o->key == key) return o;
     return nullptr;
+}
+
+// The first use of a model set on a context loads all of its kernels.  The
+// runtime loads a kernel when it is first used, and that may wait for every
+// kernel that runs: for a scan stream's, until it is drained.  Which kernels a
+// call takes depends on its size, so one that worked beside a stream would
+// otherwise stall there in another size.
+static int load_set(cor_ctx* ctx, const ModelOps* ops) {
+    for (unsigned k = 0; k < sizeof kModelOps / sizeof *kModelOps; k++) {
+        if (kModelOps[k] != ops || (ctx->loaded >> k & 1u)) continue;
+        CUDA_TRY(ctx, ops->load());
+        ctx->loaded |= 1u << k;
+    }
+    return COR_OK;
 }
 
 // Generations of the scan kernel.  Generation 0 drains the work queue; every
@@ -366,12 +381,12 @@ static int team_shape(cor_ctx* ctx, const ModelOps* ops, uint64_t live, int* slo
 }
 
 static int launch_trace(cor_ctx* ctx, const ModelOps* ops, TraceArgs a, cudaStream_t s) {
-    int per_sm = 0;
+    int per_sm = 0, rc;
+    if ((rc = load_set(ctx, ops)) != COR_OK) return rc;
     CUDA_TRY(ctx, ops->occupancy(&per_sm));
     if (per_sm < 1) per_sm = 1;
     const uint64_t cap_blocks = (uint64_t)ctx->sms * (uint64_t)per_sm;
     const size_t park_bytes = sizeof(ParkedLane) * (size_t)cap_blocks * kTraceThreads;
-    int rc;
     if ((rc = ensure(ctx, ctx->park[0], park_bytes)) != COR_OK) return rc;
     if ((rc = ensure(ctx, ctx->park[1], park_bytes)) != COR_OK) return rc;
     uint64_t live = a.n_traj;
@@ -749,6 +764,7 @@ static int field_queue(cor_ctx* ctx, const cor_model_set& models, const DevParam
     CrustalTables crust;
     if ((rc = crustal_tables(ctx, models, &crust)) != COR_OK) return rc;
     const ModelOps* ops = find_ops(models);
+    if ((rc = load_set(ctx, ops)) != COR_OK) return rc;
     if (team_takes_field(ops, models, (uint64_t)n, ctx->sms)) {
         int slots = 1;
         unsigned blocks = 1;
@@ -1054,6 +1070,7 @@ extern "C" int cor_trace_batch_device_noalloc(cor_ctx* ctx, const cor_scan_job* 
         const ModelOps* ops = find_ops(models);
         if (!ops) return fail(ctx, COR_ERR_UNSUPPORTED, "model set not available");
         int per_sm = 0;
+        if ((rc = load_set(ctx, ops)) != COR_OK) return rc;
         CUDA_TRY(ctx, ops->occupancy(&per_sm));
         if (per_sm < 1) per_sm = 1;
         const uint64_t cap = (uint64_t)ctx->sms * (uint64_t)per_sm;
@@ -1234,6 +1251,7 @@ extern "C" int cor_stream_create(cor_ctx* ctx, cor_model_set models, uint64_t st
     if (!ops) return fail(ctx, COR_ERR_UNSUPPORTED, "model set not available");
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     int per_sm = 0;
+    if ((rc = load_set(ctx, ops)) != COR_OK) return rc;
     CUDA_TRY(ctx, ops->stream_occupancy(&per_sm));
     if (per_sm < 1) return fail(ctx, COR_ERR_CUDA, "the stream kernel does not fit on an SM");
     cor_stream* s = new cor_stream();

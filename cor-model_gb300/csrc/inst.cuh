@@ -97,12 +97,17 @@
             team_field_kernel<MS><<<blocks, team_threads(n_slots), smem, s>>>(p, np, idx, pos, n, out, n_slots);\
             return cudaGetLastError();                                                                     \
         }                                                                                                  \
+        static cudaError_t load() {                                                                        \
+            const cudaError_t e = limit(team_trace_kernel<MS>);                                            \
+            return e != cudaSuccess ? e : limit(team_field_kernel<MS>);                                    \
+        }                                                                                                  \
         static constexpr auto occ_ptr = &occ;                                                              \
         static constexpr auto field_ptr = &field;                                                          \
         static constexpr auto run_ptr = &run;                                                              \
     };                                                                                                     \
     template <class MS>                                                                                    \
     struct Team_##NAME<MS, false> {                                                                        \
+        static cudaError_t load() { return cudaSuccess; }                                                  \
         static constexpr std::nullptr_t occ_ptr = nullptr;                                                 \
         static constexpr std::nullptr_t run_ptr = nullptr;                                                 \
         static constexpr std::nullptr_t field_ptr = nullptr;                                               \
@@ -118,14 +123,29 @@
             trace_kernel<MS, T><<<blocks, T, smem, s>>>(a);                                                \
             return cudaGetLastError();                                                                     \
         }                                                                                                  \
+        static cudaError_t load() {                                                                        \
+            cudaFuncAttributes at;                                                                         \
+            return cudaFuncGetAttributes(&at, trace_kernel<MS, kTraceThreads / 2>);                        \
+        }                                                                                                  \
         static constexpr auto ptr = &run;                                                                  \
     };                                                                                                     \
     template <class MS>                                                                                    \
     struct Halves_##NAME<MS, false> {                                                                      \
+        static cudaError_t load() { return cudaSuccess; }                                                  \
         static constexpr std::nullptr_t ptr = nullptr;                                                     \
     };                                                                                                     \
+    static cudaError_t load_##NAME() {                                                                     \
+        cudaFuncAttributes at;                                                                             \
+        int n = 0;                                                                                         \
+        cudaError_t e = occ_##NAME(&n);                                                                    \
+        if (e == cudaSuccess) e = socc_##NAME(&n);                                                         \
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, field_kernel<MS_##NAME>);                     \
+        if (e == cudaSuccess) e = Team_##NAME<MS_##NAME>::load();                                          \
+        if (e == cudaSuccess) e = Halves_##NAME<MS_##NAME>::load();                                        \
+        return e;                                                                                          \
+    }                                                                                                      \
     const ModelOps ops_##NAME = {I * 100 + E * 10 + C, occ_##NAME, gen_##NAME, field_##NAME, tables_##NAME, \
                                  socc_##NAME, stream_##NAME, Team_##NAME<MS_##NAME>::occ_ptr,               \
                                  Team_##NAME<MS_##NAME>::run_ptr, Team_##NAME<MS_##NAME>::field_ptr,         \
-                                 Halves_##NAME<MS_##NAME>::ptr};                                           \
+                                 Halves_##NAME<MS_##NAME>::ptr, load_##NAME};                              \
     }

@@ -32,6 +32,8 @@ struct ModelOps {
                                      int64_t n, double* out, int n_slots, unsigned blocks, cudaStream_t s);
     // launch_generation in blocks of half the threads; null for sets without it
     cudaError_t (*launch_halves)(const TraceArgs& a, unsigned blocks, cudaStream_t s);
+    // loads every kernel of the set on the current device
+    cudaError_t (*load)();
 };
 
 extern const ModelOps ops_igrf, ops_igrf_t96, ops_t96, ops_igrf_ts05, ops_ts05, ops_crustal;

@@ -40,6 +40,7 @@ struct Launch {
 // never destroyed: the library's own exit handlers run after this file's
 std::recursive_mutex& mu = *new std::recursive_mutex;
 std::vector<Copy>& pending = *new std::vector<Copy>;
+std::map<std::string, int>& loaded = *new std::map<std::string, int>;   // kernels used so far, launched or not
 std::vector<Launch>& launches = *new std::vector<Launch>;
 std::map<const void*, std::string>& names = *new std::map<const void*, std::string>;
 std::map<const void*, size_t>& limits = *new std::map<const void*, size_t>;
@@ -99,6 +100,7 @@ void fake_reset(void) {
     after_attribute = nullptr;
     during_wait = nullptr;
     last = cudaSuccess;
+    loaded.clear();
 }
 void fake_fail_launch(const char* part) { fail_launch = part; }
 void fake_fail_call(const char* call, int nth) { fail_call[call] = nth; }
@@ -114,6 +116,13 @@ int fake_launch(int i, char* name, int cap, unsigned* grid, unsigned* block, uin
     *block = launches[i].block;
     *smem = launches[i].smem;
     return 0;
+}
+// Kernels with `part` in their names that were used for the first time by their launch.
+int fake_loaded_by_launch(const char* part) {
+    int n = 0;
+    for (const auto& k : loaded)
+        if (k.first.find(part) != std::string::npos) n += k.second;
+    return n;
 }
 // The number of different limits set for the functions whose name has `part`.
 int fake_limits_set(const char* part) {
@@ -175,6 +184,7 @@ cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3 block, void**, si
     const auto lim = limits.find((const void*)k);
     if (smem > (lim == limits.end() ? 48 * 1024 : lim->second)) return set(cudaErrorInvalidValue);
     if (!fail_launch.empty() && name.find(fail_launch) != std::string::npos) return set(cudaErrorLaunchOutOfResources);
+    loaded.emplace(name, 1);
     launches.push_back({name, grid.x, block.x, smem});
     return cudaSuccess;
 }
@@ -183,6 +193,7 @@ cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
     {
         Lock l(mu);
         name = names[f];
+        loaded.emplace(name, 0);
         if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) {
             limits[f] = (size_t)v;
             limits_set[name].push_back((size_t)v);
@@ -190,6 +201,12 @@ cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
     }
     if (fails("cudaFuncSetAttribute")) return set(cudaErrorInvalidValue);
     if (after_attribute) after_attribute(name.c_str());
+    return cudaSuccess;
+}
+cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void* f) {
+    Lock l(mu);
+    *a = cudaFuncAttributes{};
+    loaded.emplace(names[f], 0);
     return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned) {

@@ -306,3 +306,25 @@ def test_teams_beside_a_stream_are_full(host, models, n):
         st.drain()
         assert blocks() == free and min(free) >= min(n, 100)
         assert max(beside) <= (n + 15) // 16        # 16 slots, the fewest of a full block
+
+
+@pytest.mark.parametrize("models", TEAM_SETS + [(1, 0, 1)])
+@pytest.mark.parametrize("first", [lambda c, m: scan(c, 100000, m), lambda c, m: scan(c, 1, m),
+                                   lambda c, m: c.field_batch(points(40000), params(1), ct.model_set(*m)),
+                                   lambda c, m: c.field_batch(points(1), params(1), ct.model_set(*m)),
+                                   lambda c, m: ct.Stream(c, ct.model_set(*m), slots=1, max_jobs=1,
+                                                          max_trajectories=8).close()],
+                         ids=["large scan", "small scan", "large field", "small field", "stream"])
+def test_first_use_of_a_set_loads_its_kernels(host, models, first):
+    """Loading a kernel may wait for a scan stream that is running (until it is
+    drained), so a set's kernels are all loaded by the first call, whatever the
+    sizes of the later ones."""
+    with ct.Context(0) as ctx:
+        first(ctx, models)
+        for n in (1, 20000, 100000):
+            scan(ctx, n, models)
+        for n in (1, 40000):
+            ctx.field_batch(points(n), params(1), ct.model_set(*models))
+        own = [k for k, _ in launched(host) if "trace_kernel" in k or "field_kernel" in k]
+        assert len(set(own)) >= (2 if models[2] else 4)
+        assert host.fake_loaded_by_launch(b"trace_kernel") == host.fake_loaded_by_launch(b"field_kernel") == 0
