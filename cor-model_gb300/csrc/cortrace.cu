@@ -739,20 +739,44 @@ extern "C" int cor_trace_steps(cor_ctx* ctx, const cor_batch_req* req, cor_batch
     return COR_OK;
 }
 
-// A field batch on the context's stream, in the context's own buffers (an
-// allocation and a free a call were 45 us).  The output buffer outlives the
-// call: every copy and launch is checked, since after one that failed it holds
-// an earlier call's fields.  On return, copies from and to all four host arrays
-// may be pending: a copy from pageable memory need not be staged where the GPU
+// A field batch's device buffers are kept between calls up to this size: an
+// allocation and a free a call were 45 us, of 53 to 240 us for a few thousand
+// points.  Larger ones (2.8 million points, 10 ms and more) are of the size
+// needed, and given back when the call ends.
+constexpr size_t kFieldKeep = 64u << 20;
+
+static bool field_is_large(int64_t n, int32_t n_params) {
+    return sizeof(double) * 3 * (size_t)n > kFieldKeep || sizeof(DevParams) * (size_t)n_params > kFieldKeep;
+}
+
+static int field_buffer(cor_ctx* ctx, DevBuf& b, size_t bytes, bool large) {
+    if (!large) return ensure(ctx, b, bytes);
+    CUDA_TRY(ctx, cudaMalloc(&b.p, bytes));
+    b.cap = bytes;
+    return COR_OK;
+}
+
+static void field_give_back(cor_ctx* ctx) {
+    for (DevBuf* b : {&ctx->f_params, &ctx->f_pos, &ctx->f_out, &ctx->f_idx}) {
+        if (b->p) cudaFree(b->p);
+        *b = DevBuf();
+    }
+}
+
+// A field batch on the context's stream, in the context's own buffers.  The
+// output buffer outlives the call: every copy and launch is checked, since after
+// one that failed it holds an earlier call's fields.  On return, copies from and
+// to all four host arrays may be pending: a copy from pageable memory need not be staged where the GPU
 // reads it through the host's page tables, as GB300's does.
 static int field_queue(cor_ctx* ctx, const cor_model_set& models, const DevParams* params, int32_t n_params,
                        const int32_t* param_index, const double* gsm_pos, int64_t n, double* geo_field) {
     cudaStream_t s = ctx->stream;
+    const bool large = field_is_large(n, n_params);
     int rc;
-    if ((rc = ensure(ctx, ctx->f_params, sizeof(DevParams) * (size_t)n_params)) != COR_OK) return rc;
-    if ((rc = ensure(ctx, ctx->f_pos, sizeof(double) * 3 * (size_t)n)) != COR_OK) return rc;
-    if ((rc = ensure(ctx, ctx->f_out, sizeof(double) * 3 * (size_t)n)) != COR_OK) return rc;
-    if (param_index && (rc = ensure(ctx, ctx->f_idx, sizeof(int32_t) * (size_t)n)) != COR_OK) return rc;
+    if ((rc = field_buffer(ctx, ctx->f_params, sizeof(DevParams) * (size_t)n_params, large)) != COR_OK) return rc;
+    if ((rc = field_buffer(ctx, ctx->f_pos, sizeof(double) * 3 * (size_t)n, large)) != COR_OK) return rc;
+    if ((rc = field_buffer(ctx, ctx->f_out, sizeof(double) * 3 * (size_t)n, large)) != COR_OK) return rc;
+    if (param_index && (rc = field_buffer(ctx, ctx->f_idx, sizeof(int32_t) * (size_t)n, large)) != COR_OK) return rc;
     const DevParams* dp = (const DevParams*)ctx->f_params.p;
     const double* dpos = (const double*)ctx->f_pos.p;
     const int32_t* didx = param_index ? (const int32_t*)ctx->f_idx.p : nullptr;
@@ -791,6 +815,8 @@ extern "C" int cor_field_batch(cor_ctx* ctx, cor_model_set models, const cor_mod
             return fail(ctx, COR_ERR_INVALID, "point %lld: param_index %d out of range", (long long)i, param_index[i]);
     if (n == 0) return COR_OK;
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
+    const bool large = field_is_large(n, n_params);
+    if (large) field_give_back(ctx);
     DevParams* hp = (DevParams*)malloc(sizeof(DevParams) * (size_t)n_params);
     if (!hp) return fail(ctx, COR_ERR_NOMEM, "host allocation");
     prepare_params(params, n_params, hp);
@@ -798,6 +824,7 @@ extern "C" int cor_field_batch(cor_ctx* ctx, cor_model_set models, const cor_mod
     // also after a failure: copies may be pending from hp and the caller's arrays
     const cudaError_t e = cudaStreamSynchronize(ctx->stream);
     free(hp);
+    if (large) field_give_back(ctx);
     if (rc != COR_OK) return rc;
     CUDA_TRY(ctx, e);
     return COR_OK;

@@ -47,6 +47,8 @@ std::map<const void*, size_t>& limits = *new std::map<const void*, size_t>;
 std::map<std::string, std::vector<size_t>>& limits_set = *new std::map<std::string, std::vector<size_t>>;
 std::string& fail_launch = *new std::string;
 std::map<std::string, int>& fail_call = *new std::map<std::string, int>;   // calls until the one that fails
+std::map<void*, size_t>& allocated = *new std::map<void*, size_t>;
+size_t in_use = 0, memory = ~(size_t)0;
 int freed_pending = 0;
 void (*after_attribute)(const char*) = nullptr;
 void (*during_wait)() = nullptr;
@@ -101,7 +103,11 @@ void fake_reset(void) {
     during_wait = nullptr;
     last = cudaSuccess;
     loaded.clear();
+    memory = ~(size_t)0;
 }
+// Device memory in all, and how much of it is allocated.
+void fake_memory(uint64_t bytes) { memory = bytes; }
+uint64_t fake_in_use(void) { return in_use; }
 void fake_fail_launch(const char* part) { fail_launch = part; }
 void fake_fail_call(const char* call, int nth) { fail_call[call] = nth; }
 int fake_freed_pending(void) { return freed_pending; }
@@ -237,12 +243,21 @@ cudaError_t cudaGetLastError(void) {
 }
 const char* cudaGetErrorString(cudaError_t e) { return e == cudaSuccess ? "no error" : "an error"; }
 cudaError_t cudaMalloc(void** p, size_t n) {
-    if (fails("cudaMalloc")) return set(cudaErrorMemoryAllocation);
+    Lock l(mu);
+    if (fails("cudaMalloc") || n > memory || in_use > memory - n) return set(cudaErrorMemoryAllocation);
     *p = calloc(1, n ? n : 1);
+    allocated[*p] = n;
+    in_use += n;
     return cudaSuccess;
 }
 cudaError_t cudaFree(void* p) {
     finish(true, nullptr);   // waits for the device
+    Lock l(mu);
+    const auto a = allocated.find(p);
+    if (a != allocated.end()) {
+        in_use -= a->second;
+        allocated.erase(a);
+    }
     __real_free(p);
     return cudaSuccess;
 }

@@ -37,6 +37,8 @@ def fake(tmp_path_factory):
     lib = ct.load(so)
     lib.fake_fail_launch.argtypes = [C.c_char_p]
     lib.fake_fail_call.argtypes = [C.c_char_p, C.c_int]
+    lib.fake_memory.argtypes = [C.c_uint64]
+    lib.fake_in_use.restype = C.c_uint64
     lib.fake_limits_set.argtypes = [C.c_char_p]
     lib.fake_launch.argtypes = [C.c_int, C.c_char_p, C.c_int, C.POINTER(C.c_uint), C.POINTER(C.c_uint),
                                 C.POINTER(C.c_uint64)]
@@ -328,3 +330,17 @@ def test_first_use_of_a_set_loads_its_kernels(host, models, first):
         own = [k for k, _ in launched(host) if "trace_kernel" in k or "field_kernel" in k]
         assert len(set(own)) >= (2 if models[2] else 4)
         assert host.fake_loaded_by_launch(b"trace_kernel") == host.fake_loaded_by_launch(b"field_kernel") == 0
+
+
+def test_large_field_batch_takes_what_it_needs_and_gives_it_back(host):
+    """Buffers kept between calls are those of small batches: a large one needs
+    48 bytes of device memory a point and no more, and leaves none behind."""
+    n = 4_000_000
+    with ct.Context(0) as ctx:
+        ctx.field_batch(points(21), params())
+        kept = host.fake_in_use()
+        host.fake_memory(kept + 48 * n + 1_000_000)
+        ctx.field_batch(points(n), params())
+        assert host.fake_in_use() < kept + 48 * n // 100
+        ctx.field_batch(points(n), params())
+        ctx.field_batch(points(21), params())
