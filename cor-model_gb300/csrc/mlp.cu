@@ -28,7 +28,9 @@
 // role leaves its loop, and the tile waits out what it issued and frees the TMEM.
 //
 // Measured: 2,664 rows forward 405 -> 43 us a call (kernel 22 us); a training
-// step of 512 rows 1,150 -> 103 us (rows_kernel 49, grad_kernel 16 us).  One
+// step of 512 rows, its loss read back, 1,150 -> 113 us (rows_kernel 49,
+// grad_kernel 16 us).  By one CTA to a tile 61 and 186 us, and 0.44 and 0.46 ms on
+// the two SMs that a scan stream leaves.  One
 // GEMM per launch had spent its time in synchronous stages (load, fence, MMA,
 // wait: 5 to 7 us each), in epilogues that wrote rows with a stride, and in 25
 // launches a step.  One CTA per 128 rows (without the cluster) took 38 and 111
